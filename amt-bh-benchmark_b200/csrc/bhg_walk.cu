@@ -116,20 +116,54 @@ __device__ __forceinline__ double far2(const double lo[3], const double hi[3], d
 // lane group g is target g + k * gp; lane k mod L of the group adds that
 // target's partial sums into its FP64 sum.
 
+// Two FP32 values in one 64-bit register: the SM's packed FP32 instructions
+// (add, mul, fma .f32x2) work on both halves in one issue slot, each half
+// rounded as the scalar instruction rounds it.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_pack(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_unpack(f2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 // Split precision.  Sources are staged once per batch in shared memory as
-// FP32 records relative to the walk box's centre (the subtraction in FP64),
-// and the warp is laid out as a grid of lanes: each lane owns kt (1 or 2)
-// targets and one of ng lane groups, which split the batch's sources
-// between them (group g takes sources g, g + ng, ...).  Every lane reads
-// the records it needs from shared memory (all lanes of a group read the
-// same record: a broadcast), so a source costs one global gather per warp,
-// not one per lane group, and the lanes never exchange partial sums inside
-// a batch.  Each loop iteration evaluates two independent (source, target)
-// pairs: two sources for one target (kt = 1) or one source for two targets
-// (kt = 2).  FP32 partials are added into per-lane FP64 sums once they hold
-// 32 or more terms (at most one batch's worth) and at the end of the walk;
-// then the lane groups' FP64 sums are added in group order (deterministic)
-// into the targets' FP64 sums.
+// FP32 values relative to the walk box's centre (the subtraction in FP64),
+// two sources to a record of packed pairs, and the warp is laid out as a grid
+// of lanes: each lane owns two targets and one of ng lane groups, which split
+// the batch's records between them (group g takes records g, g + ng, ...).
+// Every lane reads the records it needs from shared memory (all lanes of a
+// group read the same record: a broadcast), so a source costs one global
+// gather per warp, not one per lane group, and the lanes never exchange
+// partial sums inside a batch.  A loop iteration evaluates the four
+// interactions of a record's two sources with the lane's two targets in
+// packed FP32 arithmetic.  The FP32 partials (per target one for the first
+// and one for the second source of the records) are added into per-lane FP64
+// sums once they hold 32 or more terms (at most one batch's worth) and at the
+// end of the walk; then the lane groups' FP64 sums are added in group order
+// (deterministic) into the targets' FP64 sums.
+// What bounds it: issue slots and latency with 16 warps per SM, so halving the
+// FP32 instructions pays although the FMA pipe's own rate stays the same.
+// Walk per evaluation, scalar / packed: 32.9 / 30.5 ms at 4M (leaf 16),
+// 6.53 / 5.52 at 1M with leaf 48, 4.04 / 3.35 at 1M with monopoles; warp
+// instructions of a 1M walk 5.48e9 / 4.16e9.
 // rsqrt.approx.ftz.f32 (PTX ISA): the approximate reciprocal square root,
 // subnormal inputs and results flushed to zero.  The split evaluator's r^2 is
 // in units scaled to the system's size (at least eps^2 there, or masked when
@@ -142,18 +176,19 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
 
 template <bool QUAD, bool MASK>
 struct SplitEval {
-  // particle batches fill the staging records cells use (192 + the zero
-  // record <= kStageF4): 0.35% faster at 4M than batches of 128
+  // particle batches fill the staging area cells use
   static constexpr int kCellBatch = 64, kPartBatch = 192;
   // FP32 partials go into the FP64 sums once a lane has added kFlushTerms
-  // or more terms to them (so they never hold more than one 64-cell
-  // batch's worth), and at the end of the walk
+  // or more terms to them, and at the end of the walk
   static constexpr int kFlushTerms = 32;
-  static constexpr int kCellDummy = kCellBatch;  // record index of the zero cell (written once)
-  static constexpr int kPartDummy = kPartBatch;  // record index of the zero particle (written per batch)
-  static_assert(kPartBatch + 1 <= kStageF4 && kPartBatch + 32 <= kPartQ, "particle batch too large");
+  // Staged records, one plane of 16 bytes per record for each two components:
+  // cells (x, y) (z, m) (q0, q1) (q2, q3) (q4, q5), particles (x, y) (z, m).
+  // A 16-byte stride keeps the lane groups' reads free of bank conflicts.
+  static constexpr int kCellPlane = kCellBatch / 2, kPartPlane = kPartBatch / 2;
+  static_assert(5 * kCellPlane <= kStageF4 && 2 * kPartPlane <= kStageF4 && kPartBatch + 32 <= kPartQ,
+                "batches too large");
   const WalkArgs& a;
-  float4* stage;  // records: cells 3 float4 each, particles 1 float4 each
+  float4* stage;  // the planes
   double* red;    // per-lane FP64 sums at the end of a walk (aliases stage)
   double cx, cy, cz;  // reference point: the walk box's centre
   float eps2;         // softening in scaled units
@@ -164,21 +199,15 @@ struct SplitEval {
   // sums are scaled back
   double scale = 1.0, unscale2 = 1.0;  // see set_system
   float scale2f = 1.f;
-  int lane, tb, kt, lpg, ng, first, stride, offb;
-  float t0x, t0y, t0z, t1x, t1y, t1z;  // target positions (t1 = t0 when kt = 1)
-  float a0x, a0y, a0z, a1x, a1y, a1z;  // FP32 partials of the current batch
+  int lane, tb, lpg, ng, first;
+  f2 t0x, t0y, t0z, t1x, t1y, t1z;  // minus the targets' positions, in both halves (t1 = t0 where there is none)
+  f2 a0x, a0y, a0z, a1x, a1y, a1z;  // FP32 partials
   double s0x, s0y, s0z, s1x, s1y, s1z;  // FP64 sums of this lane
   double (*acc)[3];  // the targets' FP64 sums (shared memory)
   int pend;  // terms in this lane's FP32 partials since the last flush (an upper bound, warp-uniform)
 
   __device__ SplitEval(const WalkArgs& args, float4* stage_, int lane_) : a(args), stage(stage_), lane(lane_) {
     red = reinterpret_cast<double*>(stage_);
-    if (lane == 0) {
-      stage[3 * kCellDummy + 0] = make_float4(kFarAway, 0.f, 0.f, 0.f);
-      stage[3 * kCellDummy + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-      stage[3 * kCellDummy + 2] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    __syncwarp();
   }
 
   __device__ int cell_chunk() const { return kCellBatch; }
@@ -199,123 +228,147 @@ struct SplitEval {
   __device__ void setup(int, uint32_t p0, int n, double (*sums)[3]) {
     acc = sums;
     tb = n;
-    // one target per lane with 32 / tb lane groups, or two targets per lane
-    // with 32 / ceil(tb / 2) groups: whichever leaves fewer slots idle
-    const int n1 = tb <= 32 ? 32 / tb : 0;
-    const int l2 = (tb + 1) >> 1, n2 = 32 / l2;
-    kt = (n1 == 0 || n2 >= 2 * n1) ? 2 : 1;
-    lpg = kt == 1 ? tb : l2;
-    ng = kt == 1 ? n1 : n2;
-    const bool active = lane < lpg * ng;
-    const int slot = lane % lpg;
-    first = active ? lane / lpg : 1 << 30;  // inactive lanes take no sources
-    stride = kt == 1 ? 2 * ng : ng;
-    offb = kt == 1 ? ng : 0;
-    const int t0 = slot, t1 = (kt == 2 && slot + lpg < tb) ? slot + lpg : slot;
+    lpg = (tb + 1) >> 1;
+    ng = 32 / lpg;
+    first = lane < lpg * ng ? lane / lpg : 1 << 30;  // inactive lanes take no sources
+    const int t0 = lane % lpg, t1 = t0 + lpg < tb ? t0 + lpg : t0;
     const double4 q0 = a.pm[p0 + t0], q1 = a.pm[p0 + t1];
-    t0x = (float)(__dsub_rn(q0.x, cx) * scale), t0y = (float)(__dsub_rn(q0.y, cy) * scale);
-    t0z = (float)(__dsub_rn(q0.z, cz) * scale);
-    t1x = (float)(__dsub_rn(q1.x, cx) * scale), t1y = (float)(__dsub_rn(q1.y, cy) * scale);
-    t1z = (float)(__dsub_rn(q1.z, cz) * scale);
-    a0x = a0y = a0z = a1x = a1y = a1z = 0.f;
+    t0x = twice(__dsub_rn(cx, q0.x)), t0y = twice(__dsub_rn(cy, q0.y)), t0z = twice(__dsub_rn(cz, q0.z));
+    t1x = twice(__dsub_rn(cx, q1.x)), t1y = twice(__dsub_rn(cy, q1.y)), t1z = twice(__dsub_rn(cz, q1.z));
+    a0x = a0y = a0z = a1x = a1y = a1z = 0ull;
     s0x = s0y = s0z = s1x = s1y = s1z = 0.0;
     pend = 0;
   }
 
+  __device__ __forceinline__ f2 twice(double d) const {
+    const float f = (float)(d * scale);
+    return f2_pack(f, f);
+  }
+
+  // one target's FP32 partials (their two halves added in FP32: they hold
+  // every other term of one chain) into its FP64 sum
+  __device__ __forceinline__ void flush_one(f2& p, double& s) const {
+    float lo, hi;
+    f2_unpack(p, lo, hi);
+    s += (double)(lo + hi) * unscale2;
+    p = 0ull;
+  }
+
   __device__ __forceinline__ void flush() {
-    s0x += (double)a0x * unscale2, s0y += (double)a0y * unscale2, s0z += (double)a0z * unscale2;
-    if (kt == 1) {
-      s0x += (double)a1x * unscale2, s0y += (double)a1y * unscale2, s0z += (double)a1z * unscale2;
-    } else {
-      s1x += (double)a1x * unscale2, s1y += (double)a1y * unscale2, s1z += (double)a1z * unscale2;
-    }
-    a0x = a0y = a0z = a1x = a1y = a1z = 0.f;
+    flush_one(a0x, s0x), flush_one(a0y, s0y), flush_one(a0z, s0z);
+    flush_one(a1x, s1x), flush_one(a1y, s1y), flush_one(a1z, s1z);
   }
 
-  // one cell record's contribution to the target at (tx, ty, tz)
-  __device__ __forceinline__ void cell_body(const float4* r, float tx, float ty, float tz, float& ax, float& ay,
-                                            float& az) const {
-    const float4 r0 = r[0];
-    const float dx = r0.x - tx, dy = r0.y - ty, dz = r0.z - tz;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-    float ri = rsqrt_ftz(r2);
-    if (!QUAD && MASK) ri = r2 > 0.f ? ri : 0.f;
-    const float ri2 = ri * ri;
-    const float ri3 = ri * ri2;
+  // 1 / sqrt(r^2) of both halves (0 where r^2 = 0 when `zero`)
+  template <bool ZERO>
+  static __device__ __forceinline__ f2 rsqrt2(f2 r2) {
+    float lo, hi;
+    f2_unpack(r2, lo, hi);
+    float ilo = rsqrt_ftz(lo), ihi = rsqrt_ftz(hi);
+    if (ZERO) ilo = lo > 0.f ? ilo : 0.f, ihi = hi > 0.f ? ihi : 0.f;
+    return f2_pack(ilo, ihi);
+  }
+
+  // a record of two cells acting on the target at -(tx, ty, tz); the staged
+  // quadrupoles are negated: n.. = -Q..
+  __device__ __forceinline__ void cell_body(ulonglong2 xy, ulonglong2 zm, ulonglong2 n01, ulonglong2 n23,
+                                            ulonglong2 n45, f2 e2, f2 tx, f2 ty, f2 tz, f2& ax, f2& ay, f2& az) const {
+    const f2 dx = f2_add(xy.x, tx), dy = f2_add(xy.y, ty), dz = f2_add(zm.x, tz);
+    const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, e2)));
+    const f2 ri = rsqrt2<!QUAD && MASK>(r2);
+    const f2 ri2 = f2_mul(ri, ri);
+    const f2 ri3 = f2_mul(ri, ri2);
     if (QUAD) {
-      const float4 r1 = r[1];
-      const float2 r3 = *reinterpret_cast<const float2*>(&r[2]);
       // Q = [[q0 q3 q4] [q3 q1 q5] [q4 q5 q2]]
-      const float qx = fmaf(r1.x, dx, fmaf(r1.w, dy, r3.x * dz));
-      const float qy = fmaf(r1.w, dx, fmaf(r1.y, dy, r3.y * dz));
-      const float qz = fmaf(r3.x, dx, fmaf(r3.y, dy, r1.z * dz));
-      const float dqd = fmaf(dx, qx, fmaf(dy, qy, dz * qz));
-      const float ri5 = ri3 * ri2;
+      const f2 qx = f2_fma(n01.x, dx, f2_fma(n23.y, dy, f2_mul(n45.x, dz)));
+      const f2 qy = f2_fma(n23.y, dx, f2_fma(n01.y, dy, f2_mul(n45.y, dz)));
+      const f2 qz = f2_fma(n45.x, dx, f2_fma(n45.y, dy, f2_mul(n23.x, dz)));
+      const f2 dqd = f2_fma(dx, qx, f2_fma(dy, qy, f2_mul(dz, qz)));
+      const f2 ri5 = f2_mul(ri3, ri2);
       // m d / r^3 - Q d / r^5 + 2.5 (d Q d) d / r^7
-      const float c = fmaf(2.5f * dqd, ri5 * ri2, r0.w * ri3);
-      ax = fmaf(-ri5, qx, fmaf(c, dx, ax));
-      ay = fmaf(-ri5, qy, fmaf(c, dy, ay));
-      az = fmaf(-ri5, qz, fmaf(c, dz, az));
+      const f2 c = f2_fma(f2_mul(f2_pack(-2.5f, -2.5f), dqd), f2_mul(ri5, ri2), f2_mul(zm.y, ri3));
+      ax = f2_fma(ri5, qx, f2_fma(c, dx, ax));
+      ay = f2_fma(ri5, qy, f2_fma(c, dy, ay));
+      az = f2_fma(ri5, qz, f2_fma(c, dz, az));
     } else {
-      const float c = r0.w * ri3;
-      ax = fmaf(c, dx, ax), ay = fmaf(c, dy, ay), az = fmaf(c, dz, az);
+      const f2 c = f2_mul(zm.y, ri3);
+      ax = f2_fma(c, dx, ax), ay = f2_fma(c, dy, ay), az = f2_fma(c, dz, az);
     }
   }
 
-  __device__ __forceinline__ void part_body(const float4 r, float tx, float ty, float tz, float& ax, float& ay,
-                                            float& az) const {
-    const float dx = r.x - tx, dy = r.y - ty, dz = r.z - tz;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-    float ri = rsqrt_ftz(r2);
-    if (MASK) ri = r2 > 0.f ? ri : 0.f;
-    const float c = r.w * (ri * ri) * ri;
-    ax = fmaf(c, dx, ax), ay = fmaf(c, dy, ay), az = fmaf(c, dz, az);
+  __device__ __forceinline__ void part_body(ulonglong2 xy, ulonglong2 zm, f2 e2, f2 tx, f2 ty, f2 tz, f2& ax, f2& ay,
+                                            f2& az) const {
+    const f2 dx = f2_add(xy.x, tx), dy = f2_add(xy.y, ty), dz = f2_add(zm.x, tz);
+    const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, e2)));
+    const f2 ri = rsqrt2<MASK>(r2);
+    const f2 c = f2_mul(f2_mul(zm.y, f2_mul(ri, ri)), ri);
+    ax = f2_fma(c, dx, ax), ay = f2_fma(c, dy, ay), az = f2_fma(c, dz, az);
   }
 
   // accepted cells: node ids ring[(head + i) % kCellQ], i < cnt <= kCellBatch
   __device__ void cells(const uint32_t* ring, uint32_t head, int cnt) {
-    for (int i = lane; i < cnt; i += 32) {
-      const uint32_t n = ring[(head + (uint32_t)i) & (kCellQ - 1)];
-      const WNode* w = a.w + n;
-      const double2 cxy = *reinterpret_cast<const double2*>(&w->cx);
-      const double czz = w->cz;
-      const float4 r0 = make_float4((float)(__dsub_rn(cxy.x, cx) * scale), (float)(__dsub_rn(cxy.y, cy) * scale),
-                                    (float)(__dsub_rn(czz, cz) * scale), w->mass);
-      stage[3 * i] = r0;
-      if (QUAD) {
-        const float4 qa = *reinterpret_cast<const float4*>(w->q);
-        const float2 qb = a.q45[n];
-        // record layout: (q0 q1 q2 q3) (q4 q5 - -), in scaled units
-        stage[3 * i + 1] = make_float4(qa.x * scale2f, qa.y * scale2f, qa.z * scale2f, qa.w * scale2f);
-        stage[3 * i + 2] = make_float4(qb.x * scale2f, qb.y * scale2f, 0.f, 0.f);
+    float* st = reinterpret_cast<float*>(stage);
+    const int rounded = (cnt + 1) & ~1;  // an odd batch ends with a source that contributes exactly 0
+    for (int i = lane; i < rounded; i += 32) {
+      float* r = st + 4 * (i >> 1) + (i & 1);
+      float v[10] = {kFarAway, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (i < cnt) {
+        const uint32_t n = ring[(head + (uint32_t)i) & (kCellQ - 1)];
+        const WNode* w = a.w + n;
+        const double2 cxy = *reinterpret_cast<const double2*>(&w->cx);
+        const double czz = w->cz;
+        v[0] = (float)(__dsub_rn(cxy.x, cx) * scale), v[1] = (float)(__dsub_rn(cxy.y, cy) * scale);
+        v[2] = (float)(__dsub_rn(czz, cz) * scale), v[3] = w->mass;
+        if (QUAD) {
+          const float4 qa = *reinterpret_cast<const float4*>(w->q);
+          const float2 qb = a.q45[n];
+          v[4] = -qa.x * scale2f, v[5] = -qa.y * scale2f, v[6] = -qa.z * scale2f, v[7] = -qa.w * scale2f;
+          v[8] = -qb.x * scale2f, v[9] = -qb.y * scale2f;
+        }
       }
+#pragma unroll
+      for (int k = 0; k < (QUAD ? 10 : 4); ++k) r[(k >> 1) * (4 * kCellPlane) + (k & 1) * 2] = v[k];
     }
     __syncwarp();
-    for (int s = first; s < cnt; s += stride) {
-      const int sb = s + offb < cnt ? s + offb : kCellDummy;
-      cell_body(stage + 3 * s, t0x, t0y, t0z, a0x, a0y, a0z);
-      cell_body(stage + 3 * sb, t1x, t1y, t1z, a1x, a1y, a1z);
+    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(stage);
+    const f2 e2 = f2_pack(eps2, eps2);
+    const int nrec = rounded >> 1;
+    for (int s = first; s < nrec; s += ng) {
+      const ulonglong2 xy = rec[s], zm = rec[kCellPlane + s];
+      ulonglong2 n01 = {}, n23 = {}, n45 = {};
+      if (QUAD) n01 = rec[2 * kCellPlane + s], n23 = rec[3 * kCellPlane + s], n45 = rec[4 * kCellPlane + s];
+      cell_body(xy, zm, n01, n23, n45, e2, t0x, t0y, t0z, a0x, a0y, a0z);
+      cell_body(xy, zm, n01, n23, n45, e2, t1x, t1y, t1z, a1x, a1y, a1z);
     }
-    pend += (cnt + stride - 1) / stride;
+    pend += (nrec + ng - 1) / ng;
     if (pend >= kFlushTerms) flush(), pend = 0;
     __syncwarp();
   }
 
   // direct particles: particle indices ring[(head + i) % kPartQ], i < cnt <= kPartBatch
   __device__ void parts(const uint32_t* ring, uint32_t head, int cnt) {
-    for (int i = lane; i < cnt; i += 32) {
-      const double4 p = a.pm[ring[(head + (uint32_t)i) & (kPartQ - 1)]];
-      stage[i] = make_float4((float)(__dsub_rn(p.x, cx) * scale), (float)(__dsub_rn(p.y, cy) * scale),
-                             (float)(__dsub_rn(p.z, cz) * scale), (float)p.w);
+    float* st = reinterpret_cast<float*>(stage);
+    const int rounded = (cnt + 1) & ~1;
+    for (int i = lane; i < rounded; i += 32) {
+      float* r = st + 4 * (i >> 1) + (i & 1);
+      float4 v = make_float4(kFarAway, 0.f, 0.f, 0.f);
+      if (i < cnt) {
+        const double4 p = a.pm[ring[(head + (uint32_t)i) & (kPartQ - 1)]];
+        v = make_float4((float)(__dsub_rn(p.x, cx) * scale), (float)(__dsub_rn(p.y, cy) * scale),
+                        (float)(__dsub_rn(p.z, cz) * scale), (float)p.w);
+      }
+      r[0] = v.x, r[2] = v.y, r[4 * kPartPlane] = v.z, r[4 * kPartPlane + 2] = v.w;
     }
-    if (lane == 0) stage[kPartDummy] = make_float4(kFarAway, 0.f, 0.f, 0.f);
     __syncwarp();
-    for (int s = first; s < cnt; s += stride) {
-      const int sb = s + offb < cnt ? s + offb : kPartDummy;
-      part_body(stage[s], t0x, t0y, t0z, a0x, a0y, a0z);
-      part_body(stage[sb], t1x, t1y, t1z, a1x, a1y, a1z);
+    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(stage);
+    const f2 e2 = f2_pack(eps2, eps2);
+    const int nrec = rounded >> 1;
+    for (int s = first; s < nrec; s += ng) {
+      const ulonglong2 xy = rec[s], zm = rec[kPartPlane + s];
+      part_body(xy, zm, e2, t0x, t0y, t0z, a0x, a0y, a0z);
+      part_body(xy, zm, e2, t1x, t1y, t1z, a1x, a1y, a1z);
     }
-    pend += (cnt + stride - 1) / stride;
+    pend += (nrec + ng - 1) / ng;
     if (pend >= kFlushTerms) flush(), pend = 0;
     __syncwarp();
   }

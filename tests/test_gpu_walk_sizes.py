@@ -1,0 +1,36 @@
+"""The walk at the sizes where its batches and lane layouts change: targets of
+1 .. 65 particles (odd and even, one to 32 lane groups, past the largest walk
+group), source batches with remainders, both expansions, with and without the
+r^2 = 0 mask.  Interaction counts equal the oracle's; forces within the
+suite's bounds (FP64 1e-12, split 1e-5 of the global norm)."""
+import numpy as np
+import pytest
+
+import bhg
+from helpers import cube, rel_error
+from oracle import Params, soa
+from test_gpu_parity import _oracle_build
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [2, 3, 31, 32, 33, 63, 64, 65, 127, 129, 191, 193, 257, 1021, 4099]
+
+
+@pytest.mark.parametrize("precision,tol", [(bhg.PRECISION_FP64, 1e-12), (bhg.PRECISION_SPLIT, 1e-5)])
+@pytest.mark.parametrize("leaf", [1, 2, 3, 5, 7, 16, 31, 33, 64, 65, 300])
+def test_walk_sizes_match_oracle(gpu, oracle, leaf, precision, tol):
+    for n in SIZES:
+        parts = cube(n, 100 + n, spread=3.0)
+        dom, sk, perm, mp, t = _oracle_build(oracle, parts, leaf)
+        tg = oracle.targets(t, leaf, 1024)
+        for quad, eps2 in ((True, 1e-4), (True, 0.0), (False, 1e-4), (False, 0.0)):
+            racc, counts = oracle.walk(t, tg, soa(mp), [Params(0.6, eps2, 1.0, int(quad))] * len(tg))
+            gpu.upload(parts)
+            gpu.stats(reset=True)
+            gpu.build_tree(leaf, 1024)
+            gpu.compute_multipoles()
+            acc = gpu.walk_forces(bhg.Context.params(0.6, eps2, 1.0, quad, precision), leaf)
+            st = gpu.stats()
+            assert (st["pp"], st["pc"]) == (int(counts[0]), int(counts[1])), (n, quad, eps2)
+            assert np.all(np.isfinite(acc))
+            assert rel_error(acc, racc) <= tol, (n, quad, eps2)
