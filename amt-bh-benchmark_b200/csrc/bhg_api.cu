@@ -46,10 +46,11 @@ struct bhg_context {
   // capacities (cap_n covers the scratch, cap_part the state; a capacity is
   // 0 after a growth that failed part-way)
   size_t cap_n = 0, cap_part = 0, cap_nodes = 0, cap_sys = 0, cap_tiles = 0, cap_stiles = 0;
-  // the walk's per-warp lists of sources only some targets of a group take
-  // (list_warps warps' worth), and the particle cap of a walk group
+  // the walk's lists (list_warps slots of sources only some targets of a
+  // group take, dense_warps lists of sources all of them take), and the
+  // particle cap of a walk group
   void* list_buf = nullptr;
-  size_t list_warps = 0;
+  size_t list_warps = 0, dense_warps = 0;
   uint32_t walk_pack = kGroupMax;
 
   // device buffers
@@ -297,42 +298,46 @@ int walk_grid(bhg_context* c) {
   return c->sms * per;
 }
 
-// The walk's list slots (walk_slot_bytes(), ~34 KB each): two per warp of
-// the walk grid (161 MB on a 148-SM B200) - one list per warp in the one-pass
-// schedule, one per group in the two-pass schedule, which therefore serves
-// up to two groups per warp.  Allocated before the walk is captured
-// (walk_grid has also set the kernels' shared-memory limit by then).  Under
-// a tight HBM budget there are fewer slots and the walk runs on as many
-// blocks as have a slot per warp (at least one block): a group's result does
-// not depend on the warp that walks it nor on the schedule, so the bits are
-// the same, only fewer groups at a time.
-constexpr size_t kSlotsPerWarp = 2;
+// The walk's lists: a dense list per warp of the grid, and list slots
+// (walk_slot_bytes(), ~34 KB each) - one per warp in the one-pass schedule,
+// one per group in the two-pass schedule, which therefore serves as many
+// groups as there are slots: 32 per SM, 4,736 on a 148-SM B200 (161 MB, and
+// 58 MB of dense lists).  Allocated before the walk is captured (walk_grid has
+// also set the kernels' shared-memory limit by then).  Under a tight HBM
+// budget there are fewer and the walk runs on as many blocks as have both per
+// warp (at least one block): a group's result does not depend on the warp
+// that walks it nor on the schedule, so the bits are the same, only fewer
+// groups at a time.
+constexpr size_t kSlotsPerSm = 32;
 
 int ensure_walk_scratch(bhg_context* c, int grid) {
-  const size_t per_slot = walk_slot_bytes();
+  const size_t per_slot = walk_slot_bytes(), per_dense = walk_dense_bytes();
   const size_t wpb = walk_threads() / 32;
-  size_t slots = (size_t)grid * wpb * kSlotsPerWarp;
-  if (c->list_warps >= slots) return BHG_OK;
+  size_t warps = (size_t)grid * wpb;
+  size_t slots = std::max(warps, kSlotsPerSm * (size_t)c->sms / wpb * wpb);
+  if (c->list_warps >= slots && c->dense_warps >= warps) return BHG_OK;
   if (c->budget) {
-    const size_t held = c->list_warps * per_slot;  // freed below, so it counts as room
+    const size_t held = c->list_warps * per_slot + c->dense_warps * per_dense;  // freed below, so it counts as room
     const size_t room = c->budget > c->allocated - held ? c->budget - (c->allocated - held) : 0;
-    slots = std::min(slots, std::max(wpb, room / per_slot / wpb * wpb));
-    if (c->list_warps >= slots) return BHG_OK;
+    if (room < slots * per_slot + warps * per_dense)
+      slots = warps = std::min(warps, std::max(wpb, room / (per_slot + per_dense) / wpb * wpb));
+    if (c->list_warps >= slots && c->dense_warps >= warps) return BHG_OK;
   }
   drop_graph(c);
   dev_free(c, c->list_buf);
   c->list_buf = nullptr;
-  c->list_warps = 0;
-  int r = dev_alloc(c, &c->list_buf, slots * per_slot);
+  c->list_warps = c->dense_warps = 0;
+  int r = dev_alloc(c, &c->list_buf, slots * per_slot + warps * per_dense);
   if (r) return r;
   c->list_warps = slots;
+  c->dense_warps = warps;
   return BHG_OK;
 }
 
 // Blocks of the walk launch: the occupancy grid, or fewer when the HBM
-// budget limited the slots (one per warp at least).
+// budget limited the lists (both kinds per warp at least).
 int walk_launch_grid(bhg_context* c) {
-  return (int)std::min<size_t>((size_t)walk_grid(c), c->list_warps / (walk_threads() / 32));
+  return (int)std::min<size_t>((size_t)walk_grid(c), std::min(c->list_warps, c->dense_warps) / (walk_threads() / 32));
 }
 
 // Lays out the systems c->counts back to back with their sort tiles, sizes
@@ -480,12 +485,14 @@ void enq_walk(bhg_context* c, bool want_accel) {
   a.out = c->part;
   a.accel = want_accel ? c->accel : nullptr;
   a.st = c->st;
-  // slots: the lists, then the groups' sums, then the list lengths
+  // the slots' lists, then the groups' sums, the list lengths, the dense lists
   a.nslots = (uint32_t)c->list_warps;
   a.wlist = static_cast<uint2*>(c->list_buf);
-  a.gsum = reinterpret_cast<double*>(reinterpret_cast<char*>(c->list_buf) +
-                                     c->list_warps * (walk_slot_bytes() - kGroupMax * 3 * sizeof(double) - sizeof(uint32_t)));
+  a.gsum = reinterpret_cast<double*>(
+      reinterpret_cast<char*>(c->list_buf) +
+      c->list_warps * (walk_slot_bytes() - kGroupMax * 3 * sizeof(double) - sizeof(uint32_t)));
   a.gnl = reinterpret_cast<uint32_t*>(a.gsum + c->list_warps * kGroupMax * 3);
+  a.dlist = reinterpret_cast<uint2*>(reinterpret_cast<char*>(c->list_buf) + c->list_warps * walk_slot_bytes());
   // list lengths "pending" (bytes 0xfe): the two-pass schedule's target jobs
   // wait for their group's length
   cudaMemsetAsync(a.gnl, 0xfe, c->list_warps * sizeof(uint32_t), c->stream);

@@ -61,7 +61,9 @@ struct WalkArgs {
   // list slots (nslots, at least one per warp of the grid): the sources only
   // some targets of a group take, per warp (one pass) or per group (two
   // passes, when there are at most nslots groups); per slot also the group's
-  // FP64 sums (kGroupMax x 3) and list length
+  // FP64 sums (kGroupMax x 3) and list lengths; per warp of the grid a dense
+  // list (the sources every target of the group takes)
+  uint2* dlist;
   uint2* wlist;
   double* gsum;
   uint32_t* gnl;
@@ -73,8 +75,9 @@ struct WalkArgs {
 void launch_walk(const WalkArgs& a, int precision, bool quad, bool mask, int grid, cudaStream_t s);
 int walk_blocks_per_sm(int precision, bool quad, bool mask);
 int walk_threads();
-// device bytes of one list slot
+// device bytes of one list slot, and of one warp's dense list
 size_t walk_slot_bytes();
+size_t walk_dense_bytes();
 
 void launch_integrate(Particle* p, const double* accel, uint32_t n, const SysDev* sys, const SysParam* prm, int nsys,
                       int sms, cudaStream_t s);

@@ -15,28 +15,26 @@
 // most kGroupMax particles and kMaxTargets targets, k_pack_groups), sharing
 // the walk among the group's targets as GroupWalker::visit does, taken to
 // every level: one traversal from the root whose stack entries carry the
-// mask of targets that still need the node.  A node accepted for the
+// mask of targets that still need the nodes.  A node accepted for the
 // group's bounding box is accepted by every target in the mask; one rejected
 // for every point of it (mac_reject_all, multipole.h:158-160) is opened by
-// all of them; otherwise each target in the mask tests its own box, one
-// (node, target) pair per lane.  Sources every target of the group takes are
-// evaluated once against all the group's particles; sources only some take
-// go to the warp's list as (node or leaf run, target mask), and each target
-// then passes over the list taking its own entries.  Each target's list is
-// the same as a separate walk of its box from the root would build.
+// all of them; otherwise each target tests its own box.  Sources every
+// target of the group takes go to the warp's dense list, sources only some
+// take to its partial list as (node or leaf run, target mask).  Each target's
+// list is the same as a separate walk of its box from the root would build.
 //
-// A walk step pops up to 32 entries (one per lane) from a shared-memory
-// stack; accepted cells and opened leaves' particles go to two
-// shared-memory queues, and a full queue is evaluated as one batch (64 cells
-// or 192 particles in split precision; one source per lane against up to 2
-// targets per lane in FP64).
+// Then the lists are evaluated: the dense one once against all the group's
+// particles, the partial one once per target, which takes its own entries.
+// A list pass gathers the picked sources into batches (64 cells or 128
+// particles in split precision, 32 or 64 in FP64).  Traversal and evaluation
+// take turns, so that neither holds registers or shared memory of the other.
 //
-// Split precision: sources and targets become FP32 offsets from the walk's
-// bounding-box centre (the subtraction in FP64), staged once per batch in
-// shared memory; interactions are FP32 FMA + rsqrt.approx.ftz, lanes laid out as
-// (target, source subset) (SplitEval below); FP32 partials go into FP64
-// sums every 32 or more terms.  The kick/drift of integrate_ttg.h:74-77 is
-// applied in FP64 in the epilogue.
+// Split precision: sources and targets become FP32 offsets from the
+// particles' bounding-box centre (the subtraction in FP64), staged once per
+// batch in shared memory; interactions are packed FP32 FMA +
+// rsqrt.approx.ftz, lanes laid out as (target, source subset) (SplitEval
+// below); FP32 partials go into FP64 sums every 32 or more terms.  The
+// kick/drift of integrate_ttg.h:74-77 is applied in FP64 in the epilogue.
 #include "bhg_kernels.h"
 
 #include <type_traits>
@@ -45,43 +43,73 @@ namespace bhg {
 
 constexpr int kWalkWarps = 4;
 constexpr int kWalkThreads = kWalkWarps * 32;
-constexpr int kCellQ = 128;   // ring of accepted cells (a batch of up to 64 + one step's 32)
-constexpr int kPartQ = 256;   // ring of direct particles (a batch of up to 192 + 32 enqueued)
-constexpr int kStackCap = 704;   // per-warp stack: node + target mask per entry
-constexpr int kStageF4 = 3 * 64 + 3;  // staged source records (float4): 64 cells + the zero cell
+constexpr int kStackCap = 192;       // per-warp traversal stack: runs of sibling nodes
+constexpr int kRing = 160;           // sources picked for the next batch (a batch of up to 128, less one, + 32)
+constexpr int kStageBytes = 2560;    // staged sources of one batch
 constexpr float kFarAway = 1.0e10f;  // padding source: contributes exactly 0
 constexpr uint32_t kFull = 0xffffffffu;
-// A list entry is (node, target mask) for a cell, or (first particle |
-// kLeafBit, target mask | count << kCountShift) for a run of at most
-// kMaxRun particles of a leaf (a larger leaf takes several entries), so that
-// the targets' passes need no second load for it.
-constexpr uint32_t kLeafBit = 0x80000000u;
+// Lists are two-ended arrays of uint2: cells from the front, runs of particles
+// (opened leaves) from the back.  The dense list (sources every target of
+// the group takes): (node, 1) and (first particle, count).  The partial list
+// (sources some targets take): (node, target mask) and (first particle, mask
+// | count << kCountShift), or (leaf node, mask | kByNode << kCountShift) for
+// a leaf of kByNode particles or more.
 constexpr int kCountShift = 24;
-constexpr uint32_t kMaxRun = 255;
-static_assert(kMaxTargets <= kCountShift, "target masks and run lengths share a word");
-constexpr uint32_t kListCap = 4096;         // entries of one partial-source list (32 KB)
-constexpr uint32_t kNotShared = 0xffffffffu;  // a group whose list overflowed: its targets walk alone
-// a group's list length before its shared walk has finished (two-pass schedule;
-// the host fills the lengths with this byte pattern before every walk)
+constexpr uint32_t kMaskBits = (1u << kCountShift) - 1u;
+constexpr uint32_t kByNode = 255;
+static_assert(kMaxTargets <= kCountShift, "target masks and counts share a word");
+constexpr uint32_t kDenseCap = 2048;  // entries of a dense list (16 KB)
+constexpr uint32_t kListCap = 4096;   // entries of a partial list (32 KB)
+// a group's list lengths (cells | runs << 16) before its shared walk has
+// finished (two-pass schedule; the host fills the lengths with this byte
+// pattern before every walk)
 constexpr uint32_t kListPending = 0xfefefefeu;
-// a walk that pops one node at a time holds at most 7 entries per level
-// below the one it pops from, plus the root
-static_assert(kStackCap >= 7 * kLevels + 1 + 8, "a one-at-a-time walk must fit the stack");
-static_assert(kStageF4 * 16 >= 32 * 6 * 8, "the end-of-walk reduction reuses the staging records");
+static_assert(kListCap < 0xfefe, "list lengths never look pending");
+// a traversal step pops at most (free entries - kLevels - 1) nodes, one at
+// least, and every popped node pushes at most one run of children, so that
+// one-node steps (depth first, at most one run per level) never overflow
+static_assert(kStackCap >= 32 + 2 * (kLevels + 1), "the stack holds a step's pushes");
+
+struct Walk {
+  uint32_t top, steps;          // stack entries; steps so far
+  uint32_t ndc, ndr, npc, npr;  // dense cells and runs, partial cells and runs
+};
+
+// A warp's job, kept in shared memory (every lane writes the same values, a
+// __syncwarp away from reads of older ones): the evaluation loops need the
+// registers.
+struct Job {
+  uint32_t gi, ti;         // walk group; target (target jobs)
+  uint32_t t0, k, p0, sys;  // the group's first target, targets, first particle, system
+  uint32_t n, b0;          // particles; a large target's batch start
+  uint32_t pass1;          // the last pass to run
+  uint32_t more, jobs;     // the traversal paused; this is a target job
+  Walk w;
+};
 
 struct WarpSmem {
-  uint32_t snode[kStackCap];  // traversal stack: node
-  uint32_t smask[kStackCap];  //                  targets that still need it
-  uint32_t cell[kCellQ];
-  uint32_t part[kPartQ];
-  float4 stage[kStageF4];
-  double acc[kGroupMax][3];   // FP64 sum per particle of the group
+  uint2 stack[kStackCap];  // run of sibling nodes: (first node, targets that still need them | nodes << 24)
+  alignas(16) unsigned char stage[kStageBytes];  // a batch's staged sources; scratch of a traversal step
+  double sums[6][32];        // FP64 sums of the lanes (evaluators)
+  double acc[kGroupMax][3];  // FP64 sum per particle of the group
   double tlo[kMaxTargets][3], thi[kMaxTargets][3];  // the targets' particle boxes
-  double glo[3], ghi[3];                              // the group's particle box
-  uint32_t tbeg[kMaxTargets], tcnt[kMaxTargets];      // the targets' particles
-  uint32_t accbits[32];  // per popped entry: targets that accept it (per-target tests)
+  double glo[3], ghi[3];                            // the group's particle box
+  double centre[3], scale, scale2, eps2;            // evaluators' reference point and units
+  unsigned long long ncell, npart;                  // interactions of this warp
+  Job job;
+  uint32_t tbeg[kMaxTargets], tcnt[kMaxTargets];    // the targets' particles
+  uint32_t ring[kRing];
+  uint32_t delta[32];  // runs of a window: first particle less the particles of the runs before it
 };
 constexpr size_t kWalkSmem = sizeof(WarpSmem) * kWalkWarps;
+
+// Scratch of a traversal step (in WarpSmem::stage): the nodes that targets
+// test on their own, and the targets that accept them.
+struct StepScratch {
+  double4 node[32];  // centre of mass, edge^2
+  uint32_t accepts[32];
+};
+static_assert(sizeof(StepScratch) <= kStageBytes && kGroupMax * 3 * 8 <= kStageBytes, "scratch in the staging area");
 
 __device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t v, int lane) {
 #pragma unroll
@@ -159,10 +187,10 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
 // sums once they hold 32 or more terms (at most one batch's worth) and at the
 // end of the walk; then the lane groups' FP64 sums are added in group order
 // (deterministic) into the targets' FP64 sums.
-// What bounds it: issue slots and latency with 16 warps per SM, so halving the
-// FP32 instructions pays although the FMA pipe's own rate stays the same.
-// Walk per evaluation, scalar / packed: 32.9 / 30.5 ms at 4M (leaf 16),
-// 6.53 / 5.52 at 1M with leaf 48, 4.04 / 3.35 at 1M with monopoles; warp
+// What bounds it: issue slots and latency, so halving the FP32 instructions
+// pays although the FMA pipe's own rate stays the same.  Walk per evaluation,
+// scalar / packed, with 16 warps per SM: 32.9 / 30.5 ms at 4M (leaf 16), 6.53
+// / 5.52 at 1M with leaf 48, 4.04 / 3.35 at 1M with monopoles; warp
 // instructions of a 1M walk 5.48e9 / 4.16e9.
 // rsqrt.approx.ftz.f32 (PTX ISA): the approximate reciprocal square root,
 // subnormal inputs and results flushed to zero.  The split evaluator's r^2 is
@@ -174,92 +202,98 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
+// The lane groups' sums (S.sums; lane g * lpg + l: targets l and l + lpg),
+// added in group order into the targets' FP64 sums out[0 .. tb).
+__device__ __forceinline__ void add_group_sums(const WarpSmem& S, int lane, int tb, int lpg, int ng, double (*out)[3]) {
+  for (int t = lane; t < tb; t += 32) {
+    const int k = t >= lpg ? 3 : 0, sl = k ? t - lpg : t;
+    double x = 0.0, y = 0.0, z = 0.0;
+    for (int g = 0; g < ng; ++g) {
+      const int l = g * lpg + sl;
+      x += S.sums[k][l], y += S.sums[k + 1][l], z += S.sums[k + 2][l];
+    }
+    out[t][0] += x, out[t][1] += y, out[t][2] += z;
+  }
+  __syncwarp();
+}
+
 template <bool QUAD, bool MASK>
 struct SplitEval {
-  // particle batches fill the staging area cells use
-  static constexpr int kCellBatch = 64, kPartBatch = 192;
+  static constexpr int kCellBatch = 64, kPartBatch = 128;
+  static constexpr int kBlocksPerSm = 6;
   // FP32 partials go into the FP64 sums once a lane has added kFlushTerms
-  // or more terms to them, and at the end of the walk
+  // or more terms to them, and at the end of a list
   static constexpr int kFlushTerms = 32;
   // Staged records, one plane of 16 bytes per record for each two components:
   // cells (x, y) (z, m) (q0, q1) (q2, q3) (q4, q5), particles (x, y) (z, m).
   // A 16-byte stride keeps the lane groups' reads free of bank conflicts.
   static constexpr int kCellPlane = kCellBatch / 2, kPartPlane = kPartBatch / 2;
-  static_assert(5 * kCellPlane <= kStageF4 && 2 * kPartPlane <= kStageF4 && kPartBatch + 32 <= kPartQ,
+  static_assert(5 * 16 * kCellPlane <= kStageBytes && 2 * 16 * kPartPlane <= kStageBytes && kPartBatch + 31 < kRing,
                 "batches too large");
   const WalkArgs& a;
-  float4* stage;  // the planes
-  double* red;    // per-lane FP64 sums at the end of a walk (aliases stage)
-  double cx, cy, cz;  // reference point: the walk box's centre
-  float eps2;         // softening in scaled units
+  WarpSmem& S;
   // the FP32 arithmetic runs on offsets times a power of two near the
   // system's size (1 / 2^ilogb(domain half width)), so that r^-7 of the
   // smallest and largest systems stays inside FP32's range; the powers of two
   // make the scaling exact (rsqrt of an even power of two too), and the FP64
-  // sums are scaled back
-  double scale = 1.0, unscale2 = 1.0;  // see set_system
-  float scale2f = 1.f;
-  int lane, tb, lpg, ng, first;
+  // sums are scaled back.  The scales and the reference point (the box's
+  // centre) stay in shared memory: no registers while a batch is evaluated.
+  int lane, ng, first;
   f2 t0x, t0y, t0z, t1x, t1y, t1z;  // minus the targets' positions, in both halves (t1 = t0 where there is none)
   f2 a0x, a0y, a0z, a1x, a1y, a1z;  // FP32 partials
-  double s0x, s0y, s0z, s1x, s1y, s1z;  // FP64 sums of this lane
-  double (*acc)[3];  // the targets' FP64 sums (shared memory)
   int pend;  // terms in this lane's FP32 partials since the last flush (an upper bound, warp-uniform)
 
-  __device__ SplitEval(const WalkArgs& args, float4* stage_, int lane_) : a(args), stage(stage_), lane(lane_) {
-    red = reinterpret_cast<double*>(stage_);
-  }
-
-  __device__ int cell_chunk() const { return kCellBatch; }
-  __device__ int part_chunk() const { return kPartBatch; }
-
   // softening eps2_ and the system's domain half width hw
-  __device__ void set_system(double eps2_, double hw) {
+  __device__ SplitEval(const WalkArgs& args, WarpSmem& S_, int lane_, double eps2_, double hw)
+      : a(args), S(S_), lane(lane_) {
     int k = hw > 0.0 ? ilogb(hw) : 0;
     k = k < -100 ? -100 : (k > 100 ? 100 : k);
-    scale = ldexp(1.0, -k);            // offsets d' = d * scale
-    unscale2 = ldexp(1.0, -2 * k);     // a = a' * scale^2 (a' = m d' / r'^3 = a / scale^2)
-    scale2f = (float)ldexp(1.0, -2 * k);  // Q' = Q * scale^2, eps2' = eps2 * scale^2
-    eps2 = (float)(eps2_ * (scale * scale));
+    const double scale = ldexp(1.0, -k);
+    S.scale = scale;                   // offsets d' = d * scale
+    S.scale2 = ldexp(1.0, -2 * k);     // a = a' * scale^2 (a' = m d' / r'^3 = a / scale^2), Q' = Q * scale^2
+    S.eps2 = eps2_ * (scale * scale);  // eps2' = eps2 * scale^2
   }
 
-  // targets: particles p0 .. p0 + n - 1 (n <= 64); their FP64 sums are
-  // added to sums[0 .. n)
-  __device__ void setup(int, uint32_t p0, int n, double (*sums)[3]) {
-    acc = sums;
-    tb = n;
-    lpg = (tb + 1) >> 1;
+  // targets: particles p0 .. p0 + n - 1 (n <= 64), offsets from (x, y, z)
+  __device__ void setup(uint32_t p0, int n, double x, double y, double z) {
+    S.centre[0] = x, S.centre[1] = y, S.centre[2] = z;
+    const int lpg = (n + 1) >> 1;
     ng = 32 / lpg;
     first = lane < lpg * ng ? lane / lpg : 1 << 30;  // inactive lanes take no sources
-    const int t0 = lane % lpg, t1 = t0 + lpg < tb ? t0 + lpg : t0;
+    const int t0 = lane % lpg, t1 = t0 + lpg < n ? t0 + lpg : t0;
     const double4 q0 = a.pm[p0 + t0], q1 = a.pm[p0 + t1];
-    t0x = twice(__dsub_rn(cx, q0.x)), t0y = twice(__dsub_rn(cy, q0.y)), t0z = twice(__dsub_rn(cz, q0.z));
-    t1x = twice(__dsub_rn(cx, q1.x)), t1y = twice(__dsub_rn(cy, q1.y)), t1z = twice(__dsub_rn(cz, q1.z));
+    const double scale = S.scale;
+    t0x = twice(__dsub_rn(x, q0.x) * scale), t0y = twice(__dsub_rn(y, q0.y) * scale);
+    t0z = twice(__dsub_rn(z, q0.z) * scale);
+    t1x = twice(__dsub_rn(x, q1.x) * scale), t1y = twice(__dsub_rn(y, q1.y) * scale);
+    t1z = twice(__dsub_rn(z, q1.z) * scale);
     a0x = a0y = a0z = a1x = a1y = a1z = 0ull;
-    s0x = s0y = s0z = s1x = s1y = s1z = 0.0;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) S.sums[c][lane] = 0.0;
     pend = 0;
   }
 
-  __device__ __forceinline__ f2 twice(double d) const {
-    const float f = (float)(d * scale);
+  static __device__ __forceinline__ f2 twice(double d) {
+    const float f = (float)d;
     return f2_pack(f, f);
   }
 
-  // one target's FP32 partials (their two halves added in FP32: they hold
-  // every other term of one chain) into its FP64 sum
-  __device__ __forceinline__ void flush_one(f2& p, double& s) const {
+  // one FP32 partial (its two halves added in FP32: they hold every other
+  // term of one chain) into its FP64 sum
+  __device__ __forceinline__ void flush_one(f2& p, int c) const {
     float lo, hi;
     f2_unpack(p, lo, hi);
-    s += (double)(lo + hi) * unscale2;
+    S.sums[c][lane] += (double)(lo + hi) * S.scale2;
     p = 0ull;
   }
 
   __device__ __forceinline__ void flush() {
-    flush_one(a0x, s0x), flush_one(a0y, s0y), flush_one(a0z, s0z);
-    flush_one(a1x, s1x), flush_one(a1y, s1y), flush_one(a1z, s1z);
+    flush_one(a0x, 0), flush_one(a0y, 1), flush_one(a0z, 2);
+    flush_one(a1x, 3), flush_one(a1y, 4), flush_one(a1z, 5);
+    pend = 0;
   }
 
-  // 1 / sqrt(r^2) of both halves (0 where r^2 = 0 when `zero`)
+  // 1 / sqrt(r^2) of both halves (0 where r^2 = 0 when ZERO)
   template <bool ZERO>
   static __device__ __forceinline__ f2 rsqrt2(f2 r2) {
     float lo, hi;
@@ -305,15 +339,17 @@ struct SplitEval {
     ax = f2_fma(c, dx, ax), ay = f2_fma(c, dy, ay), az = f2_fma(c, dz, az);
   }
 
-  // accepted cells: node ids ring[(head + i) % kCellQ], i < cnt <= kCellBatch
-  __device__ void cells(const uint32_t* ring, uint32_t head, int cnt) {
-    float* st = reinterpret_cast<float*>(stage);
+  // cells: node ids ring[0 .. cnt), cnt <= kCellBatch
+  __device__ __forceinline__ void cells(const uint32_t* ring, int cnt) {
+    float* st = reinterpret_cast<float*>(S.stage);
     const int rounded = (cnt + 1) & ~1;  // an odd batch ends with a source that contributes exactly 0
+    const double cx = S.centre[0], cy = S.centre[1], cz = S.centre[2], scale = S.scale;
+    const float scale2f = (float)S.scale2;
     for (int i = lane; i < rounded; i += 32) {
       float* r = st + 4 * (i >> 1) + (i & 1);
       float v[10] = {kFarAway, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (i < cnt) {
-        const uint32_t n = ring[(head + (uint32_t)i) & (kCellQ - 1)];
+        const uint32_t n = ring[i];
         const WNode* w = a.w + n;
         const double2 cxy = *reinterpret_cast<const double2*>(&w->cx);
         const double czz = w->cz;
@@ -330,8 +366,8 @@ struct SplitEval {
       for (int k = 0; k < (QUAD ? 10 : 4); ++k) r[(k >> 1) * (4 * kCellPlane) + (k & 1) * 2] = v[k];
     }
     __syncwarp();
-    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(stage);
-    const f2 e2 = f2_pack(eps2, eps2);
+    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(S.stage);
+    const f2 e2 = twice(S.eps2);
     const int nrec = rounded >> 1;
     for (int s = first; s < nrec; s += ng) {
       const ulonglong2 xy = rec[s], zm = rec[kCellPlane + s];
@@ -341,27 +377,28 @@ struct SplitEval {
       cell_body(xy, zm, n01, n23, n45, e2, t1x, t1y, t1z, a1x, a1y, a1z);
     }
     pend += (nrec + ng - 1) / ng;
-    if (pend >= kFlushTerms) flush(), pend = 0;
+    if (pend >= kFlushTerms) flush();
     __syncwarp();
   }
 
-  // direct particles: particle indices ring[(head + i) % kPartQ], i < cnt <= kPartBatch
-  __device__ void parts(const uint32_t* ring, uint32_t head, int cnt) {
-    float* st = reinterpret_cast<float*>(stage);
+  // direct particles: particle indices ring[0 .. cnt), cnt <= kPartBatch
+  __device__ __forceinline__ void parts(const uint32_t* ring, int cnt) {
+    float* st = reinterpret_cast<float*>(S.stage);
     const int rounded = (cnt + 1) & ~1;
+    const double cx = S.centre[0], cy = S.centre[1], cz = S.centre[2], scale = S.scale;
     for (int i = lane; i < rounded; i += 32) {
       float* r = st + 4 * (i >> 1) + (i & 1);
       float4 v = make_float4(kFarAway, 0.f, 0.f, 0.f);
       if (i < cnt) {
-        const double4 p = a.pm[ring[(head + (uint32_t)i) & (kPartQ - 1)]];
+        const double4 p = a.pm[ring[i]];
         v = make_float4((float)(__dsub_rn(p.x, cx) * scale), (float)(__dsub_rn(p.y, cy) * scale),
                         (float)(__dsub_rn(p.z, cz) * scale), (float)p.w);
       }
       r[0] = v.x, r[2] = v.y, r[4 * kPartPlane] = v.z, r[4 * kPartPlane + 2] = v.w;
     }
     __syncwarp();
-    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(stage);
-    const f2 e2 = f2_pack(eps2, eps2);
+    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(S.stage);
+    const f2 e2 = twice(S.eps2);
     const int nrec = rounded >> 1;
     for (int s = first; s < nrec; s += ng) {
       const ulonglong2 xy = rec[s], zm = rec[kPartPlane + s];
@@ -369,497 +406,348 @@ struct SplitEval {
       part_body(xy, zm, e2, t1x, t1y, t1z, a1x, a1y, a1z);
     }
     pend += (nrec + ng - 1) / ng;
-    if (pend >= kFlushTerms) flush(), pend = 0;
+    if (pend >= kFlushTerms) flush();
     __syncwarp();
   }
 
-  // After a walk: the lane groups' sums, added in group order into every
-  // target's FP64 sum.
-  __device__ void finish() {
-    if (pend) flush(), pend = 0;
-    if (first < (1 << 30)) {
-      double* r = red + 6 * lane;
-      r[0] = s0x, r[1] = s0y, r[2] = s0z, r[3] = s1x, r[4] = s1y, r[5] = s1z;
-    }
+  // After a list: the lane groups' sums, added in group order into the
+  // targets' FP64 sums out[0 .. n).
+  __device__ __forceinline__ void finish(int n, double (*out)[3]) {
+    if (pend) flush();
     __syncwarp();
-    for (int t = lane; t < tb; t += 32) {
-      const int k = t / lpg, sl = t - k * lpg;
-      double x = 0.0, y = 0.0, z = 0.0;
-      for (int g = 0; g < ng; ++g) {
-        const double* r = red + 6 * (g * lpg + sl) + 3 * k;
-        x += r[0], y += r[1], z += r[2];
-      }
-      acc[t][0] += x, acc[t][1] += y, acc[t][2] += z;
-    }
-    __syncwarp();
+    add_group_sums(S, lane, n, (n + 1) >> 1, ng, out);
   }
 };
 
-// Plain FP64, up to 2 targets per lane, up to 64 per warp.  Absolute FP64
-// positions; the formula of accel_from_source with multiplications by 1/r^2
-// in place of its divisions.
+// Plain FP64: the same lane layout and lists; absolute positions, the formula
+// of accel_from_source with multiplications by 1/r^2 in place of its
+// divisions.
 template <bool QUAD, bool MASK>
 struct F64Eval {
-  static constexpr int TB = 2;
+  static constexpr int kCellBatch = 32, kPartBatch = 64;
+  static constexpr int kBlocksPerSm = 4;
+  // planes of double2 per source: (x, y) (z, m) (q0, q1) (q2, q3) (q4, q5)
+  static_assert(5 * 16 * kCellBatch <= kStageBytes && 2 * 16 * kPartBatch <= kStageBytes && kPartBatch + 31 < kRing,
+                "batches too large");
   const WalkArgs& a;
-  double cx, cy, cz;  // unused: absolute positions
-  double eps2;
-  int L, gp, g, j, kmax;
-  double tx[TB], ty[TB], tz[TB];
-  double ax[TB], ay[TB], az[TB];
-  double (*acc)[3];
-  int ntb;
+  WarpSmem& S;
+  int lane, ng, first;
+  double t0x, t0y, t0z, t1x, t1y, t1z;
+  double a0x, a0y, a0z, a1x, a1y, a1z;
 
-  __device__ F64Eval(const WalkArgs& args, float4*, int) : a(args) {}
-
-  __device__ int cell_chunk() const { return 2 * L; }
-  __device__ int part_chunk() const { return 2 * L; }
-  __device__ void set_system(double eps2_, double) { eps2 = eps2_; }
-
-  static __device__ int groups_for(int tb) {
-    return tb <= 2 ? 1 : tb <= 4 ? 2 : tb <= 8 ? 4 : tb <= 16 ? 8 : tb <= 32 ? 16 : 32;
+  __device__ F64Eval(const WalkArgs& args, WarpSmem& S_, int lane_, double eps2_, double)
+      : a(args), S(S_), lane(lane_) {
+    S.eps2 = eps2_;
   }
 
-  __device__ void setup(int lane, uint32_t p0, int tb, double (*sums)[3]) {
-    acc = sums;
-    ntb = tb;
-    gp = groups_for(tb);
-    L = 32 / gp;
-    g = lane / L;
-    j = lane & (L - 1);
-    kmax = (tb + gp - 1) / gp;
-    double p0x = 0, p0y = 0, p0z = 0, p1x = 0, p1y = 0, p1z = 0;
-    if (lane < tb) {
-      const double4 q = a.pm[p0 + lane];
-      p0x = q.x, p0y = q.y, p0z = q.z;
-    }
-    if (lane + 32 < tb) {
-      const double4 q = a.pm[p0 + 32 + lane];
-      p1x = q.x, p1y = q.y, p1z = q.z;
-    }
-#pragma unroll
-    for (int k = 0; k < TB; ++k) {
-      const int t = g + k * gp;
-      const double x0 = __shfl_sync(kFull, p0x, t & 31), x1 = __shfl_sync(kFull, p1x, t & 31);
-      const double y0 = __shfl_sync(kFull, p0y, t & 31), y1 = __shfl_sync(kFull, p1y, t & 31);
-      const double z0 = __shfl_sync(kFull, p0z, t & 31), z1 = __shfl_sync(kFull, p1z, t & 31);
-      tx[k] = t < 32 ? x0 : x1;
-      ty[k] = t < 32 ? y0 : y1;
-      tz[k] = t < 32 ? z0 : z1;
-      ax[k] = ay[k] = az[k] = 0.0;
-    }
+  __device__ void setup(uint32_t p0, int n, double, double, double) {
+    const int lpg = (n + 1) >> 1;
+    ng = 32 / lpg;
+    first = lane < lpg * ng ? lane / lpg : 1 << 30;
+    const int t0 = lane % lpg, t1 = t0 + lpg < n ? t0 + lpg : t0;
+    const double4 q0 = a.pm[p0 + t0], q1 = a.pm[p0 + t1];
+    t0x = q0.x, t0y = q0.y, t0z = q0.z;
+    t1x = q1.x, t1y = q1.y, t1z = q1.z;
+    a0x = a0y = a0z = a1x = a1y = a1z = 0.0;
   }
 
-  __device__ __forceinline__ void cell_one(int k, double sx, double sy, double sz, double m, const double q[6],
-                                           double& rx, double& ry, double& rz) {
-    const double dx = sx - tx[k], dy = sy - ty[k], dz = sz - tz[k];
+  __device__ __forceinline__ void cell_body(double2 xy, double2 zm, double2 q01, double2 q23, double2 q45, double eps2,
+                                            double tx, double ty, double tz, double& ax, double& ay, double& az) const {
+    const double dx = xy.x - tx, dy = xy.y - ty, dz = zm.x - tz;
     const double r2 = dx * dx + dy * dy + dz * dz + eps2;
     double ri = rsqrt(r2);
     if (!QUAD && MASK) ri = r2 > 0.0 ? ri : 0.0;
     const double ri2 = ri * ri;
     const double ri3 = ri * ri2;
     if (QUAD) {
-      const double qx = q[0] * dx + q[3] * dy + q[4] * dz;
-      const double qy = q[3] * dx + q[1] * dy + q[5] * dz;
-      const double qz = q[4] * dx + q[5] * dy + q[2] * dz;
+      const double qx = q01.x * dx + q23.y * dy + q45.x * dz;
+      const double qy = q23.y * dx + q01.y * dy + q45.y * dz;
+      const double qz = q45.x * dx + q45.y * dy + q23.x * dz;
       const double dqd = dx * qx + dy * qy + dz * qz;
       const double ri5 = ri3 * ri2;
-      const double c = m * ri3 + 2.5 * dqd * (ri5 * ri2);
-      rx = c * dx - ri5 * qx;
-      ry = c * dy - ri5 * qy;
-      rz = c * dz - ri5 * qz;
+      const double c = zm.y * ri3 + 2.5 * dqd * (ri5 * ri2);
+      ax += c * dx - ri5 * qx;
+      ay += c * dy - ri5 * qy;
+      az += c * dz - ri5 * qz;
     } else {
-      const double c = m * ri3;
-      rx = c * dx, ry = c * dy, rz = c * dz;
+      const double c = zm.y * ri3;
+      ax += c * dx, ay += c * dy, az += c * dz;
     }
   }
 
-  __device__ __forceinline__ void load_cell(const uint32_t* ring, uint32_t at, bool live, double& sx, double& sy,
-                                            double& sz, double& m, double q[6]) {
-    sx = 1.0e30, sy = sz = m = 0.0;
-    q[0] = q[1] = q[2] = q[3] = q[4] = q[5] = 0.0;
-    if (live) {
-      const uint32_t n = ring[at & (kCellQ - 1)];
-      const double4 cm = a.mom[n];
-      sx = cm.x, sy = cm.y, sz = cm.z, m = cm.w;
-      if (QUAD) {
-        const double* qq = a.q64 + (size_t)n * 6;
-#pragma unroll
-        for (int t = 0; t < 6; ++t) q[t] = qq[t];
-      }
-    }
-  }
-
-  __device__ void cells(const uint32_t* ring, uint32_t head, int cnt) {
-    double s0x, s0y, s0z, m0, q0[6], s1x, s1y, s1z, m1, q1[6];
-    load_cell(ring, head + j, j < cnt, s0x, s0y, s0z, m0, q0);
-    load_cell(ring, head + L + j, L + j < cnt, s1x, s1y, s1z, m1, q1);
-#pragma unroll
-    for (int k = 0; k < TB; ++k) {
-      if (k < kmax) {
-        double ax0, ay0, az0, ax1, ay1, az1;
-        cell_one(k, s0x, s0y, s0z, m0, q0, ax0, ay0, az0);
-        cell_one(k, s1x, s1y, s1z, m1, q1, ax1, ay1, az1);
-        ax[k] += ax0 + ax1;
-        ay[k] += ay0 + ay1;
-        az[k] += az0 + az1;
-      }
-    }
-  }
-
-  __device__ __forceinline__ void part_one(int k, double sx, double sy, double sz, double m, double& rx, double& ry,
-                                           double& rz) {
-    const double dx = sx - tx[k], dy = sy - ty[k], dz = sz - tz[k];
+  __device__ __forceinline__ void part_body(double2 xy, double2 zm, double eps2, double tx, double ty, double tz, double& ax,
+                                            double& ay, double& az) const {
+    const double dx = xy.x - tx, dy = xy.y - ty, dz = zm.x - tz;
     const double r2 = dx * dx + dy * dy + dz * dz + eps2;
     double ri = rsqrt(r2);
     if (MASK) ri = r2 > 0.0 ? ri : 0.0;
-    const double c = m * (ri * ri) * ri;
-    rx = c * dx, ry = c * dy, rz = c * dz;
+    const double c = zm.y * (ri * ri) * ri;
+    ax += c * dx, ay += c * dy, az += c * dz;
   }
 
-  __device__ void parts(const uint32_t* ring, uint32_t head, int cnt) {
-    double s0x = 1.0e30, s0y = 0, s0z = 0, m0 = 0, s1x = 1.0e30, s1y = 0, s1z = 0, m1 = 0;
-    if (j < cnt) {
-      const double4 p = a.pm[ring[(head + j) & (kPartQ - 1)]];
-      s0x = p.x, s0y = p.y, s0z = p.z, m0 = p.w;
-    }
-    if (L + j < cnt) {
-      const double4 p = a.pm[ring[(head + L + j) & (kPartQ - 1)]];
-      s1x = p.x, s1y = p.y, s1z = p.z, m1 = p.w;
-    }
-#pragma unroll
-    for (int k = 0; k < TB; ++k) {
-      if (k < kmax) {
-        double ax0, ay0, az0, ax1, ay1, az1;
-        part_one(k, s0x, s0y, s0z, m0, ax0, ay0, az0);
-        part_one(k, s1x, s1y, s1z, m1, ax1, ay1, az1);
-        ax[k] += ax0 + ax1;
-        ay[k] += ay0 + ay1;
-        az[k] += az0 + az1;
-      }
-    }
-  }
-
-  __device__ void finish() {
-#pragma unroll
-    for (int k = 0; k < TB; ++k) {
-      if (k < kmax) {
-        double vx = ax[k], vy = ay[k], vz = az[k];
-        for (int o = L >> 1; o > 0; o >>= 1) {
-          vx += __shfl_xor_sync(kFull, vx, o);
-          vy += __shfl_xor_sync(kFull, vy, o);
-          vz += __shfl_xor_sync(kFull, vz, o);
-        }
-        const int t = g + k * gp;
-        if (j == (k & (L - 1)) && t < ntb) {
-          acc[t][0] += vx;
-          acc[t][1] += vy;
-          acc[t][2] += vz;
-        }
+  __device__ __forceinline__ void cells(const uint32_t* ring, int cnt) {
+    double2* rec = reinterpret_cast<double2*>(S.stage);
+    if (lane < cnt) {
+      const uint32_t n = ring[lane];
+      const double2* cm = reinterpret_cast<const double2*>(a.mom + n);
+      rec[lane] = cm[0], rec[kCellBatch + lane] = cm[1];
+      if (QUAD) {
+        const double2* q = reinterpret_cast<const double2*>(a.q64 + (size_t)n * 6);
+        rec[2 * kCellBatch + lane] = q[0], rec[3 * kCellBatch + lane] = q[1], rec[4 * kCellBatch + lane] = q[2];
       }
     }
     __syncwarp();
+    const double e2 = S.eps2;
+    for (int s = first; s < cnt; s += ng) {
+      const double2 xy = rec[s], zm = rec[kCellBatch + s];
+      double2 q01 = {}, q23 = {}, q45 = {};
+      if (QUAD) q01 = rec[2 * kCellBatch + s], q23 = rec[3 * kCellBatch + s], q45 = rec[4 * kCellBatch + s];
+      cell_body(xy, zm, q01, q23, q45, e2, t0x, t0y, t0z, a0x, a0y, a0z);
+      cell_body(xy, zm, q01, q23, q45, e2, t1x, t1y, t1z, a1x, a1y, a1z);
+    }
+    __syncwarp();
+  }
+
+  __device__ __forceinline__ void parts(const uint32_t* ring, int cnt) {
+    double2* rec = reinterpret_cast<double2*>(S.stage);
+    for (int i = lane; i < cnt; i += 32) {
+      const double2* p = reinterpret_cast<const double2*>(a.pm + ring[i]);
+      rec[i] = p[0], rec[kPartBatch + i] = p[1];
+    }
+    __syncwarp();
+    const double e2 = S.eps2;
+    for (int s = first; s < cnt; s += ng) {
+      const double2 xy = rec[s], zm = rec[kPartBatch + s];
+      part_body(xy, zm, e2, t0x, t0y, t0z, a0x, a0y, a0z);
+      part_body(xy, zm, e2, t1x, t1y, t1z, a1x, a1y, a1z);
+    }
+    __syncwarp();
+  }
+
+  __device__ __forceinline__ void finish(int n, double (*out)[3]) {
+    S.sums[0][lane] = a0x, S.sums[1][lane] = a0y, S.sums[2][lane] = a0z;
+    S.sums[3][lane] = a1x, S.sums[4][lane] = a1y, S.sums[5][lane] = a1z;
+    __syncwarp();
+    add_group_sums(S, lane, n, (n + 1) >> 1, ng, out);
   }
 };
 
 // ---------------------------------------------------------------------------
-// Source queues shared by every traversal below.  Accepted cells go to a ring
-// of node ids and opened leaves' particles to a ring of particle indices; a
-// full ring (or the end of the walk) is evaluated as one batch.  A loop
-// iteration does exactly one thing: evaluate a cell batch, evaluate a
-// particle batch, enqueue up to 32 particles of the leaves opened last, or
-// let the producer (a traversal step, a list scan) add sources.  The
-// evaluators are reached from this one place each (their bodies would
-// otherwise be inlined many times over).
+// The shared walk of a group of k <= kMaxTargets targets, in the spirit of
+// GroupWalker::visit (grouped_ttg.h:204-289) taken to every level: one
+// traversal from the root whose stack entries (runs of sibling nodes) carry
+// the mask of targets that still need them.  Each popped node is first tested
+// against the group's particle box: accepted there (mac_accept_bbox) ->
+// accepted by every target in the mask; rejected for every point of it
+// (mac_reject_all, multipole.h:158-160) -> opened by every target in the
+// mask; otherwise each target tests its own box: lane t + k * r holds target
+// t's box and tests the r-th of the 32 / k nodes taken at a time.  A node
+// taken by every target of the group goes to the dense list, one taken by
+// some to the partial list with its mask; opened interior nodes push their
+// children with the mask of the targets that opened them.  Every target's
+// list is exactly what a walk of its own box from the root gives
+// (multipole.h's tests are monotone in the box).
+// The traversal only writes lists.  Without the evaluators' registers and
+// queues beside it the kernel runs 24 warps per SM (80 registers, 9.3 KB of
+// shared memory per warp) instead of 16, and each part is a loop of its own:
+// walk per evaluation 30.5 to 23.2 ms at 4M, 7.39 to 5.80 at 1M, 1.89 to 1.46
+// at 262k (leaf 16, theta 0.5); in FP64 12.8 to 9.5 ms at 1M.  With 5 blocks
+// of 4 warps per SM 23.8 ms at 4M, with 4 25.1.
 
-struct Queues {
-  uint32_t chead = 0, phead = 0;
-  int ncell = 0, npart = 0;
-  // particles of the leaves opened by the last producer step, still to enqueue
-  uint32_t ptot = 0, pbase = 0, pinc = 0, pc = 0, pfirst = 0;
-  unsigned long long ncells = 0, nparts = 0;  // sources evaluated
-};
-
-// Appends the lanes' accepted cells (one per lane where `take`).
-__device__ __forceinline__ void push_cells(WarpSmem& S, Queues& q, bool take, uint32_t node, uint32_t lt) {
-  const uint32_t am = __ballot_sync(kFull, take);
-  if (take) S.cell[(q.chead + q.ncell + __popc(am & lt)) & (kCellQ - 1)] = node;
-  q.ncell += __popc(am);
-}
-
-// Records the lanes' opened leaves (cnt particles from `first`; cnt 0 = none):
-// their particles are enqueued by the next loop iterations.
-__device__ __forceinline__ void open_leaves(Queues& q, uint32_t cnt, uint32_t first, int lane) {
-  q.pc = cnt;
-  q.pinc = warp_incl_scan_u32(cnt, lane);
-  q.ptot = __shfl_sync(kFull, q.pinc, 31);
-  q.pbase = 0;
-  q.pfirst = first;
-}
-
-// One iteration's queue work; returns false when the producer should run
-// (queues below a batch and no particles left to enqueue), true otherwise.
-// `more`: the producer has more to add.
-template <class E>
-__device__ __forceinline__ bool drain_step(E& ev, WarpSmem& S, Queues& q, bool more, int lane) {
-  const bool done = !more && q.pbase >= q.ptot;
-  const int C = ev.cell_chunk(), CP = ev.part_chunk();
-  if (q.ncell >= C || (done && q.ncell > 0)) {
-    const int c = min(q.ncell, C);
-    ev.cells(S.cell, q.chead, c);
-    q.chead += c;
-    q.ncell -= c;
-    q.ncells += c;
-    return true;
-  }
-  if (q.npart >= CP || (done && q.npart > 0)) {
-    const int c = min(q.npart, CP);
-    ev.parts(S.part, q.phead, c);
-    q.phead += c;
-    q.npart -= c;
-    q.nparts += c;
-    return true;
-  }
-  if (q.pbase < q.ptot) {  // enqueue up to 32 particles of the opened leaves
-    const uint32_t idx = q.pbase + lane;
-    uint32_t src = 0;
-#pragma unroll
-    for (int step = 16; step >= 1; step >>= 1) {
-      const uint32_t v = __shfl_sync(kFull, q.pinc, (src + step - 1) & 31);
-      if (v <= idx) src += step;
-    }
-    src = min(src, 31u);
-    const uint32_t sf = __shfl_sync(kFull, q.pfirst, src);
-    const uint32_t sinc = __shfl_sync(kFull, q.pinc, src);
-    const uint32_t spc = __shfl_sync(kFull, q.pc, src);
-    const uint32_t take = min(32u, q.ptot - q.pbase);
-    if ((uint32_t)lane < take) S.part[(q.phead + q.npart + lane) & (kPartQ - 1)] = sf + (idx - (sinc - spc));
-    q.npart += take;
-    q.pbase += take;
-    __syncwarp();
-    return true;
-  }
-  return false;
-}
-
-// ---------------------------------------------------------------------------
-// Walk of one target's particle box from the root (the reference's
-// per-target list): accepted -> cells, otherwise opened (leaves contribute
-// their particles, interior nodes push their children).  Used for targets of
-// more than kGroupMax particles (in batches of kGroupMax targets) and for the
-// targets of a group whose shared walk outgrew its list.  Returns 1 if the
-// stack would overflow (redo popping one node at a time, which bounds it).
-
-template <class E>
-__device__ __forceinline__ int target_walk(E& ev, const WalkArgs& a, WarpSmem& S, uint32_t root, const double lo[3],
-                                           const double hi[3], double theta2, bool dfs, int lane, Queues& q) {
-  const uint32_t lt = lanemask_lt();
-  if (lane == 0) S.snode[0] = root;
-  uint32_t top = 1;
-  __syncwarp();
-  q = Queues();
-  // a walk pops each node at most once: more steps than nodes means a corrupt tree
-  uint32_t steps = 0;
-  const uint32_t max_steps = a.st->n_nodes + 2;
-  for (;;) {
-    if (drain_step(ev, S, q, top > 0, lane)) continue;
-    if (top == 0) break;
-    if (++steps > max_steps) {
-      if (lane == 0) atomicOr(&a.st->status, kStWalkLimit);
-      top = 0;
-      continue;
-    }
-    const uint32_t n = dfs ? 1u : min(top, 32u);
-    top -= n;
-    const bool valid = (uint32_t)lane < n;
-    const uint32_t node = valid ? S.snode[top + lane] : 0u;
-    __syncwarp();
-    bool accept = false, leaf = false;
-    uint32_t first = 0, cnt = 0, info = 0;
-    if (valid) {
-      const WNode* w = a.w + node;
-      const double4 c4 = *reinterpret_cast<const double4*>(&w->cx);  // com xyz, edge^2
-      const uint4 u4 = *reinterpret_cast<const uint4*>(&w->first);   // first, count, info, mass
-      first = u4.x, cnt = u4.y, info = u4.z;
-      leaf = info_leaf(info);
-      // mac_accept_bbox: theta^2 * near^2 > edge^2 (multipole.h:151-153)
-      accept = __dmul_rn(theta2, near2(lo, hi, c4.x, c4.y, c4.z)) > c4.w;
-    }
-    push_cells(S, q, accept, node, lt);
-    const uint32_t nch = (valid && !accept && !leaf) ? info_nchild(info) : 0u;
-    const uint32_t cinc = warp_incl_scan_u32(nch, lane);
-    const uint32_t ctot = __shfl_sync(kFull, cinc, 31);
-    if (top + ctot > (uint32_t)kStackCap) return 1;
-    for (uint32_t k = 0; k < nch; ++k) S.snode[top + cinc - nch + k] = first + k;
-    top += ctot;
-    open_leaves(q, (valid && !accept && leaf) ? cnt : 0u, first, lane);
-    __syncwarp();
-  }
-  __syncwarp();
-  return 0;
-}
-
-// ---------------------------------------------------------------------------
-// The shared walk of a group of k <= kMaxTargets targets (particles p0 ..
-// p0 + np - 1, np <= kGroupMax), in the spirit of GroupWalker::visit
-// (grouped_ttg.h:204-289) taken to every level: one traversal from the root
-// whose stack entries carry the mask of targets that still need the node.
-// Each popped node is first tested against the group's particle box:
-// accepted there (mac_accept_bbox) -> accepted by every target in the mask;
-// rejected for every point of it (mac_reject_all, multipole.h:158-160) ->
-// opened by every target in the mask; otherwise each target in the mask
-// tests its own box, one (node, target) pair per lane.  A node taken by every
-// target of the group goes to the group queues and is evaluated once against
-// all np particles; one taken by some targets only goes to the warp's list as
-// (node, mask) for the targets' own passes (target_pass).  Opened interior
-// nodes push their children with the mask of the targets that opened them.
-// Every target's list is exactly what a walk of its own box from the root
-// gives (multipole.h's tests are monotone in the box).
-// Returns 0, 1 (stack overflow: redo popping one node at a time) or 2 (list
-// overflow: the targets walk on their own).
-
-template <class E>
-__device__ __forceinline__ int group_walk(E& ev, const WalkArgs& a, WarpSmem& S, uint32_t root, uint32_t k,
-                                          double theta2, bool dfs, int lane, uint2* list, uint32_t& nlist, Queues& q) {
+// Returns true when a list may be too full for another step (the lists are
+// then to be taken and reset, and the traversal goes on where it stopped).
+__device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double theta2, uint2* __restrict__ dl,
+                                         uint2* __restrict__ pl, int lane) {
+  const uint32_t k = S.job.k;
+  Walk w = S.job.w;
   const uint32_t lt = lanemask_lt();
   const uint32_t full = (1u << k) - 1u;  // k <= kMaxTargets < 32
-  if (lane == 0) S.snode[0] = root, S.smask[0] = full;
-  uint32_t top = 1;
-  __syncwarp();
-  q = Queues();
-  nlist = 0;
-  uint32_t steps = 0;
-  const uint32_t max_steps = a.st->n_nodes + 2;
-  for (;;) {
-    if (drain_step(ev, S, q, top > 0, lane)) continue;
-    if (top == 0) break;
-    if (++steps > max_steps) {
-      if (lane == 0) atomicOr(&a.st->status, kStWalkLimit);
-      top = 0;
-      continue;
+  StepScratch& X = *reinterpret_cast<StepScratch*>(S.stage);
+  const uint32_t per = 32u / k, sub = (uint32_t)lane / k, tgt = (uint32_t)lane - sub * k;
+  double lo[3], hi[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) lo[d] = S.tlo[tgt][d], hi[d] = S.thi[tgt][d];
+  const uint32_t max_steps = a.st->n_nodes + 2;  // a walk pops each node at most once
+  bool more = false;
+  while (w.top) {
+    if (w.ndc + w.ndr + 32 > kDenseCap || w.npc + w.npr + 64 > kListCap) {
+      more = true;
+      break;
     }
-    // pop up to 32 entries, fewer when the stack is nearly full (each popped
-    // node pushes at most 8)
-    uint32_t n = dfs ? 1u : min(top, 32u);
-    if (!dfs) n = min(n, max((kStackCap - top) / 7u, 1u));
-    top -= n;
+    if (++w.steps > max_steps) {  // a corrupt tree
+      if (lane == 0) atomicOr(&a.st->status, kStWalkLimit);
+      w.top = 0;
+      break;
+    }
+    // pop up to 32 nodes off the top runs: lane i looks at the i-th run from the top
+    const uint32_t have = min(w.top, 32u);
+    uint2 ent = make_uint2(0u, 0u);
+    if ((uint32_t)lane < have) ent = S.stack[w.top - 1 - lane];
+    const uint32_t c = ent.y >> 24;
+    const uint32_t inc = warp_incl_scan_u32(c, lane), excl = inc - c;
+    const uint32_t room = (uint32_t)kStackCap - (kLevels + 1);
+    uint32_t n = min(__shfl_sync(kFull, inc, 31), 32u);
+    n = min(n, w.top < room ? room - w.top : 1u);
+    // the run holding node slot `lane`: the runs' first slots as bits, counted up to the lane
+    const uint32_t heads = __reduce_or_sync(kFull, (c && excl < 32u) ? 1u << excl : 0u);
+    const uint32_t run = (uint32_t)__popc(heads & (lt | (1u << lane))) - 1u;
+    const uint32_t node = __shfl_sync(kFull, ent.x - excl, run) + (uint32_t)lane;
+    const uint32_t mask = __shfl_sync(kFull, ent.y, run) & kMaskBits;
     const bool valid = (uint32_t)lane < n;
-    uint32_t node = 0, mask = 0;
-    if (valid) node = S.snode[top + lane], mask = S.smask[top + lane];
+    const uint32_t done = (uint32_t)__popc(__ballot_sync(kFull, c && inc <= n));
     __syncwarp();
+    if (c && excl < n && n < inc) S.stack[w.top - 1 - lane] = make_uint2(ent.x + (n - excl), ent.y - ((n - excl) << 24));
+    w.top -= done;
     double4 c4 = make_double4(0.0, 0.0, 0.0, 0.0);
     uint4 u4 = make_uint4(0u, 0u, 0u, 0u);
     bool acc = false, rej = false;
     if (valid) {
-      const WNode* w = a.w + node;
-      c4 = *reinterpret_cast<const double4*>(&w->cx);
-      u4 = *reinterpret_cast<const uint4*>(&w->first);
+      const WNode* wn = a.w + node;
+      c4 = *reinterpret_cast<const double4*>(&wn->cx);  // com xyz, edge^2
+      u4 = *reinterpret_cast<const uint4*>(&wn->first);  // first, count, info, mass
+      // mac_accept_bbox: theta^2 * near^2 > edge^2 (multipole.h:151-153)
       acc = __dmul_rn(theta2, near2(S.glo, S.ghi, c4.x, c4.y, c4.z)) > c4.w;
       // one target: its box is the group's, so not accepted means opened
       if (!acc) rej = k == 1 || __dmul_rn(theta2, far2(S.glo, S.ghi, c4.x, c4.y, c4.z)) <= c4.w;
     }
     uint32_t A = acc ? mask : 0u, O = rej ? mask : 0u;
-    // undecided nodes: every target in the mask tests its own box
+    // undecided nodes: every target tests its own box
     const bool und = valid && !acc && !rej;
-    const uint32_t pcnt = und ? (uint32_t)__popc(mask) : 0u;
-    const uint32_t pincl = warp_incl_scan_u32(pcnt, lane);
-    const uint32_t ptotal = __shfl_sync(kFull, pincl, 31);
-    if (ptotal) {
-      S.accbits[lane] = 0u;
+    const uint32_t um = __ballot_sync(kFull, und);
+    if (um) {
+      const uint32_t rank = (uint32_t)__popc(um & lt), nu = (uint32_t)__popc(um);
+      if (und) X.node[rank] = c4;
       __syncwarp();
-      for (uint32_t base = 0; base < ptotal; base += 32) {
-        const uint32_t j = base + (uint32_t)lane;
-        // the entry holding pair j: the first lane whose inclusive count exceeds j
-        uint32_t e = 0;
-#pragma unroll
-        for (int st = 16; st >= 1; st >>= 1) {
-          const uint32_t v = __shfl_sync(kFull, pincl, (e + st - 1) & 31);
-          if (v <= j) e += st;
+      for (uint32_t base = 0; base < nu; base += per) {
+        const uint32_t e = base + sub;
+        bool ok = false;
+        if (sub < per && e < nu) {
+          const double4 q = X.node[e];
+          ok = __dmul_rn(theta2, near2(lo, hi, q.x, q.y, q.z)) > q.w;
         }
-        e = min(e, 31u);
-        const uint32_t einc = __shfl_sync(kFull, pincl, e), ecnt = __shfl_sync(kFull, pcnt, e);
-        uint32_t em = __shfl_sync(kFull, mask, e);
-        const double ex = __shfl_sync(kFull, c4.x, e), ey = __shfl_sync(kFull, c4.y, e);
-        const double ez = __shfl_sync(kFull, c4.z, e), ee = __shfl_sync(kFull, c4.w, e);
-        if (j < ptotal) {
-          // target t: the r-th set bit of the entry's mask
-          uint32_t r = j - (einc - ecnt), t = 0;
-#pragma unroll
-          for (int wdt = 16; wdt >= 1; wdt >>= 1) {
-            const uint32_t low = (uint32_t)__popc(em & ((1u << wdt) - 1u));
-            if (r >= low) r -= low, em >>= wdt, t += wdt;
-          }
-          if (__dmul_rn(theta2, near2(S.tlo[t], S.thi[t], ex, ey, ez)) > ee) atomicOr(&S.accbits[e], 1u << t);
-        }
+        const uint32_t bits = __ballot_sync(kFull, ok);
+        if (tgt == 0 && sub < per && e < nu) X.accepts[e] = (bits >> (sub * k)) & full;
       }
       __syncwarp();
-      if (und) A = S.accbits[lane], O = mask & ~A;
-      __syncwarp();
+      if (und) A = X.accepts[rank] & mask, O = mask & ~A;
     }
     const bool leaf = valid && info_leaf(u4.z);
-    // sources every target takes: the group queues
-    push_cells(S, q, A != 0u && A == full, node, lt);
-    // sources some targets take: the list
-    const bool cpart = A != 0u && A != full, lpart = leaf && O != 0u && O != full;
-    const uint32_t runs = lpart ? (u4.y + kMaxRun - 1) / kMaxRun : 0u;
-    const uint32_t nl = (cpart ? 1u : 0u) + runs;
-    const uint32_t linc = warp_incl_scan_u32(nl, lane);
-    const uint32_t ltot = __shfl_sync(kFull, linc, 31);
-    if (nlist + ltot > kListCap) return 2;
-    uint32_t at = nlist + linc - nl;
-    if (cpart) list[at++] = make_uint2(node, A);
-    for (uint32_t r = 0; r < runs; ++r) {
-      const uint32_t c = min(kMaxRun, u4.y - r * kMaxRun);
-      list[at++] = make_uint2((u4.x + r * kMaxRun) | kLeafBit, O | (c << kCountShift));
-    }
-    nlist += ltot;
-    // opened interior nodes: children, with the targets that opened them
-    const uint32_t nch = (O != 0u && !leaf) ? info_nchild(u4.z) : 0u;
-    const uint32_t cinc = warp_incl_scan_u32(nch, lane);
-    const uint32_t ctot = __shfl_sync(kFull, cinc, 31);
-    if (top + ctot > (uint32_t)kStackCap) return 1;
-    for (uint32_t c = 0; c < nch; ++c) S.snode[top + cinc - nch + c] = u4.x + c, S.smask[top + cinc - nch + c] = O;
-    top += ctot;
-    // leaves every target opens: their particles, for the group queues
-    open_leaves(q, (leaf && O == full) ? u4.y : 0u, u4.x, lane);
+    // cells every target takes, some take
+    const bool dc = A != 0u && A == full, pc = A != 0u && A != full;
+    uint32_t m = __ballot_sync(kFull, dc);
+    if (dc) dl[w.ndc + __popc(m & lt)] = make_uint2(node, 1u);
+    w.ndc += __popc(m);
+    m = __ballot_sync(kFull, pc);
+    if (pc) pl[w.npc + __popc(m & lt)] = make_uint2(node, A);
+    w.npc += __popc(m);
+    // leaves every target opens, some open
+    const bool dr = leaf && O == full, pr = leaf && O != 0u && O != full;
+    m = __ballot_sync(kFull, dr);
+    if (dr) dl[kDenseCap - 1u - (w.ndr + __popc(m & lt))] = make_uint2(u4.x, u4.y);
+    w.ndr += __popc(m);
+    m = __ballot_sync(kFull, pr);
+    if (pr)
+      pl[kListCap - 1u - (w.npr + __popc(m & lt))] =
+          u4.y < kByNode ? make_uint2(u4.x, O | (u4.y << kCountShift)) : make_uint2(node, O | (kByNode << kCountShift));
+    w.npr += __popc(m);
+    // opened interior nodes: their children, with the targets that opened them
+    const bool in = O != 0u && !leaf;
+    m = __ballot_sync(kFull, in);
+    if (in) S.stack[w.top + __popc(m & lt)] = make_uint2(u4.x, O | (info_nchild(u4.z) << 24));
+    w.top += __popc(m);
     __syncwarp();
   }
-  __syncwarp();
-  return 0;
+  S.job.w = w;
+  return more;
 }
 
-// Target `bit` of the group takes, from the list, the entries whose mask
-// holds it: cells into its cell queue, leaves' particles into its particle
-// queue; evaluated with the evaluator set up for its particles.  The scan
-// moves a window of 32 entries at a time and skips windows without an entry
-// for the target.
+// Evaluates the entries of a two-ended list that `sel` picks (bits of the
+// entry's second word; dense lists: any) on the evaluator's targets: cells
+// list[0 .. nc), runs list[cap - nr .. cap).  Windows of 32 entries, the next
+// one loaded while the current one is used, fill a ring; full batches of it
+// are evaluated.  tn: the targets.
 template <class E>
-__device__ __forceinline__ void target_pass(E& ev, const WalkArgs& a, WarpSmem& S, const uint2* list, uint32_t nlist,
-                                            uint32_t bit, int lane, Queues& q) {
+__device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S, const uint2* list, uint32_t nc,
+                                          uint32_t cap, uint32_t nr, bool dense, uint32_t sel, uint32_t tn,
+                                          int lane) {
   const uint32_t lt = lanemask_lt();
-  q = Queues();
-  uint32_t at = 0;
-  // the window after `at` is loaded one window ahead, so that its load
-  // overlaps the work on the current one
-  uint2 next = (uint32_t)lane < nlist ? list[lane] : make_uint2(0u, 0u);
+  uint32_t at = 0, held = 0;
+  uint2 next = (uint32_t)lane < nc ? list[lane] : make_uint2(0u, 0u);
   for (;;) {
-    if (drain_step(ev, S, q, at < nlist, lane)) continue;
-    if (at >= nlist) break;
-    uint2 e;
-    bool hit;
-    do {
-      e = next;
-      hit = (e.y >> bit) & 1u;
+    while (held < (uint32_t)E::kCellBatch && at < nc) {
+      const uint2 e = next;
       at += 32;
       const uint32_t j = at + (uint32_t)lane;
-      next = j < nlist ? list[j] : make_uint2(0u, 0u);
-    } while (!__any_sync(kFull, hit) && at < nlist);
-    const bool isleaf = (e.x & kLeafBit) != 0u;
-    const bool chit = hit && !isleaf, lhit = hit && isleaf;
-    if (__any_sync(kFull, chit)) push_cells(S, q, chit, e.x, lt);
-    if (__any_sync(kFull, lhit)) open_leaves(q, lhit ? e.y >> kCountShift : 0u, e.x & ~kLeafBit, lane);
+      next = j < nc ? list[j] : make_uint2(0u, 0u);
+      const bool hit = (e.y & sel) != 0u;
+      const uint32_t m = __ballot_sync(kFull, hit);
+      if (hit) S.ring[held + __popc(m & lt)] = e.x;
+      held += __popc(m);
+    }
+    if (!held) break;
+    __syncwarp();
+    const uint32_t cnt = min(held, (uint32_t)E::kCellBatch);
+    ev.cells(S.ring, (int)cnt);
+    if (lane == 0) S.ncell += cnt * tn;
+    held -= cnt;
+    if (held) {
+      const uint32_t v = S.ring[cnt + lane];  // at most 31 are left
+      __syncwarp();
+      if ((uint32_t)lane < held) S.ring[lane] = v;
+    }
   }
-  __syncwarp();
+  // runs: the particles of the picked runs of a window, 32 at a time
+  const uint2* back = list + cap - 1;
+  at = 0;
+  next = (uint32_t)lane < nr ? back[-lane] : make_uint2(0u, 0u);
+  uint32_t tot = 0, base = 0, before = 0, cnt = 0, excl = 0;
+  for (;;) {
+    while (held < (uint32_t)E::kPartBatch) {
+      if (base < tot) {
+        // the run holding particle base + lane: first particles as bits
+        const uint32_t heads =
+            __reduce_or_sync(kFull, (cnt && excl >= base && excl < base + 32u) ? 1u << (excl - base) : 0u);
+        const uint32_t run = before + (uint32_t)__popc(heads & (lt | (1u << lane))) - 1u;
+        const uint32_t take = min(32u, tot - base);
+        if ((uint32_t)lane < take) S.ring[held + lane] = S.delta[run] + base + (uint32_t)lane;
+        before += __popc(heads);
+        held += take;
+        base += 32u;
+        continue;
+      }
+      if (at >= nr) break;
+      uint2 e = next;
+      at += 32;
+      const uint32_t j = at + (uint32_t)lane;
+      next = j < nr ? back[-(int)j] : make_uint2(0u, 0u);
+      const bool hit = (e.y & sel) != 0u;
+      const uint32_t m = __ballot_sync(kFull, hit);
+      if (!m) continue;
+      cnt = hit ? (dense ? e.y : e.y >> kCountShift) : 0u;
+      if (!dense && cnt == kByNode) {
+        const WNode* wn = a.w + e.x;
+        e.x = wn->first, cnt = wn->count;
+      }
+      const uint32_t inc = warp_incl_scan_u32(cnt, lane);
+      excl = inc - cnt;
+      tot = __shfl_sync(kFull, inc, 31);
+      base = before = 0;
+      __syncwarp();
+      if (hit) S.delta[__popc(m & lt)] = e.x - excl;
+      __syncwarp();
+    }
+    if (!held) break;
+    __syncwarp();
+    const uint32_t c = min(held, (uint32_t)E::kPartBatch);
+    ev.parts(S.ring, (int)c);
+    if (lane == 0) S.npart += c * tn;
+    held -= c;
+    if (held) {
+      const uint32_t v = S.ring[c + lane];
+      __syncwarp();
+      if ((uint32_t)lane < held) S.ring[lane] = v;
+    }
+  }
 }
 
 // Bounding box of particles [b, b + T) (BBox::add, multipole.h:121-128).
@@ -880,18 +768,6 @@ __device__ __forceinline__ void particle_box(const double4* pm, uint32_t b, uint
       lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], o));
       hi[d] = fmax(hi[d], __shfl_xor_sync(kFull, hi[d], o));
     }
-  }
-}
-
-// The interaction counts of one evaluated list: quad -> cells are
-// particle-cell interactions, else monopoles counted as particle-particle.
-__device__ __forceinline__ void add_counts(const Queues& q, uint32_t targets, bool quad, unsigned long long& n_pp,
-                                      unsigned long long& n_pc) {
-  if (quad) {
-    n_pc += q.ncells * (unsigned long long)targets;
-    n_pp += q.nparts * (unsigned long long)targets;
-  } else {
-    n_pp += (q.ncells + q.nparts) * (unsigned long long)targets;
   }
 }
 
@@ -933,253 +809,210 @@ __device__ __forceinline__ uint32_t system_of(const WalkArgs& a, uint32_t p) {
   return lo;
 }
 
-// Every target of the group [t0, t1) (particles p0 .. p0 + np) walks on its
-// own from the root into S.acc (the group walk outgrew its list).
-template <class E, bool QUAD>
-__device__ void targets_alone(E& ev, const WalkArgs& a, WarpSmem& S, uint32_t root, double theta2, uint32_t k,
-                              uint32_t p0, int lane, unsigned long long& n_pp, unsigned long long& n_pc) {
-  Queues q;
-  for (uint32_t i = 0; i < k; ++i) {
-    const uint32_t tb = S.tbeg[i], tn = S.tcnt[i];
-    ev.cx = 0.5 * (S.tlo[i][0] + S.thi[i][0]), ev.cy = 0.5 * (S.tlo[i][1] + S.thi[i][1]);
-    ev.cz = 0.5 * (S.tlo[i][2] + S.thi[i][2]);
-    int r = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      ev.setup(lane, tb, (int)tn, S.acc + (tb - p0));
-      r = target_walk(ev, a, S, root, S.tlo[i], S.thi[i], theta2, attempt == 1, lane, q);
-      if (r == 0) break;
-    }
-    ev.finish();
-    add_counts(q, tn, QUAD, n_pp, n_pc);
+// The group of walk group gi: its targets, first particle and system.
+__device__ __forceinline__ void group_info(const WalkArgs& a, Job& j, uint32_t ngroups, uint32_t ntargets) {
+  const uint32_t gi = j.gi, t0 = a.groups[gi];
+  const uint32_t p0 = a.nbegin[a.targets[t0]];
+  j.t0 = t0;
+  j.k = (gi + 1 < ngroups ? a.groups[gi + 1] : ntargets) - t0;
+  j.p0 = p0;
+  j.sys = a.nsys > 1 ? system_of(a, p0) : 0u;
+}
+
+// The targets' particle ranges and boxes and the group's box; returns the
+// group's particles.
+__device__ __forceinline__ uint32_t group_boxes(const WalkArgs& a, WarpSmem& S, int lane) {
+  const Job& g = S.job;
+  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  uint32_t tb = 0, tc = 0;
+  if ((uint32_t)lane < g.k) {
+    const uint32_t tn = a.targets[g.t0 + lane];
+    tb = a.nbegin[tn], tc = a.ncount[tn];
+    S.tbeg[lane] = tb, S.tcnt[lane] = tc;
   }
-}
-
-// The group of walk group gi: its targets [t0, t1), first particle, system.
-struct GroupInfo {
-  uint32_t t0, t1, k, p0, s;
-};
-
-__device__ __forceinline__ GroupInfo group_info(const WalkArgs& a, uint32_t gi, uint32_t ngroups, uint32_t ntargets) {
-  GroupInfo g;
-  g.t0 = a.groups[gi];
-  g.t1 = gi + 1 < ngroups ? a.groups[gi + 1] : ntargets;
-  g.k = g.t1 - g.t0;
-  g.p0 = a.nbegin[a.targets[g.t0]];
-  g.s = a.nsys > 1 ? system_of(a, g.p0) : 0u;
-  return g;
-}
-
-// The second pass of the two-pass schedule (see k_walk): one warp per target
-// of a group of more than one target, once its group's shared walk has
-// finished (its list length is no longer kListPending): the group's FP64 sums
-// for its particles, then its pass over the group's list (or, if the list
-// overflowed, its own walk from the root), then the kick/drift.  A job waits
-// only for a group whose walk a running warp has taken, so every wait ends;
-// a wait is still bounded (kStSpinLimit, the job skipped).
-template <class E, bool QUAD>
-__device__ __forceinline__ void target_jobs(E& ev, const WalkArgs& a, WarpSmem& S, uint32_t ngroups, uint32_t ntargets,
-                                            int lane, Queues& q, unsigned long long& n_pp, unsigned long long& n_pc) {
-  for (;;) {
-    uint32_t ti = 0;
-    if (lane == 0) ti = atomicAdd(&a.st->walk_next2, 1u);
-    ti = __shfl_sync(kFull, ti, 0);
-    if (ti >= ntargets) break;
-    // its group: the last whose first target is at or before ti
-    uint32_t gi = 0, hi = ngroups;
-    while (hi - gi > 1) {
-      const uint32_t mid = (gi + hi) >> 1;
-      if (a.groups[mid] <= ti) gi = mid;
-      else hi = mid;
+  const uint32_t n = __shfl_sync(kFull, tb + tc, (int)g.k - 1) - g.p0;
+  if (n > (uint32_t)kGroupMax) {  // one large target
+    particle_box(a.pm, g.p0, n, lane, lo, hi);
+  } else {
+    double (*pos)[3] = reinterpret_cast<double (*)[3]>(S.stage);
+    for (uint32_t i = lane; i < n; i += 32) {
+      const double4 q = a.pm[g.p0 + i];
+      pos[i][0] = q.x, pos[i][1] = q.y, pos[i][2] = q.z;
     }
-    const GroupInfo g = group_info(a, gi, ngroups, ntargets);
-    if (g.k == 1) continue;  // done whole in the first pass
-    uint32_t nlist = ld_volatile(a.gnl + gi);
-    for (int spins = 0; nlist == kListPending && spins < kSpinLimit; ++spins) {
-      __nanosleep(128);
-      nlist = ld_volatile(a.gnl + gi);
+    __syncwarp();
+    for (uint32_t i = 0; i < tc; ++i) {
+      const double* q = pos[tb - g.p0 + i];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) lo[d] = fmin(lo[d], q[d]), hi[d] = fmax(hi[d], q[d]);
     }
-    nlist = __shfl_sync(kFull, nlist, 0);  // one value for the warp
-    if (nlist == kListPending) {
-      if (lane == 0) atomicOr(&a.st->status, kStSpinLimit);
-      continue;
-    }
-    __threadfence();  // the group's sums and list after its length
-    const uint32_t tnode = a.targets[ti];
-    const uint32_t tb = a.nbegin[tnode], tn = a.ncount[tnode];  // tn <= kGroupMax: inside a group
-    const uint32_t root = a.sys[g.s].root;
-    const SysParam& sp = a.prm[g.s];
-    ev.set_system(sp.eps2, a.sys[g.s].hw);
-    double lo[3], hi3[3];
-    particle_box(a.pm, tb, tn, lane, lo, hi3);
-    ev.cx = 0.5 * (lo[0] + hi3[0]), ev.cy = 0.5 * (lo[1] + hi3[1]), ev.cz = 0.5 * (lo[2] + hi3[2]);
-    if (nlist == kNotShared) {
-      for (uint32_t i = lane; i < tn; i += 32) S.acc[i][0] = S.acc[i][1] = S.acc[i][2] = 0.0;
-      __syncwarp();
-      int r = 0;
-      for (int attempt = 0; attempt < 2; ++attempt) {
-        ev.setup(lane, tb, (int)tn, S.acc);
-        r = target_walk(ev, a, S, root, lo, hi3, sp.theta2, attempt == 1, lane, q);
-        if (r == 0) break;
-      }
-      ev.finish();
-      add_counts(q, tn, QUAD, n_pp, n_pc);
-    } else {
-      const double* gs = a.gsum + (size_t)gi * (kGroupMax * 3) + 3 * (size_t)(tb - g.p0);
-      for (uint32_t i = lane; i < tn; i += 32) S.acc[i][0] = gs[3 * i], S.acc[i][1] = gs[3 * i + 1], S.acc[i][2] = gs[3 * i + 2];
-      __syncwarp();
-      if (nlist) {
-        ev.setup(lane, tb, (int)tn, S.acc);
-        target_pass(ev, a, S, a.wlist + (size_t)gi * kListCap, nlist, ti - g.t0, lane, q);
-        ev.finish();
-        add_counts(q, tn, QUAD, n_pp, n_pc);
-      }
-    }
-    kick_drift(a, sp, S.acc, tb, tn, lane);
   }
+  if ((uint32_t)lane < g.k) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) S.tlo[lane][d] = lo[d], S.thi[lane][d] = hi[d];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], o));
+      hi[d] = fmax(hi[d], __shfl_xor_sync(kFull, hi[d], o));
+    }
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) S.glo[d] = lo[d], S.ghi[d] = hi[d];
+  }
+  __syncwarp();
+  return n;
 }
 
-// One warp per walk group (a run of targets, k_pack_groups).  A group of one
-// target larger than kGroupMax particles walks in batches of kGroupMax
-// targets.  Otherwise: the group's shared walk with every source all its
-// targets take evaluated against all its particles, then each target's pass
-// over the list of the sources only some take, each adding its part onto the
-// group's FP64 sums in target order; then the kick/drift.
+// One warp per walk group (a run of targets, k_pack_groups): the group's
+// traversal writes its lists, then list passes evaluate them - pass 0 the
+// dense list on all the group's particles, pass 1 + i the partial list's
+// entries that target i takes on that target's particles, each pass adding
+// its part onto the group's FP64 sums - and the kick/drift follows.  When a
+// list fills up, the traversal pauses: that list's passes run (pass 0, or
+// all), and it goes on with the list empty.  A group of one target larger
+// than kGroupMax particles is walked once per kGroupMax of its particles.
 //
 // With few groups (n_groups <= a.nslots: about as many as warps, so the
 // largest group's targets would set the kernel's time) the work is cut in
-// two passes instead: the warps first take the shared walks (and the groups
-// of one target whole), each leaving its group's FP64 sums and list in the
-// group's slot, then take every target's pass as a job of its own, each
-// starting as soon as its group's walk is done (target_jobs).  Both
-// schedules run the same passes and add each target's part onto the group's
-// sums the same way, so the results are the same bits.
+// two: the warps first take the groups' traversals and dense passes (and the
+// groups of one target whole), each leaving its group's FP64 sums and partial
+// list in the group's slot and publishing the list's lengths; then they take
+// every target's pass as a job of its own, starting as soon as the group's
+// lengths are published.  A job waits only for a group whose walk a running
+// warp has taken, so every wait ends; a wait is still bounded (kStSpinLimit,
+// the job skipped).  Both schedules run the same passes and add their parts
+// in the same order, so the results are the same bits.
 template <class E, bool QUAD>
-__global__ void __launch_bounds__(kWalkThreads, 4) k_walk(WalkArgs a) {
+__global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpSmem& S = reinterpret_cast<WarpSmem*>(smem_raw)[warp];
   if (a.st->status & (kStNonFinite | kStNodeOverflow | kStSpinLimit)) return;  // the build failed: touch nothing
-  const uint32_t ngroups = a.st->n_groups, ntargets = a.st->n_targets;
-  const bool two_pass = ngroups <= a.nslots;
-  const size_t wid = (size_t)blockIdx.x * kWalkWarps + warp;
-  unsigned long long n_pp = 0, n_pc = 0;
-  E ev(a, S.stage, lane);
-  Queues q;
+  Job& J = S.job;
+  if (lane == 0) S.ncell = S.npart = 0ull;
+  J.jobs = 0u;
   for (;;) {
-    uint32_t gi = 0;
-    if (lane == 0) gi = atomicAdd(&a.st->walk_next, 1u);
-    gi = __shfl_sync(kFull, gi, 0);
-    if (gi >= ngroups) break;
-    const GroupInfo g = group_info(a, gi, ngroups, ntargets);
-    const uint32_t k = g.k, p0 = g.p0;
-    const uint32_t root = a.sys[g.s].root;
-    const SysParam& sp = a.prm[g.s];
-    const double theta2 = sp.theta2;
-    ev.set_system(sp.eps2, a.sys[g.s].hw);
-    const uint32_t n0 = a.ncount[a.targets[g.t0]];
-    if (k == 1 && n0 > (uint32_t)kGroupMax) {
-      // a large target: batches of kGroupMax particles, each walking the
-      // whole target's box from the root
-      double lo[3], hi[3];
-      particle_box(a.pm, p0, n0, lane, lo, hi);
-      ev.cx = 0.5 * (lo[0] + hi[0]), ev.cy = 0.5 * (lo[1] + hi[1]), ev.cz = 0.5 * (lo[2] + hi[2]);
-      for (uint32_t b0 = 0; b0 < n0; b0 += kGroupMax) {
-        const uint32_t nb = min((uint32_t)kGroupMax, n0 - b0);
-        for (uint32_t i = lane; i < nb; i += 32) S.acc[i][0] = S.acc[i][1] = S.acc[i][2] = 0.0;
-        __syncwarp();
-        int r = 0;
-        for (int attempt = 0; attempt < 2; ++attempt) {
-          ev.setup(lane, p0 + b0, (int)nb, S.acc);
-          r = target_walk(ev, a, S, root, lo, hi, theta2, attempt == 1, lane, q);
-          if (r == 0) break;
-        }
-        ev.finish();
-        add_counts(q, nb, QUAD, n_pp, n_pc);
-        kick_drift(a, sp, S.acc, p0 + b0, nb, lane);
+    const uint32_t ngroups = a.st->n_groups, ntargets = a.st->n_targets;
+    const bool two_pass = ngroups <= a.nslots;
+    const size_t wid = (size_t)blockIdx.x * kWalkWarps + warp;
+    uint32_t next = 0;
+    if (lane == 0) next = atomicAdd(J.jobs ? &a.st->walk_next2 : &a.st->walk_next, 1u);
+    next = __shfl_sync(kFull, next, 0);
+    __syncwarp();  // every lane is done with the last job
+    if (J.jobs) {
+      if (next >= ntargets) break;
+      // its group: the last whose first target is at or before it
+      uint32_t gi = 0, hi = ngroups;
+      while (hi - gi > 1) {
+        const uint32_t mid = (gi + hi) >> 1;
+        if (a.groups[mid] <= next) gi = mid;
+        else hi = mid;
       }
+      J.gi = gi, J.ti = next;
+    } else if (next < ngroups) {
+      J.gi = next;
+    } else if (two_pass) {
+      J.jobs = 1u;
       continue;
-    }
-    // the targets: particle ranges and boxes (lane i: target i), the group box
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    if ((uint32_t)lane < k) {
-      const uint32_t tn = a.targets[g.t0 + lane];
-      const uint32_t tb = a.nbegin[tn], tc = a.ncount[tn];
-      for (uint32_t i = 0; i < tc; ++i) {
-        const double4 p = a.pm[tb + i];
-        lo[0] = fmin(lo[0], p.x), hi[0] = fmax(hi[0], p.x);
-        lo[1] = fmin(lo[1], p.y), hi[1] = fmax(hi[1], p.y);
-        lo[2] = fmin(lo[2], p.z), hi[2] = fmax(hi[2], p.z);
-      }
-      S.tbeg[lane] = tb, S.tcnt[lane] = tc;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) S.tlo[lane][d] = lo[d], S.thi[lane][d] = hi[d];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], o));
-        hi[d] = fmax(hi[d], __shfl_xor_sync(kFull, hi[d], o));
-      }
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) S.glo[d] = lo[d], S.ghi[d] = hi[d];
-    }
-    __syncwarp();
-    const uint32_t np = S.tbeg[k - 1] + S.tcnt[k - 1] - p0;
-    for (uint32_t i = lane; i < np; i += 32) S.acc[i][0] = S.acc[i][1] = S.acc[i][2] = 0.0;
-    __syncwarp();
-    // the list: the warp's slot, or in the two-pass schedule the group's
-    const bool split = two_pass && k > 1;
-    uint2* list = a.wlist + (split ? (size_t)gi : wid) * kListCap;
-    // the shared walk (redone one node at a time if the stack would overflow)
-    ev.cx = 0.5 * (lo[0] + hi[0]), ev.cy = 0.5 * (lo[1] + hi[1]), ev.cz = 0.5 * (lo[2] + hi[2]);
-    uint32_t nlist = 0;
-    int r = 0;
-    for (int attempt = 0; attempt < 2; ++attempt) {
-      ev.setup(lane, p0, (int)np, S.acc);
-      r = group_walk(ev, a, S, root, k, theta2, attempt == 1, lane, list, nlist, q);
-      if (r != 1) break;
-    }
-    if (r == 0) {
-      ev.finish();
-      add_counts(q, np, QUAD, n_pp, n_pc);
-    }
-    if (split) {  // the targets' passes run as jobs of their own (target_jobs)
-      if (r == 0) {
-        double* gs = a.gsum + (size_t)gi * (kGroupMax * 3);
-        for (uint32_t i = lane; i < np; i += 32) gs[3 * i] = S.acc[i][0], gs[3 * i + 1] = S.acc[i][1], gs[3 * i + 2] = S.acc[i][2];
-      }
-      __threadfence();  // the sums and the list before the length
-      __syncwarp();
-      if (lane == 0) st_volatile(a.gnl + gi, r == 0 ? nlist : kNotShared);
-      continue;
-    }
-    if (r == 0) {
-      // each target's part from the list, in target order
-      if (nlist) {
-        for (uint32_t i = 0; i < k; ++i) {
-          const uint32_t tb = S.tbeg[i], tn = S.tcnt[i];
-          ev.cx = 0.5 * (S.tlo[i][0] + S.thi[i][0]), ev.cy = 0.5 * (S.tlo[i][1] + S.thi[i][1]);
-          ev.cz = 0.5 * (S.tlo[i][2] + S.thi[i][2]);
-          ev.setup(lane, tb, (int)tn, S.acc + (tb - p0));
-          target_pass(ev, a, S, list, nlist, i, lane, q);
-          ev.finish();
-          add_counts(q, tn, QUAD, n_pp, n_pc);
-        }
-      }
     } else {
-      // the list overflowed: nothing of the shared walk is kept (its partial
-      // sums were never added); every target walks on its own
-      targets_alone<E, QUAD>(ev, a, S, root, theta2, k, p0, lane, n_pp, n_pc);
+      break;
     }
-    kick_drift(a, sp, S.acc, p0, np, lane);
+    group_info(a, J, ngroups, ntargets);
+    J.w = Walk{0u, 0u, 0u, 0u, 0u, 0u};
+    if (J.jobs) {
+      if (J.k == 1) continue;  // done whole by its group
+      uint32_t len = ld_volatile(a.gnl + J.gi);
+      for (int spins = 0; len == kListPending && spins < kSpinLimit; ++spins) {
+        __nanosleep(128);
+        len = ld_volatile(a.gnl + J.gi);
+      }
+      len = __shfl_sync(kFull, len, 0);  // one value for the warp
+      if (len == kListPending) {
+        if (lane == 0) atomicOr(&a.st->status, kStSpinLimit);
+        continue;
+      }
+      __threadfence();  // the group's sums and list after its lengths
+      J.w.npc = len & 0xffffu, J.w.npr = len >> 16;
+      const uint32_t bit = J.ti - J.t0, tn = a.targets[J.ti];
+      const uint32_t tb = a.nbegin[tn], tc = a.ncount[tn];  // tc <= kGroupMax: inside a group
+      double lo[3], hi[3];
+      particle_box(a.pm, tb, tc, lane, lo, hi);
+      S.tbeg[bit] = tb, S.tcnt[bit] = tc;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) S.tlo[bit][d] = lo[d], S.thi[bit][d] = hi[d];
+      const double* gs = a.gsum + (size_t)J.gi * (kGroupMax * 3) + 3 * (tb - J.p0);
+      for (uint32_t i = lane; i < 3 * tc; i += 32) (&S.acc[tb - J.p0][0])[i] = gs[i];
+      J.n = tc;
+      J.pass1 = 1 + bit;
+      __syncwarp();
+    } else {
+      J.n = group_boxes(a, S, lane);
+    }
+    for (uint32_t b0 = 0; b0 < J.n; b0 += kGroupMax) {  // once, but for a large target
+      J.b0 = b0;
+      if (!J.jobs) {
+        for (uint32_t i = lane; i < 3 * kGroupMax; i += 32) (&S.acc[0][0])[i] = 0.0;
+        // the traversal starts with the root
+        S.stack[0] = make_uint2(a.sys[J.sys].root, ((1u << J.k) - 1u) | (1u << 24));
+        J.w.top = 1, J.w.steps = 0;
+        __syncwarp();
+      }
+      // the lists: the dense one is the warp's, the partial one the warp's or
+      // (two-pass schedule) the group's
+      do {
+        uint32_t pass = J.pass1;
+        if (!J.jobs) {
+          const bool more = traverse(a, S, a.prm[J.sys].theta2, a.dlist + wid * kDenseCap,
+                                     a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap, lane);
+          // all passes when the partial list is full or complete, else the dense one
+          const bool all = more ? J.w.npc + J.w.npr + 64 > kListCap : !(two_pass && J.k > 1);
+          J.more = more;
+          pass = 0, J.pass1 = all && J.w.npc + J.w.npr ? J.k : 0u;
+        } else {
+          J.more = 0u;
+        }
+        E ev(a, S, lane, a.prm[J.sys].eps2, a.sys[J.sys].hw);
+        for (; pass <= J.pass1; ++pass) {
+          const bool dense = pass == 0;
+          const uint32_t nc = dense ? J.w.ndc : J.w.npc, nr = dense ? J.w.ndr : J.w.npr;
+          if (nc + nr == 0) continue;
+          const uint32_t i = pass - 1;
+          const uint32_t tn = dense ? min(J.n - J.b0, (uint32_t)kGroupMax) : S.tcnt[i];
+          {
+            const double* lo = dense ? S.glo : S.tlo[i];
+            const double* hi = dense ? S.ghi : S.thi[i];
+            ev.setup(dense ? J.p0 + J.b0 : S.tbeg[i], (int)tn, 0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]),
+                     0.5 * (lo[2] + hi[2]));
+          }
+          list_pass(ev, a, S,
+                    dense ? a.dlist + wid * kDenseCap : a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap, nc,
+                    dense ? kDenseCap : kListCap, nr, dense, dense ? kFull : 1u << i, tn, lane);
+          ev.finish((int)tn, S.acc + (dense ? 0u : S.tbeg[i] - J.p0));
+        }
+        __syncwarp();
+        J.w.ndc = J.w.ndr = 0;
+        if (J.pass1) J.w.npc = J.w.npr = 0;
+        __syncwarp();
+      } while (J.more);
+      const uint32_t nb = min(J.n - J.b0, (uint32_t)kGroupMax);
+      if (two_pass && J.k > 1 && !J.jobs) {  // leave the sums and the partial list to the target jobs
+        double* gs = a.gsum + (size_t)J.gi * (kGroupMax * 3);
+        for (uint32_t i = lane; i < 3 * nb; i += 32) gs[i] = (&S.acc[0][0])[i];
+        __threadfence();  // the sums and the list before the lengths
+        __syncwarp();
+        if (lane == 0) st_volatile(a.gnl + J.gi, J.w.npc | (J.w.npr << 16));
+      } else {
+        const uint32_t off = J.jobs ? S.tbeg[J.ti - J.t0] - J.p0 : 0u;
+        kick_drift(a, a.prm[J.sys], S.acc + off, J.p0 + off + J.b0, nb, lane);
+      }
+    }
   }
-  if (two_pass) target_jobs<E, QUAD>(ev, a, S, ngroups, ntargets, lane, q, n_pp, n_pc);
-  if (lane == 0) {
-    atomicAdd(&a.st->pp, n_pp);
-    atomicAdd(&a.st->pc, n_pc);
+  if (lane == 0) {  // quad: cells are particle-cell interactions, else monopoles counted as particles
+    atomicAdd(&a.st->pp, S.npart + (QUAD ? 0ull : S.ncell));
+    atomicAdd(&a.st->pc, QUAD ? S.ncell : 0ull);
   }
 }
 
@@ -1226,9 +1059,10 @@ int walk_blocks_per_sm(int precision, bool quad, bool mask) {
 
 int walk_threads() { return kWalkThreads; }
 
-// Device bytes of one list slot: the list, and the group's FP64 sums and
-// list length for the two-pass schedule.
+// Device bytes of one list slot: the partial list, and the group's FP64 sums
+// and list lengths for the two-pass schedule; and of a warp's dense list.
 size_t walk_slot_bytes() { return kListCap * sizeof(uint2) + kGroupMax * 3 * sizeof(double) + sizeof(uint32_t); }
+size_t walk_dense_bytes() { return kDenseCap * sizeof(uint2); }
 
 // ---------------------------------------------------------------------------
 // Unfused integrate phase: kick_one / drift_one (integrate.h:15-16) with

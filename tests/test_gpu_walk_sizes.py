@@ -34,3 +34,39 @@ def test_walk_sizes_match_oracle(gpu, oracle, leaf, precision, tol):
             assert (st["pp"], st["pc"]) == (int(counts[0]), int(counts[1])), (n, quad, eps2)
             assert np.all(np.isfinite(acc))
             assert rel_error(acc, racc) <= tol, (n, quad, eps2)
+
+
+@pytest.mark.parametrize("precision,tol", [(bhg.PRECISION_FP64, 1e-12), (bhg.PRECISION_SPLIT, 1e-5)])
+def test_leaf_too_large_for_a_list_entry(gpu, oracle, precision, tol):
+    """300 particles at one point: a leaf of more particles than a partial
+    list's entry counts, which some targets of the groups around it open."""
+    parts = cube(2000, 41)
+    parts["pos"][:300] = [1.25, -3.5, 2.0]
+    dom, sk, perm, mp, t = _oracle_build(oracle, parts, 8)
+    tg = oracle.targets(t, 8, 1024)
+    for theta in (0.3, 0.6):
+        racc, counts = oracle.walk(t, tg, soa(mp), [Params(theta, 1e-4, 1.0, 1)] * len(tg))
+        gpu.upload(parts)
+        gpu.stats(reset=True)
+        gpu.build_tree(8, 1024)
+        gpu.compute_multipoles()
+        acc = gpu.walk_forces(bhg.Context.params(theta, 1e-4, 1.0, True, precision), 8)
+        st = gpu.stats()
+        assert (st["pp"], st["pc"]) == (int(counts[0]), int(counts[1]))
+        assert rel_error(acc, racc) <= tol
+
+
+@pytest.mark.parametrize("precision", [bhg.PRECISION_SPLIT, bhg.PRECISION_FP64])
+def test_full_lists_give_the_same_bits_in_both_schedules(precision):
+    """theta 0.15 with one particle per leaf fills both lists of most groups,
+    so their traversals pause and go on; the two-pass schedule (all slots) and
+    the one-pass schedule (a budget with few slots) agree bit for bit."""
+    parts = cube(20000, 5)
+    fp = bhg.Context.params(0.15, 1e-6, 1.0, True, precision)
+    out = []
+    for budget in (0, 36 << 20):
+        with bhg.Context(device=0, hbm_budget=budget) as ctx:
+            ctx.upload(parts)
+            ctx.step(fp, 1, 64, 1, 0.01, 0.01)
+            out.append(ctx.download().tobytes())
+    assert out[0] == out[1]
