@@ -163,7 +163,7 @@ void drop_graph(bhg_context* c) {
 
 // Device bytes of one node slot (the SoA arrays, the walk record, the cut
 // lists) and of the slots one particle brings at max_leaf 16 (0.45 each).
-constexpr size_t kNodeBytes = 16 + 32 + 32 + 48 + 64 + 8 + 48 + 8 + 12 + 4;
+constexpr size_t kNodeBytes = 16 + 32 + 32 + 48 + 32 + 8 + 64 + 8 + 12 + 4;
 constexpr size_t kNodeBytesPerParticle = kNodeBytes * 45 / 100;
 // Device bytes of the particle-sized buffers, per particle: the state and
 // its staging copy, sources, sort keys and values, marks, accelerations.
@@ -189,8 +189,8 @@ int ensure_nodes(bhg_context* c, size_t need) {
   int r;
   if ((r = grow(c, &c->nd.begin, cap)) || (r = grow(c, &c->nd.count, cap)) || (r = grow(c, &c->nd.first, cap)) ||
       (r = grow(c, &c->nd.info, cap)) || (r = grow(c, &c->nd.box, cap)) || (r = grow(c, &c->nd.mom, cap)) ||
-      (r = grow(c, &c->nd.iab, cap * 6)) || (r = grow(c, &c->nd.w, cap)) || (r = grow(c, &c->nd.q45, cap)) ||
-      (r = grow(c, &c->nd.q64, cap * 6)) || (r = grow(c, &c->nd.parent, cap)) || (r = grow(c, &c->nd.upcnt, cap)) ||
+      (r = grow(c, &c->nd.iab, cap * 6)) || (r = grow(c, &c->nd.wcom, cap)) || (r = grow(c, &c->nd.wlink, cap)) ||
+      (r = grow(c, &c->nd.src, cap)) || (r = grow(c, &c->nd.parent, cap)) || (r = grow(c, &c->nd.upcnt, cap)) ||
       (r = grow(c, &c->targets, cap)) || (r = grow(c, &c->groups, cap)) || (r = grow(c, &c->chunks, cap)) ||
       (r = grow(c, &c->level_lb, cap / 32 + kLevels + 8)))
     return r;
@@ -469,10 +469,11 @@ void enq_targets(bhg_context* c, uint32_t target_size) {
 
 void enq_walk(bhg_context* c, bool want_accel) {
   WalkArgs a;
-  a.w = c->nd.w;
-  a.q45 = c->nd.q45;
-  a.q64 = c->nd.q64;
+  a.wcom = c->nd.wcom;
+  a.wlink = c->nd.wlink;
+  a.src = c->nd.src;
   a.mom = c->nd.mom;
+  a.iab = c->nd.iab;
   a.nbegin = c->nd.begin;
   a.ncount = c->nd.count;
   a.pm = c->pm;

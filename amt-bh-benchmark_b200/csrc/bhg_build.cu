@@ -841,25 +841,17 @@ __device__ void finalize_node(const Nodes& nd, const double4* __restrict__ pm, u
     for (int t = 0; t < 3; ++t) q[t] = __dsub_rn(__dmul_rn(3.0, iab[t]), tr);
 #pragma unroll
     for (int t = 3; t < 6; ++t) q[t] = __dmul_rn(3.0, iab[t]);
-    double* qo = nd.q64 + (size_t)i * 6;
-#pragma unroll
-    for (int t = 0; t < 6; ++t) qo[t] = q[t];
-    WNode w;
-    w.cx = com[0];
-    w.cy = com[1];
-    w.cz = com[2];
     const double edge = __dmul_rn(2.0, bx.w);
-    w.edge2 = __dmul_rn(edge, edge);
-    w.first = nd.first[i];
-    w.count = nd.count[i];
-    w.info = info;
-    w.mass = (float)r.m;
-    w.q[0] = (float)q[0];
-    w.q[1] = (float)q[1];
-    w.q[2] = (float)q[2];
-    w.q[3] = (float)q[3];
-    nd.w[i] = w;
-    nd.q45[i] = make_float2((float)q[4], (float)q[5]);
+    nd.wcom[i] = make_double4(com[0], com[1], com[2], __dmul_rn(edge, edge));
+    nd.wlink[i] = info_leaf(info) ? make_uint2(nd.begin[i], nd.count[i] | kLeafBit)
+                                  : make_uint2(nd.first[i], info_nchild(info));
+    // two 32-byte stores
+    float4* src = reinterpret_cast<float4*>(nd.src + i);
+    reinterpret_cast<double2*>(src)[0] = make_double2(com[0], com[1]);
+    src[1] = make_float4(__int_as_float(__double2loint(com[2])), __int_as_float(__double2hiint(com[2])), (float)r.m,
+                         (float)q[0]);
+    src[2] = make_float4((float)q[1], (float)q[2], (float)q[3], (float)q[4]);
+    src[3] = make_float4((float)q[5], 0.f, 0.f, 0.f);
   }
 }
 

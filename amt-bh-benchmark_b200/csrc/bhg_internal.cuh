@@ -7,8 +7,8 @@
 //   keys/vals   2 x (u64+u32)[n]    radix-sort ping-pong buffers
 //   nodes       per node: begin/count/first/info (16 B), box double4 (32 B),
 //               multipole double4 com+mass (32 B) + iab double[6] (48 B),
-//               walk record WNode (64 B) + the last two quadrupole terms
-//               (8 B), FP64 traceless quadrupole (48 B)
+//               for the walk: centre of mass + edge^2 double4 (32 B),
+//               links uint2 (8 B), SourceNode (64 B)
 //   systems     SysDev[S]     one per independent system (domain, params)
 // Every size that changes from step to step (node counts per level, target
 // count, sort tiles taken) lives in DevState in device memory, so a captured
@@ -65,17 +65,23 @@ struct Tile {
   uint32_t sys, start, count, first_tile;  // first_tile: first tile of the system
 };
 
-// Walk record of a node: what every visit reads, in one 64-byte line.
-struct alignas(64) WNode {
+// What the walk's evaluators read of a node: one 64-byte record, two 32-byte
+// loads.  Gathering sources is bound by passes through the load unit: with
+// this record in place of five loads from two arrays, staged by two sources
+// per lane, a 1M walk makes 0.77e9 of them instead of 1.07e9 and takes 5.36
+// instead of 5.80 ms (4M: 21.4 instead of 23.2).
+struct alignas(64) SourceNode {
   double cx, cy, cz;  // centre of mass
-  double edge2;       // (2 * half_width)^2, as mac_accept_bbox forms it
-  uint32_t first;     // first child (interior) or first particle (leaf)
-  uint32_t count;     // particles
-  uint32_t info;      // nchild | leaf << 4 | depth << 8
   float mass;         // FP32 mass (split walk)
-  float q[4];         // FP32 traceless quadrupole xx, yy, zz, xy
+  float q[6];         // FP32 traceless quadrupole xx, yy, zz, xy, xz, yz
+  float pad[3];
 };
-static_assert(sizeof(WNode) == 64, "WNode is one 64-byte line");
+static_assert(sizeof(SourceNode) == 64, "two 32-byte loads");
+
+// What its traversal reads besides the centre of mass and edge^2: the first
+// child and the children (an interior node), or the first particle and the
+// particles with kLeafBit (a leaf).
+constexpr uint32_t kLeafBit = 0x80000000u;
 
 __host__ __device__ inline uint32_t info_nchild(uint32_t i) { return i & 15u; }
 __host__ __device__ inline bool info_leaf(uint32_t i) { return (i >> 4) & 1u; }
@@ -135,9 +141,9 @@ struct Nodes {
   double4* box;     // cell centre xyz, half width
   double4* mom;     // centre of mass xyz, mass
   double* iab;      // 6 per node: second moment about the centre of mass
-  WNode* w;         // walk records
-  float2* q45;      // FP32 traceless quadrupole xz, yz
-  double* q64;      // 6 per node: FP64 traceless quadrupole (the FP64 walk)
+  double4* wcom;    // walk: centre of mass xyz, edge^2 ((2 * half_width)^2, as mac_accept_bbox forms it)
+  uint2* wlink;     // walk: first child and children, or first particle and particles | kLeafBit
+  SourceNode* src;  // walk: the evaluators' records
   uint32_t* parent; // parent slot (kNoParent for a root)
   uint32_t* upcnt;  // children whose multipoles are done (the upward pass)
   uint32_t cap;     // node slots

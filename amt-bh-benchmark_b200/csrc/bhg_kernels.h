@@ -42,10 +42,11 @@ void launch_targets(const Nodes& nd, uint32_t lim, uint32_t pack, uint32_t n, ui
 void launch_moments(const Nodes& nd, const double4* pm, const DevState* st, int sms, bool one_launch, cudaStream_t s);
 
 struct WalkArgs {
-  const WNode* w;
-  const float2* q45;
-  const double* q64;
+  const double4* wcom;
+  const uint2* wlink;
+  const SourceNode* src;
   const double4* mom;  // FP64 centre of mass + mass (the FP64 walk)
+  const double* iab;   // second moments (the FP64 walk)
   const uint32_t* nbegin;
   const uint32_t* ncount;
   const double4* pm;

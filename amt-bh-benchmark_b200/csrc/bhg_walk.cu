@@ -202,6 +202,19 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return y;
 }
 
+// 32 bytes of device memory in one load (the SM's widest): a gather of
+// records takes half the passes through the load unit that 16-byte loads take.
+__device__ __forceinline__ void ld32(const void* p, double& a, double& b, double& c, double& d) {
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+      : "=d"(a), "=d"(b), "=d"(c), "=d"(d)
+      : "l"(__cvta_generic_to_global(p)));
+}
+__device__ __forceinline__ void ld32(const void* p, float (&v)[8]) {
+  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(__cvta_generic_to_global(p)));
+}
+
 // The lane groups' sums (S.sums; lane g * lpg + l: targets l and l + lpg),
 // added in group order into the targets' FP64 sums out[0 .. tb).
 __device__ __forceinline__ void add_group_sums(const WarpSmem& S, int lane, int tb, int lpg, int ng, double (*out)[3]) {
@@ -238,7 +251,7 @@ struct SplitEval {
   // make the scaling exact (rsqrt of an even power of two too), and the FP64
   // sums are scaled back.  The scales and the reference point (the box's
   // centre) stay in shared memory: no registers while a batch is evaluated.
-  int lane, ng, first;
+  int lane, ng, inv_ng, first;
   f2 t0x, t0y, t0z, t1x, t1y, t1z;  // minus the targets' positions, in both halves (t1 = t0 where there is none)
   f2 a0x, a0y, a0z, a1x, a1y, a1z;  // FP32 partials
   int pend;  // terms in this lane's FP32 partials since the last flush (an upper bound, warp-uniform)
@@ -257,10 +270,11 @@ struct SplitEval {
   // targets: particles p0 .. p0 + n - 1 (n <= 64), offsets from (x, y, z)
   __device__ void setup(uint32_t p0, int n, double x, double y, double z) {
     S.centre[0] = x, S.centre[1] = y, S.centre[2] = z;
-    const int lpg = (n + 1) >> 1;
-    ng = 32 / lpg;
-    first = lane < lpg * ng ? lane / lpg : 1 << 30;  // inactive lanes take no sources
-    const int t0 = lane % lpg, t1 = t0 + lpg < n ? t0 + lpg : t0;
+    const int lpg = (n + 1) >> 1, inv = 65536 / lpg + 1;  // x / lpg = x * inv >> 16 for x <= 95
+    const int g = lane * inv >> 16, t0 = lane - g * lpg, t1 = t0 + lpg < n ? t0 + lpg : t0;
+    ng = 32 * inv >> 16;
+    inv_ng = 65536 / ng + 1;
+    first = g < ng ? g : 1 << 30;  // inactive lanes take no sources
     const double4 q0 = a.pm[p0 + t0], q1 = a.pm[p0 + t1];
     const double scale = S.scale;
     t0x = twice(__dsub_rn(x, q0.x) * scale), t0y = twice(__dsub_rn(y, q0.y) * scale);
@@ -339,36 +353,51 @@ struct SplitEval {
     ax = f2_fma(c, dx, ax), ay = f2_fma(c, dy, ay), az = f2_fma(c, dz, az);
   }
 
-  // cells: node ids ring[0 .. cnt), cnt <= kCellBatch
+  // one coordinate of two sources, as a packed pair of offsets
+  __device__ __forceinline__ f2 offsets(double s0, double s1, double c, double scale) const {
+    return f2_pack((float)(__dsub_rn(s0, c) * scale), (float)(__dsub_rn(s1, c) * scale));
+  }
+
+  // cells: node ids ring[0 .. cnt), cnt <= kCellBatch.  Lane r stages record
+  // r: sources r and r + nrec (for the last record of an odd batch, one that
+  // contributes exactly 0).
   __device__ __forceinline__ void cells(const uint32_t* ring, int cnt) {
-    float* st = reinterpret_cast<float*>(S.stage);
-    const int rounded = (cnt + 1) & ~1;  // an odd batch ends with a source that contributes exactly 0
-    const double cx = S.centre[0], cy = S.centre[1], cz = S.centre[2], scale = S.scale;
-    const float scale2f = (float)S.scale2;
-    for (int i = lane; i < rounded; i += 32) {
-      float* r = st + 4 * (i >> 1) + (i & 1);
-      float v[10] = {kFarAway, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      if (i < cnt) {
-        const uint32_t n = ring[i];
-        const WNode* w = a.w + n;
-        const double2 cxy = *reinterpret_cast<const double2*>(&w->cx);
-        const double czz = w->cz;
-        v[0] = (float)(__dsub_rn(cxy.x, cx) * scale), v[1] = (float)(__dsub_rn(cxy.y, cy) * scale);
-        v[2] = (float)(__dsub_rn(czz, cz) * scale), v[3] = w->mass;
-        if (QUAD) {
-          const float4 qa = *reinterpret_cast<const float4*>(w->q);
-          const float2 qb = a.q45[n];
-          v[4] = -qa.x * scale2f, v[5] = -qa.y * scale2f, v[6] = -qa.z * scale2f, v[7] = -qa.w * scale2f;
-          v[8] = -qb.x * scale2f, v[9] = -qb.y * scale2f;
-        }
+    ulonglong2* rec = reinterpret_cast<ulonglong2*>(S.stage);
+    const int nrec = (cnt + 1) >> 1;
+    if (lane < nrec) {
+      const bool two = lane + nrec < cnt;
+      const uint32_t n0 = ring[lane], n1 = two ? ring[lane + nrec] : n0;
+      double x0, y0, z0, m0, x1, y1, z1, m1;  // m: the mass and the first quadrupole term
+      ld32(a.src + n0, x0, y0, z0, m0);
+      ld32(a.src + n1, x1, y1, z1, m1);
+      float q0[8], q1[8];
+      if (QUAD) {
+        ld32(reinterpret_cast<const char*>(a.src + n0) + 32, q0);
+        ld32(reinterpret_cast<const char*>(a.src + n1) + 32, q1);
       }
+      const double scale = S.scale;
+      f2 px = offsets(x0, x1, S.centre[0], scale), py = offsets(y0, y1, S.centre[1], scale);
+      f2 pz = offsets(z0, z1, S.centre[2], scale);
+      if (!two) {
+        px = f2_pack(__uint_as_float((uint32_t)px), kFarAway), m1 = 0.0;
 #pragma unroll
-      for (int k = 0; k < (QUAD ? 10 : 4); ++k) r[(k >> 1) * (4 * kCellPlane) + (k & 1) * 2] = v[k];
+        for (int k = 0; k < 5; ++k) q1[k] = 0.f;
+      }
+      rec[lane] = make_ulonglong2(px, py);
+      rec[kCellPlane + lane] =
+          make_ulonglong2(pz, f2_pack(__int_as_float(__double2loint(m0)), __int_as_float(__double2loint(m1))));
+      if (QUAD) {
+        const float s2 = -(float)S.scale2;
+        const f2 n2 = f2_pack(s2, s2);  // the quadrupoles negated, in scaled units
+        rec[2 * kCellPlane + lane] =
+            make_ulonglong2(f2_mul(f2_pack(__int_as_float(__double2hiint(m0)), __int_as_float(__double2hiint(m1))), n2),
+                            f2_mul(f2_pack(q0[0], q1[0]), n2));
+        rec[3 * kCellPlane + lane] = make_ulonglong2(f2_mul(f2_pack(q0[1], q1[1]), n2), f2_mul(f2_pack(q0[2], q1[2]), n2));
+        rec[4 * kCellPlane + lane] = make_ulonglong2(f2_mul(f2_pack(q0[3], q1[3]), n2), f2_mul(f2_pack(q0[4], q1[4]), n2));
+      }
     }
     __syncwarp();
-    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(S.stage);
     const f2 e2 = twice(S.eps2);
-    const int nrec = rounded >> 1;
     for (int s = first; s < nrec; s += ng) {
       const ulonglong2 xy = rec[s], zm = rec[kCellPlane + s];
       ulonglong2 n01 = {}, n23 = {}, n45 = {};
@@ -376,36 +405,36 @@ struct SplitEval {
       cell_body(xy, zm, n01, n23, n45, e2, t0x, t0y, t0z, a0x, a0y, a0z);
       cell_body(xy, zm, n01, n23, n45, e2, t1x, t1y, t1z, a1x, a1y, a1z);
     }
-    pend += (nrec + ng - 1) / ng;
+    pend += (nrec + ng - 1) * inv_ng >> 16;
     if (pend >= kFlushTerms) flush();
     __syncwarp();
   }
 
   // direct particles: particle indices ring[0 .. cnt), cnt <= kPartBatch
   __device__ __forceinline__ void parts(const uint32_t* ring, int cnt) {
-    float* st = reinterpret_cast<float*>(S.stage);
-    const int rounded = (cnt + 1) & ~1;
-    const double cx = S.centre[0], cy = S.centre[1], cz = S.centre[2], scale = S.scale;
-    for (int i = lane; i < rounded; i += 32) {
-      float* r = st + 4 * (i >> 1) + (i & 1);
-      float4 v = make_float4(kFarAway, 0.f, 0.f, 0.f);
-      if (i < cnt) {
-        const double4 p = a.pm[ring[i]];
-        v = make_float4((float)(__dsub_rn(p.x, cx) * scale), (float)(__dsub_rn(p.y, cy) * scale),
-                        (float)(__dsub_rn(p.z, cz) * scale), (float)p.w);
-      }
-      r[0] = v.x, r[2] = v.y, r[4 * kPartPlane] = v.z, r[4 * kPartPlane + 2] = v.w;
+    ulonglong2* rec = reinterpret_cast<ulonglong2*>(S.stage);
+    const int nrec = (cnt + 1) >> 1;
+    for (int r = lane; r < nrec; r += 32) {
+      const bool two = r + nrec < cnt;
+      const uint32_t n0 = ring[r], n1 = two ? ring[r + nrec] : n0;
+      double x0, y0, z0, m0, x1, y1, z1, m1;
+      ld32(a.pm + n0, x0, y0, z0, m0);
+      ld32(a.pm + n1, x1, y1, z1, m1);
+      const double scale = S.scale;
+      f2 px = offsets(x0, x1, S.centre[0], scale), py = offsets(y0, y1, S.centre[1], scale);
+      f2 pz = offsets(z0, z1, S.centre[2], scale);
+      if (!two) px = f2_pack(__uint_as_float((uint32_t)px), kFarAway);
+      rec[r] = make_ulonglong2(px, py);
+      rec[kPartPlane + r] = make_ulonglong2(pz, f2_pack((float)m0, two ? (float)m1 : 0.f));
     }
     __syncwarp();
-    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(S.stage);
     const f2 e2 = twice(S.eps2);
-    const int nrec = rounded >> 1;
     for (int s = first; s < nrec; s += ng) {
       const ulonglong2 xy = rec[s], zm = rec[kPartPlane + s];
       part_body(xy, zm, e2, t0x, t0y, t0z, a0x, a0y, a0z);
       part_body(xy, zm, e2, t1x, t1y, t1z, a1x, a1y, a1z);
     }
-    pend += (nrec + ng - 1) / ng;
+    pend += (nrec + ng - 1) * inv_ng >> 16;
     if (pend >= kFlushTerms) flush();
     __syncwarp();
   }
@@ -441,10 +470,10 @@ struct F64Eval {
   }
 
   __device__ void setup(uint32_t p0, int n, double, double, double) {
-    const int lpg = (n + 1) >> 1;
-    ng = 32 / lpg;
-    first = lane < lpg * ng ? lane / lpg : 1 << 30;
-    const int t0 = lane % lpg, t1 = t0 + lpg < n ? t0 + lpg : t0;
+    const int lpg = (n + 1) >> 1, inv = 65536 / lpg + 1;
+    const int g = lane * inv >> 16, t0 = lane - g * lpg, t1 = t0 + lpg < n ? t0 + lpg : t0;
+    ng = 32 * inv >> 16;
+    first = g < ng ? g : 1 << 30;
     const double4 q0 = a.pm[p0 + t0], q1 = a.pm[p0 + t1];
     t0x = q0.x, t0y = q0.y, t0z = q0.z;
     t1x = q1.x, t1y = q1.y, t1z = q1.z;
@@ -489,11 +518,18 @@ struct F64Eval {
     double2* rec = reinterpret_cast<double2*>(S.stage);
     if (lane < cnt) {
       const uint32_t n = ring[lane];
-      const double2* cm = reinterpret_cast<const double2*>(a.mom + n);
-      rec[lane] = cm[0], rec[kCellBatch + lane] = cm[1];
+      double x, y, z, m;
+      ld32(a.mom + n, x, y, z, m);
+      rec[lane] = make_double2(x, y), rec[kCellBatch + lane] = make_double2(z, m);
       if (QUAD) {
-        const double2* q = reinterpret_cast<const double2*>(a.q64 + (size_t)n * 6);
-        rec[2 * kCellBatch + lane] = q[0], rec[3 * kCellBatch + lane] = q[1], rec[4 * kCellBatch + lane] = q[2];
+        // traceless Q = 3 I - tr(I) delta (accel_from_source, multipole.h:185-188)
+        const double2* ip = reinterpret_cast<const double2*>(a.iab + (size_t)n * 6);
+        const double2 i01 = ip[0], i23 = ip[1], i45 = ip[2];
+        const double tr = __dadd_rn(__dadd_rn(i01.x, i01.y), i23.x);
+        rec[2 * kCellBatch + lane] =
+            make_double2(__dsub_rn(__dmul_rn(3.0, i01.x), tr), __dsub_rn(__dmul_rn(3.0, i01.y), tr));
+        rec[3 * kCellBatch + lane] = make_double2(__dsub_rn(__dmul_rn(3.0, i23.x), tr), __dmul_rn(3.0, i23.y));
+        rec[4 * kCellBatch + lane] = make_double2(__dmul_rn(3.0, i45.x), __dmul_rn(3.0, i45.y));
       }
     }
     __syncwarp();
@@ -511,8 +547,9 @@ struct F64Eval {
   __device__ __forceinline__ void parts(const uint32_t* ring, int cnt) {
     double2* rec = reinterpret_cast<double2*>(S.stage);
     for (int i = lane; i < cnt; i += 32) {
-      const double2* p = reinterpret_cast<const double2*>(a.pm + ring[i]);
-      rec[i] = p[0], rec[kPartBatch + i] = p[1];
+      double x, y, z, m;
+      ld32(a.pm + ring[i], x, y, z, m);
+      rec[i] = make_double2(x, y), rec[kPartBatch + i] = make_double2(z, m);
     }
     __syncwarp();
     const double e2 = S.eps2;
@@ -599,12 +636,11 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
     if (c && excl < n && n < inc) S.stack[w.top - 1 - lane] = make_uint2(ent.x + (n - excl), ent.y - ((n - excl) << 24));
     w.top -= done;
     double4 c4 = make_double4(0.0, 0.0, 0.0, 0.0);
-    uint4 u4 = make_uint4(0u, 0u, 0u, 0u);
+    uint2 link = make_uint2(0u, 0u);  // first child and children, or first particle and particles | kLeafBit
     bool acc = false, rej = false;
     if (valid) {
-      const WNode* wn = a.w + node;
-      c4 = *reinterpret_cast<const double4*>(&wn->cx);  // com xyz, edge^2
-      u4 = *reinterpret_cast<const uint4*>(&wn->first);  // first, count, info, mass
+      ld32(a.wcom + node, c4.x, c4.y, c4.z, c4.w);  // com xyz, edge^2
+      link = a.wlink[node];
       // mac_accept_bbox: theta^2 * near^2 > edge^2 (multipole.h:151-153)
       acc = __dmul_rn(theta2, near2(S.glo, S.ghi, c4.x, c4.y, c4.z)) > c4.w;
       // one target: its box is the group's, so not accepted means opened
@@ -631,7 +667,8 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
       __syncwarp();
       if (und) A = X.accepts[rank] & mask, O = mask & ~A;
     }
-    const bool leaf = valid && info_leaf(u4.z);
+    const bool leaf = (link.y & kLeafBit) != 0u;
+    const uint32_t cnt = link.y & ~kLeafBit;
     // cells every target takes, some take
     const bool dc = A != 0u && A == full, pc = A != 0u && A != full;
     uint32_t m = __ballot_sync(kFull, dc);
@@ -643,17 +680,17 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
     // leaves every target opens, some open
     const bool dr = leaf && O == full, pr = leaf && O != 0u && O != full;
     m = __ballot_sync(kFull, dr);
-    if (dr) dl[kDenseCap - 1u - (w.ndr + __popc(m & lt))] = make_uint2(u4.x, u4.y);
+    if (dr) dl[kDenseCap - 1u - (w.ndr + __popc(m & lt))] = make_uint2(link.x, cnt);
     w.ndr += __popc(m);
     m = __ballot_sync(kFull, pr);
     if (pr)
       pl[kListCap - 1u - (w.npr + __popc(m & lt))] =
-          u4.y < kByNode ? make_uint2(u4.x, O | (u4.y << kCountShift)) : make_uint2(node, O | (kByNode << kCountShift));
+          cnt < kByNode ? make_uint2(link.x, O | (cnt << kCountShift)) : make_uint2(node, O | (kByNode << kCountShift));
     w.npr += __popc(m);
     // opened interior nodes: their children, with the targets that opened them
     const bool in = O != 0u && !leaf;
     m = __ballot_sync(kFull, in);
-    if (in) S.stack[w.top + __popc(m & lt)] = make_uint2(u4.x, O | (info_nchild(u4.z) << 24));
+    if (in) S.stack[w.top + __popc(m & lt)] = make_uint2(link.x, O | (cnt << 24));
     w.top += __popc(m);
     __syncwarp();
   }
@@ -725,8 +762,8 @@ __device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S,
       if (!m) continue;
       cnt = hit ? (dense ? e.y : e.y >> kCountShift) : 0u;
       if (!dense && cnt == kByNode) {
-        const WNode* wn = a.w + e.x;
-        e.x = wn->first, cnt = wn->count;
+        const uint2 link = a.wlink[e.x];
+        e.x = link.x, cnt = link.y & ~kLeafBit;
       }
       const uint32_t inc = warp_incl_scan_u32(cnt, lane);
       excl = inc - cnt;
