@@ -1566,28 +1566,22 @@ int bhg_direct_sum(bhg_context* c, int sys, const uint32_t* idx, size_t ns, doub
   const SysDev& d = c->sys_host[sys];
   for (size_t k = 0; k < ns; ++k)
     if (idx[k] >= d.n) return fail(c, BHG_EINVAL, "sample index out of range");
-  // positions of the current state (output order) into pm
-  int r;
+  if (ns == 0) return BHG_OK;
+  if (ns > 0x7fffffffull / 3) return fail(c, BHG_EINVAL, "too many sample rows");
+  // row indices, results and parts in the context's cached scratch
+  const DirectPlan plan = direct_plan(d.n, (uint32_t)ns, c->sms);
+  Scratch sc(c);
   uint32_t* didx = nullptr;
-  double* dout = nullptr;
-  double4* dpm = nullptr;
-  if ((r = dev_alloc(c, (void**)&didx, ns * 4)) || (r = dev_alloc(c, (void**)&dout, ns * 24)) ||
-      (r = dev_alloc(c, (void**)&dpm, (size_t)d.n * sizeof(double4)))) {
-    dev_free(c, didx), dev_free(c, dout), dev_free(c, dpm);
+  double *dout = nullptr, *parts = nullptr;
+  int r;
+  if ((r = sc.get(&didx, ns)) || (r = sc.get(&dout, ns * 3)) ||
+      (r = sc.get(&parts, plan.splits > 1 ? (size_t)plan.splits * ns * 3 : 0)))
     return r;
-  }
-  std::vector<Particle> hp(d.n);
-  cudaMemcpyAsync(hp.data(), c->part + d.begin, (size_t)d.n * sizeof(Particle), cudaMemcpyDeviceToHost, c->stream);
-  cudaStreamSynchronize(c->stream);
-  std::vector<double4> h4(d.n);
-  for (uint32_t i = 0; i < d.n; ++i) h4[i] = make_double4(hp[i].pos[0], hp[i].pos[1], hp[i].pos[2], hp[i].mass);
-  cudaMemcpyAsync(dpm, h4.data(), (size_t)d.n * sizeof(double4), cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(didx, idx, ns * 4, cudaMemcpyHostToDevice, c->stream);
-  launch_direct(dpm, 0, d.n, didx, (uint32_t)ns, eps2, G, dout, c->stream);
-  cudaError_t e = cudaMemcpyAsync(out, dout, ns * 24, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  dev_free(c, didx), dev_free(c, dout), dev_free(c, dpm);
-  if (e != cudaSuccess) return fail(c, BHG_ECUDA, cudaGetErrorString(e));
+  CK(cudaMemcpyAsync(didx, idx, ns * 4, cudaMemcpyHostToDevice, c->stream));
+  launch_direct(c->part + d.begin, d.n, didx, (uint32_t)ns, eps2, G, plan, parts, dout, c->stream);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(out, dout, ns * 24, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   return BHG_OK;
 }
 

@@ -84,8 +84,14 @@ void launch_integrate(Particle* p, const double* accel, uint32_t n, const SysDev
                       int sms, cudaStream_t s);
 // Counts a finished evaluation when no error bit is set.
 void launch_eval_done(DevState* st, cudaStream_t s);
-void launch_direct(const double4* pm, uint32_t begin, uint32_t n, const uint32_t* idx, uint32_t ns, double eps2,
-                   double G, double* out, cudaStream_t s);
+// The direct sum's grid: `blocks` blocks of `rows` sample rows, over `splits`
+// pieces of `chunk` sources (parts: splits x ns x 3 doubles when there are several).
+struct DirectPlan {
+  uint32_t rows, blocks, chunk, splits;
+};
+DirectPlan direct_plan(uint32_t n, uint32_t ns, int sms);
+void launch_direct(const Particle* p, uint32_t n, const uint32_t* idx, uint32_t ns, double eps2, double G,
+                   const DirectPlan& d, double* parts, double* out, cudaStream_t s);
 cudaError_t launch_energy(const Particle* p, uint32_t begin, uint32_t n, double G, double* out2, int sms,
                           cudaStream_t s);
 double measure_fp32_peak(int device);

@@ -70,3 +70,16 @@ def test_full_lists_give_the_same_bits_in_both_schedules(precision):
             ctx.step(fp, 1, 64, 1, 0.01, 0.01)
             out.append(ctx.download().tobytes())
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("ns", [1, 2, 3, 127, 129, 256, 257, 700])
+def test_direct_sum_rows_and_splits(gpu, oracle, ns):
+    """Row counts around the block's (1 .. 256 rows, a remainder block), source
+    counts below a tile, with remainders and over many splits, of the second
+    of two systems, softened and not."""
+    for n in (701, 1024, 1283, 50021):
+        a, b = cube(300, 3), cube(n, 4, spread=2.0)
+        idx = np.sort(np.random.default_rng(ns).choice(n, ns, replace=False)).astype(np.uint32)
+        gpu.upload_systems([a, b])
+        for eps2 in (1e-4, 0.0):
+            assert rel_error(gpu.direct_sum(idx, eps2, G=0.5, system=1), oracle.direct(soa(b), idx, eps2, 0.5)) < 1e-13
