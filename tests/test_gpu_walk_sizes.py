@@ -83,3 +83,25 @@ def test_direct_sum_rows_and_splits(gpu, oracle, ns):
         gpu.upload_systems([a, b])
         for eps2 in (1e-4, 0.0):
             assert rel_error(gpu.direct_sum(idx, eps2, G=0.5, system=1), oracle.direct(soa(b), idx, eps2, 0.5)) < 1e-13
+
+
+def test_repeated_shapes_give_the_same_bits():
+    """A shape's first evaluation runs kernel by kernel, its second is captured
+    and later ones replay the graph, across uploads, other shapes in between
+    (same particle count, other systems) and systems leaving (the state moves
+    to the other buffer): the same bits every time."""
+    one, two = cube(3000, 61), [cube(1300, 62), cube(1700, 63)]
+    fp = bhg.Context.params(0.5, 1e-4)
+    ref = {}
+    with bhg.Context(device=0) as ctx:
+        for what in "aaaabbbbabaabbrrrr":
+            if what == "a":
+                ctx.upload(one)
+            else:
+                ctx.upload_systems(two)
+            if what == "r":
+                ctx.remove_systems([ctx.system_ids()[0]])
+            for _ in range(2 if what == "r" else 1):
+                ctx.step(fp, 8, 256, 16, 0.01, 0.02)
+            got = ctx.download().tobytes()
+            assert ref.setdefault(what, got) == got, what
