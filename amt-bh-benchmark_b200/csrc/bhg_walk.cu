@@ -35,19 +35,15 @@
 // rsqrt.approx.ftz, lanes laid out as (target, source subset) (SplitEval
 // below); FP32 partials go into FP64 sums every 32 or more terms.  The
 // kick/drift of integrate_ttg.h:74-77 is applied in FP64 in the epilogue.
-#include "bhg_kernels.h"
+#include "bhg_walk.cuh"
 
 #include <type_traits>
 
 namespace bhg {
 
-constexpr int kWalkWarps = 4;
-constexpr int kWalkThreads = kWalkWarps * 32;
 constexpr int kStackCap = 192;       // per-warp traversal stack: runs of sibling nodes
 constexpr int kRing = 160;           // sources picked for the next batch (a batch of up to 128, less one, + 32)
 constexpr int kStageBytes = 2560;    // staged sources of one batch
-constexpr float kFarAway = 1.0e10f;  // padding source: contributes exactly 0
-constexpr uint32_t kFull = 0xffffffffu;
 // Lists are two-ended arrays of uint2: cells from the front, runs of particles
 // (opened leaves) from the back.  The dense list (sources every target of
 // the group takes): (node, 1) and (first particle, count).  The partial list
@@ -59,11 +55,7 @@ constexpr uint32_t kMaskBits = (1u << kCountShift) - 1u;
 constexpr uint32_t kByNode = 255;
 static_assert(kMaxTargets <= kCountShift, "target masks and counts share a word");
 constexpr uint32_t kDenseCap = 2048;  // entries of a dense list (16 KB)
-constexpr uint32_t kListCap = 4096;   // entries of a partial list (32 KB)
-// a group's list lengths (cells | runs << 16) before its shared walk has
-// finished (two-pass schedule; the host fills the lengths with this byte
-// pattern before every walk)
-constexpr uint32_t kListPending = 0xfefefefeu;
+// a group's list lengths are cells | runs << 16 (two-pass schedule)
 static_assert(kListCap < 0xfefe, "list lengths never look pending");
 // a traversal step pops at most (free entries - kLevels - 1) nodes, one at
 // least, and every popped node pushes at most one run of children, so that
@@ -111,38 +103,8 @@ struct StepScratch {
 };
 static_assert(sizeof(StepScratch) <= kStageBytes && kGroupMax * 3 * 8 <= kStageBytes, "scratch in the staging area");
 
-__device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t u = __shfl_up_sync(kFull, v, o);
-    if (lane >= o) v += u;
-  }
-  return v;
-}
-
-// Squared distance from (x, y, z) to the nearest point of the box, as
-// BBox::near2 (multipole.h:132-136) rounds it.
-__device__ __forceinline__ double near2(const double lo[3], const double hi[3], double x, double y, double z) {
-  double dx = fmax(fmax(__dsub_rn(lo[0], x), __dsub_rn(x, hi[0])), 0.0);
-  double dy = fmax(fmax(__dsub_rn(lo[1], y), __dsub_rn(y, hi[1])), 0.0);
-  double dz = fmax(fmax(__dsub_rn(lo[2], z), __dsub_rn(z, hi[2])), 0.0);
-  return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-}
-
-// Squared distance to the farthest point of the box (BBox::far2, multipole.h:137-141).
-__device__ __forceinline__ double far2(const double lo[3], const double hi[3], double x, double y, double z) {
-  double dx = fmax(__dsub_rn(x, lo[0]), __dsub_rn(hi[0], x));
-  double dy = fmax(__dsub_rn(y, lo[1]), __dsub_rn(hi[1], y));
-  double dz = fmax(__dsub_rn(z, lo[2]), __dsub_rn(hi[2], z));
-  return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-}
-
 // ---------------------------------------------------------------------------
-// Evaluators: what a lane does with one chunk of sources - two per lane
-// (sources j and j + L of the chunk for lane j of a group of L lanes), whose
-// interactions with each target are independent chains.  Target slot k of
-// lane group g is target g + k * gp; lane k mod L of the group adds that
-// target's partial sums into its FP64 sum.
+// Evaluators of the lists' sources.
 
 // Two FP32 values in one 64-bit register: the SM's packed FP32 instructions
 // (add, mul, fma .f32x2) work on both halves in one issue slot, each half
@@ -192,29 +154,6 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
 // scalar / packed, with 16 warps per SM: 32.9 / 30.5 ms at 4M (leaf 16), 6.53
 // / 5.52 at 1M with leaf 48, 4.04 / 3.35 at 1M with monopoles; warp
 // instructions of a 1M walk 5.48e9 / 4.16e9.
-// rsqrt.approx.ftz.f32 (PTX ISA): the approximate reciprocal square root,
-// subnormal inputs and results flushed to zero.  The split evaluator's r^2 is
-// in units scaled to the system's size (at least eps^2 there, or masked when
-// eps = 0), so the flush only drops contributions below FP32's normal range.
-__device__ __forceinline__ float rsqrt_ftz(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// 32 bytes of device memory in one load (the SM's widest): a gather of
-// records takes half the passes through the load unit that 16-byte loads take.
-__device__ __forceinline__ void ld32(const void* p, double& a, double& b, double& c, double& d) {
-  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
-      : "=d"(a), "=d"(b), "=d"(c), "=d"(d)
-      : "l"(__cvta_generic_to_global(p)));
-}
-__device__ __forceinline__ void ld32(const void* p, float (&v)[8]) {
-  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-      : "l"(__cvta_generic_to_global(p)));
-}
-
 // The lane groups' sums (S.sums; lane g * lpg + l: targets l and l + lpg),
 // added in group order into the targets' FP64 sums out[0 .. tb).
 __device__ __forceinline__ void add_group_sums(const WarpSmem& S, int lane, int tb, int lpg, int ng, double (*out)[3]) {
@@ -230,7 +169,7 @@ __device__ __forceinline__ void add_group_sums(const WarpSmem& S, int lane, int 
   __syncwarp();
 }
 
-template <bool QUAD, bool MASK>
+template <bool QUAD>
 struct SplitEval {
   static constexpr int kCellBatch = 64, kPartBatch = 128;
   static constexpr int kBlocksPerSm = 6;
@@ -307,14 +246,11 @@ struct SplitEval {
     pend = 0;
   }
 
-  // 1 / sqrt(r^2) of both halves (0 where r^2 = 0 when ZERO)
-  template <bool ZERO>
+  // 1 / sqrt(r^2) of both halves (softened: r^2 > 0)
   static __device__ __forceinline__ f2 rsqrt2(f2 r2) {
     float lo, hi;
     f2_unpack(r2, lo, hi);
-    float ilo = rsqrt_ftz(lo), ihi = rsqrt_ftz(hi);
-    if (ZERO) ilo = lo > 0.f ? ilo : 0.f, ihi = hi > 0.f ? ihi : 0.f;
-    return f2_pack(ilo, ihi);
+    return f2_pack(rsqrt_ftz(lo), rsqrt_ftz(hi));
   }
 
   // a record of two cells acting on the target at -(tx, ty, tz); the staged
@@ -323,7 +259,7 @@ struct SplitEval {
                                             ulonglong2 n45, f2 e2, f2 tx, f2 ty, f2 tz, f2& ax, f2& ay, f2& az) const {
     const f2 dx = f2_add(xy.x, tx), dy = f2_add(xy.y, ty), dz = f2_add(zm.x, tz);
     const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, e2)));
-    const f2 ri = rsqrt2<!QUAD && MASK>(r2);
+    const f2 ri = rsqrt2(r2);
     const f2 ri2 = f2_mul(ri, ri);
     const f2 ri3 = f2_mul(ri, ri2);
     if (QUAD) {
@@ -348,7 +284,7 @@ struct SplitEval {
                                             f2& az) const {
     const f2 dx = f2_add(xy.x, tx), dy = f2_add(xy.y, ty), dz = f2_add(zm.x, tz);
     const f2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, e2)));
-    const f2 ri = rsqrt2<MASK>(r2);
+    const f2 ri = rsqrt2(r2);
     const f2 c = f2_mul(f2_mul(zm.y, f2_mul(ri, ri)), ri);
     ax = f2_fma(c, dx, ax), ay = f2_fma(c, dy, ay), az = f2_fma(c, dz, az);
   }
@@ -787,75 +723,6 @@ __device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S,
   }
 }
 
-// Bounding box of particles [b, b + T) (BBox::add, multipole.h:121-128).
-__device__ __forceinline__ void particle_box(const double4* pm, uint32_t b, uint32_t T, int lane, double lo[3],
-                                             double hi[3]) {
-  lo[0] = lo[1] = lo[2] = INFINITY;
-  hi[0] = hi[1] = hi[2] = -INFINITY;
-  for (uint32_t i = lane; i < T; i += 32) {
-    const double4 q = pm[b + i];
-    lo[0] = fmin(lo[0], q.x), hi[0] = fmax(hi[0], q.x);
-    lo[1] = fmin(lo[1], q.y), hi[1] = fmax(hi[1], q.y);
-    lo[2] = fmin(lo[2], q.z), hi[2] = fmax(hi[2], q.z);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = fmin(lo[d], __shfl_xor_sync(kFull, lo[d], o));
-      hi[d] = fmax(hi[d], __shfl_xor_sync(kFull, hi[d], o));
-    }
-  }
-}
-
-// on_result(particle, G * acc) (grouped_ttg.h:281-283), then kick_one /
-// drift_one (integrate.h:15-16), for particles p0 .. p0 + n - 1 whose FP64
-// sums are in sums[0 .. n).
-__device__ __forceinline__ void kick_drift(const WalkArgs& a, const SysParam& sp, const double (*sums)[3], uint32_t p0,
-                                           uint32_t n, int lane) {
-  for (uint32_t i = lane; i < n; i += 32) {
-    const uint32_t p = p0 + i;
-    const double gx = __dmul_rn(sp.G, sums[i][0]), gy = __dmul_rn(sp.G, sums[i][1]), gz = __dmul_rn(sp.G, sums[i][2]);
-    if (a.accel) {
-      a.accel[3 * (size_t)p + 0] = gx;
-      a.accel[3 * (size_t)p + 1] = gy;
-      a.accel[3 * (size_t)p + 2] = gz;
-    }
-    Particle P = a.staged[p];
-    P.vel[0] = __dadd_rn(P.vel[0], __dmul_rn(sp.kick_dt, gx));
-    P.vel[1] = __dadd_rn(P.vel[1], __dmul_rn(sp.kick_dt, gy));
-    P.vel[2] = __dadd_rn(P.vel[2], __dmul_rn(sp.kick_dt, gz));
-    if (sp.drift_dt != 0.0) {
-      P.pos[0] = __dadd_rn(P.pos[0], __dmul_rn(sp.drift_dt, P.vel[0]));
-      P.pos[1] = __dadd_rn(P.pos[1], __dmul_rn(sp.drift_dt, P.vel[1]));
-      P.pos[2] = __dadd_rn(P.pos[2], __dmul_rn(sp.drift_dt, P.vel[2]));
-    }
-    a.out[p] = P;
-  }
-  __syncwarp();
-}
-
-// The system holding particle p (systems lie back to back).
-__device__ __forceinline__ uint32_t system_of(const WalkArgs& a, uint32_t p) {
-  uint32_t lo = 0, hi = (uint32_t)a.nsys;
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (a.sys[mid].begin <= p) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// The group of walk group gi: its targets, first particle and system.
-__device__ __forceinline__ void group_info(const WalkArgs& a, Job& j, uint32_t ngroups, uint32_t ntargets) {
-  const uint32_t gi = j.gi, t0 = a.groups[gi];
-  const uint32_t p0 = a.nbegin[a.targets[t0]];
-  j.t0 = t0;
-  j.k = (gi + 1 < ngroups ? a.groups[gi + 1] : ntargets) - t0;
-  j.p0 = p0;
-  j.sys = a.nsys > 1 ? system_of(a, p0) : 0u;
-}
-
 // The targets' particle ranges and boxes and the group's box; returns the
 // group's particles.
 __device__ __forceinline__ uint32_t group_boxes(const WalkArgs& a, WarpSmem& S, int lane) {
@@ -957,7 +824,10 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
     } else {
       break;
     }
-    group_info(a, J, ngroups, ntargets);
+    {
+      const GroupInfo g = group_info(a, J.gi, ngroups, ntargets);
+      J.t0 = g.t0, J.k = g.k, J.p0 = g.p0, J.sys = g.s;
+    }
     J.w = Walk{0u, 0u, 0u, 0u, 0u, 0u};
     if (J.jobs) {
       if (J.k == 1) continue;  // done whole by its group
@@ -1058,10 +928,11 @@ static void launch_one(const WalkArgs& a, int grid, cudaStream_t s) {
   k_walk<E, QUAD><<<grid, kWalkThreads, kWalkSmem, s>>>(a);
 }
 
+// Unsoftened split walks have a kernel of their own (bhg_walk_unsoftened.cu).
 void launch_walk(const WalkArgs& a, int precision, bool quad, bool mask, int grid, cudaStream_t s) {
   if (precision == 0) {
-    if (quad) mask ? launch_one<SplitEval<true, true>, true>(a, grid, s) : launch_one<SplitEval<true, false>, true>(a, grid, s);
-    else mask ? launch_one<SplitEval<false, true>, false>(a, grid, s) : launch_one<SplitEval<false, false>, false>(a, grid, s);
+    if (mask) launch_walk_unsoftened(a, quad, grid, s);
+    else quad ? launch_one<SplitEval<true>, true>(a, grid, s) : launch_one<SplitEval<false>, false>(a, grid, s);
   } else {
     if (quad) mask ? launch_one<F64Eval<true, true>, true>(a, grid, s) : launch_one<F64Eval<true, false>, true>(a, grid, s);
     else mask ? launch_one<F64Eval<false, true>, false>(a, grid, s) : launch_one<F64Eval<false, false>, false>(a, grid, s);
@@ -1078,8 +949,8 @@ static int occ() {
 
 static int walk_blocks_per_sm_query(int precision, bool quad, bool mask) {
   if (precision == 0) {
-    if (quad) return mask ? occ<SplitEval<true, true>, true>() : occ<SplitEval<true, false>, true>();
-    return mask ? occ<SplitEval<false, true>, false>() : occ<SplitEval<false, false>, false>();
+    if (mask) return walk_unsoftened_blocks_per_sm(quad);
+    return quad ? occ<SplitEval<true>, true>() : occ<SplitEval<false>, false>();
   }
   if (quad) return mask ? occ<F64Eval<true, true>, true>() : occ<F64Eval<true, false>, true>();
   return mask ? occ<F64Eval<false, true>, false>() : occ<F64Eval<false, false>, false>();
