@@ -98,7 +98,9 @@ constexpr size_t kWalkSmem = sizeof(WarpSmem) * kWalkWarps;
 // Scratch of a traversal step (in WarpSmem::stage): the nodes that targets
 // test on their own, and the targets that accept them.
 struct StepScratch {
-  double4 node[32];  // centre of mass, edge^2
+  float4 node[32];   // centre of mass, near^2 above which it is accepted
+  float reject[32];  // near^2 below which it is not
+  uint32_t id[32];
   uint32_t accepts[32];
 };
 static_assert(sizeof(StepScratch) <= kStageBytes && kGroupMax * 3 * 8 <= kStageBytes, "scratch in the staging area");
@@ -154,6 +156,15 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
 // scalar / packed, with 16 warps per SM: 32.9 / 30.5 ms at 4M (leaf 16), 6.53
 // / 5.52 at 1M with leaf 48, 4.04 / 3.35 at 1M with monopoles; warp
 // instructions of a 1M walk 5.48e9 / 4.16e9.
+// The units of FP32 arithmetic on offsets in a system of half width hw: a
+// power of two near its size (see SplitEval).
+__device__ __forceinline__ void set_units(WarpSmem& S, double hw) {
+  int k = hw > 0.0 ? ilogb(hw) : 0;
+  k = k < -100 ? -100 : (k > 100 ? 100 : k);
+  S.scale = ldexp(1.0, -k);       // offsets d' = d * scale
+  S.scale2 = ldexp(1.0, -2 * k);  // a = a' * scale^2 (a' = m d' / r'^3 = a / scale^2), Q' = Q * scale^2
+}
+
 // The lane groups' sums (S.sums; lane g * lpg + l: targets l and l + lpg),
 // added in group order into the targets' FP64 sums out[0 .. tb).
 __device__ __forceinline__ void add_group_sums(const WarpSmem& S, int lane, int tb, int lpg, int ng, double (*out)[3]) {
@@ -195,14 +206,10 @@ struct SplitEval {
   f2 a0x, a0y, a0z, a1x, a1y, a1z;  // FP32 partials
   int pend;  // terms in this lane's FP32 partials since the last flush (an upper bound, warp-uniform)
 
-  // softening eps2_ and the system's domain half width hw
-  __device__ SplitEval(const WalkArgs& args, WarpSmem& S_, int lane_, double eps2_, double hw)
+  // softening eps2_, after set_units
+  __device__ SplitEval(const WalkArgs& args, WarpSmem& S_, int lane_, double eps2_)
       : a(args), S(S_), lane(lane_) {
-    int k = hw > 0.0 ? ilogb(hw) : 0;
-    k = k < -100 ? -100 : (k > 100 ? 100 : k);
-    const double scale = ldexp(1.0, -k);
-    S.scale = scale;                   // offsets d' = d * scale
-    S.scale2 = ldexp(1.0, -2 * k);     // a = a' * scale^2 (a' = m d' / r'^3 = a / scale^2), Q' = Q * scale^2
+    const double scale = S.scale;
     S.eps2 = eps2_ * (scale * scale);  // eps2' = eps2 * scale^2
   }
 
@@ -400,7 +407,7 @@ struct F64Eval {
   double t0x, t0y, t0z, t1x, t1y, t1z;
   double a0x, a0y, a0z, a1x, a1y, a1z;
 
-  __device__ F64Eval(const WalkArgs& args, WarpSmem& S_, int lane_, double eps2_, double)
+  __device__ F64Eval(const WalkArgs& args, WarpSmem& S_, int lane_, double eps2_)
       : a(args), S(S_), lane(lane_) {
     S.eps2 = eps2_;
   }
@@ -527,6 +534,34 @@ struct F64Eval {
 // at 262k (leaf 16, theta 0.5); in FP64 12.8 to 9.5 ms at 1M.  With 5 blocks
 // of 4 warps per SM 23.8 ms at 4M, with 4 25.1.
 
+// The tests run in FP32 first, on offsets from the group's centre in the
+// system's units.  With u = 2^-24 and M the largest coordinate of the node and
+// of the group's box, an offset to a box face is off by at most E = 4 u M, and
+// a squared distance v by at most 2 sqrt(3 v) E + 3 E^2 (and a few u v), which
+// is at most 2^-14 v + 3 E^2 (1 + 2^14), and 3 E^2 (1 + 2^14) < 4e-9 M^2.  So with K =
+// 4e-9 M^2 (+ 1e-30, far below any edge^2, for the range FP32 loses) a node
+// is certainly accepted when v > accept = (edge^2 / theta^2 + K) / (1 - 2^-14)
+// and certainly not when v < reject = (edge^2 / theta^2 - K) / (1 + 2^-14), both
+// factors with 2e-5 to spare for the rounding of the terms themselves; NaN and
+// infinity leave both false.  What lies between - one test in some thousands -
+// is decided by the FP64 test, so every decision is the reference's.
+// Walk with them / with the FP64 tests alone: 20.7 / 21.4 ms at 4M, 5.17 /
+// 5.37 at 1M, 2.09 / 2.18 with monopoles (traversal instructions 0.63e9 of 0.84e9).
+
+__device__ __forceinline__ float near2f(const float lo[3], const float hi[3], float x, float y, float z) {
+  const float dx = fmaxf(fmaxf(lo[0] - x, x - hi[0]), 0.f);
+  const float dy = fmaxf(fmaxf(lo[1] - y, y - hi[1]), 0.f);
+  const float dz = fmaxf(fmaxf(lo[2] - z, z - hi[2]), 0.f);
+  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
+__device__ __forceinline__ float far2f(const float lo[3], const float hi[3], float x, float y, float z) {
+  const float dx = fmaxf(x - lo[0], hi[0] - x);
+  const float dy = fmaxf(y - lo[1], hi[1] - y);
+  const float dz = fmaxf(z - lo[2], hi[2] - z);
+  return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
 // Returns true when a list may be too full for another step (the lists are
 // then to be taken and reset, and the traversal goes on where it stopped).
 __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double theta2, uint2* __restrict__ dl,
@@ -537,9 +572,16 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
   const uint32_t full = (1u << k) - 1u;  // k <= kMaxTargets < 32
   StepScratch& X = *reinterpret_cast<StepScratch*>(S.stage);
   const uint32_t per = 32u / k, sub = (uint32_t)lane / k, tgt = (uint32_t)lane - sub * k;
-  double lo[3], hi[3];
+  const double gx = 0.5 * (S.glo[0] + S.ghi[0]), gy = 0.5 * (S.glo[1] + S.ghi[1]), gz = 0.5 * (S.glo[2] + S.ghi[2]);
+  float lo[3], hi[3], glo[3], ghi[3], reach = 0.f;
 #pragma unroll
-  for (int d = 0; d < 3; ++d) lo[d] = S.tlo[tgt][d], hi[d] = S.thi[tgt][d];
+  for (int d = 0; d < 3; ++d) {
+    const double c = d == 0 ? gx : d == 1 ? gy : gz, sc = S.scale;
+    lo[d] = (float)((S.tlo[tgt][d] - c) * sc), hi[d] = (float)((S.thi[tgt][d] - c) * sc);
+    glo[d] = (float)((S.glo[d] - c) * sc), ghi[d] = (float)((S.ghi[d] - c) * sc);
+    reach = fmaxf(reach, fmaxf(fabsf(glo[d]), fabsf(ghi[d])));
+  }
+  const float inv_theta2 = (float)(1.0 / theta2);
   const uint32_t max_steps = a.st->n_nodes + 2;  // a walk pops each node at most once
   bool more = false;
   while (w.top) {
@@ -571,16 +613,28 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
     __syncwarp();
     if (c && excl < n && n < inc) S.stack[w.top - 1 - lane] = make_uint2(ent.x + (n - excl), ent.y - ((n - excl) << 24));
     w.top -= done;
-    double4 c4 = make_double4(0.0, 0.0, 0.0, 0.0);
     uint2 link = make_uint2(0u, 0u);  // first child and children, or first particle and particles | kLeafBit
+    float x = 0.f, y = 0.f, z = 0.f, accept = 0.f, reject = 0.f;
     bool acc = false, rej = false;
     if (valid) {
+      double4 c4;
       ld32(a.wcom + node, c4.x, c4.y, c4.z, c4.w);  // com xyz, edge^2
       link = a.wlink[node];
+      const double sc = S.scale;
+      x = (float)((c4.x - gx) * sc), y = (float)((c4.y - gy) * sc), z = (float)((c4.z - gz) * sc);
+      const float m = fmaxf(fmaxf(fabsf(x), fabsf(y)), fmaxf(fabsf(z), reach));
+      const float slack = fmaf(4.0e-9f * m, m, 1.0e-30f), q = (float)(c4.w * S.scale2) * inv_theta2;
+      accept = (q + slack) * 1.00008f, reject = (q - slack) * 0.99992f;
+      const float n2 = near2f(glo, ghi, x, y, z);
+      acc = n2 > accept;
       // mac_accept_bbox: theta^2 * near^2 > edge^2 (multipole.h:151-153)
-      acc = __dmul_rn(theta2, near2(S.glo, S.ghi, c4.x, c4.y, c4.z)) > c4.w;
-      // one target: its box is the group's, so not accepted means opened
-      if (!acc) rej = k == 1 || __dmul_rn(theta2, far2(S.glo, S.ghi, c4.x, c4.y, c4.z)) <= c4.w;
+      if (!acc && !(n2 < reject)) acc = __dmul_rn(theta2, near2(S.glo, S.ghi, c4.x, c4.y, c4.z)) > c4.w;
+      if (!acc) {
+        // one target: its box is the group's, so not accepted means opened
+        const float f2v = far2f(glo, ghi, x, y, z);
+        rej = k == 1 || f2v < reject;
+        if (!rej && !(f2v > accept)) rej = __dmul_rn(theta2, far2(S.glo, S.ghi, c4.x, c4.y, c4.z)) <= c4.w;
+      }
     }
     uint32_t A = acc ? mask : 0u, O = rej ? mask : 0u;
     // undecided nodes: every target tests its own box
@@ -588,14 +642,20 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
     const uint32_t um = __ballot_sync(kFull, und);
     if (um) {
       const uint32_t rank = (uint32_t)__popc(um & lt), nu = (uint32_t)__popc(um);
-      if (und) X.node[rank] = c4;
+      if (und) X.node[rank] = make_float4(x, y, z, accept), X.reject[rank] = reject, X.id[rank] = node;
       __syncwarp();
       for (uint32_t base = 0; base < nu; base += per) {
         const uint32_t e = base + sub;
         bool ok = false;
         if (sub < per && e < nu) {
-          const double4 q = X.node[e];
-          ok = __dmul_rn(theta2, near2(lo, hi, q.x, q.y, q.z)) > q.w;
+          const float4 q = X.node[e];
+          const float n2 = near2f(lo, hi, q.x, q.y, q.z);
+          ok = n2 > q.w;
+          if (!ok && !(n2 < X.reject[e])) {
+            double4 c4;
+            ld32(a.wcom + X.id[e], c4.x, c4.y, c4.z, c4.w);
+            ok = __dmul_rn(theta2, near2(S.tlo[tgt], S.thi[tgt], c4.x, c4.y, c4.z)) > c4.w;
+          }
         }
         const uint32_t bits = __ballot_sync(kFull, ok);
         if (tgt == 0 && sub < per && e < nu) X.accepts[e] = (bits >> (sub * k)) & full;
@@ -829,6 +889,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
       J.t0 = g.t0, J.k = g.k, J.p0 = g.p0, J.sys = g.s;
     }
     J.w = Walk{0u, 0u, 0u, 0u, 0u, 0u};
+    set_units(S, a.sys[J.sys].hw);
     if (J.jobs) {
       if (J.k == 1) continue;  // done whole by its group
       uint32_t len = ld_volatile(a.gnl + J.gi);
@@ -881,7 +942,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
         } else {
           J.more = 0u;
         }
-        E ev(a, S, lane, a.prm[J.sys].eps2, a.sys[J.sys].hw);
+        E ev(a, S, lane, a.prm[J.sys].eps2);
         for (; pass <= J.pass1; ++pass) {
           const bool dense = pass == 0;
           const uint32_t nc = dense ? J.w.ndc : J.w.npc, nr = dense ? J.w.ndr : J.w.npr;
