@@ -41,7 +41,7 @@
 
 namespace bhg {
 
-constexpr int kStackCap = 192;       // per-warp traversal stack: runs of sibling nodes
+constexpr int kStackCap = 176;       // per-warp traversal stack: runs of sibling nodes
 constexpr int kRing = 160;           // sources picked for the next batch (a batch of up to 128, less one, + 32)
 constexpr int kStageBytes = 2560;    // staged sources of one batch
 // Lists are two-ended arrays of uint2: cells from the front, runs of particles
@@ -76,6 +76,7 @@ struct Job {
   uint32_t n, b0;          // particles; a large target's batch start
   uint32_t pass1;          // the last pass to run
   uint32_t more, jobs;     // the traversal paused; this is a target job
+  uint2 *dense, *partial;  // the lists
   Walk w;
 };
 
@@ -94,6 +95,8 @@ struct WarpSmem {
   uint32_t delta[32];  // runs of a window: first particle less the particles of the runs before it
 };
 constexpr size_t kWalkSmem = sizeof(WarpSmem) * kWalkWarps;
+// six blocks per SM: 228 KB, of which each block takes 1 KB for the system
+static_assert(6 * (kWalkSmem + 1024) <= 228 * 1024, "shared memory of 24 warps per SM");
 
 // Scratch of a traversal step (in WarpSmem::stage): the nodes that targets
 // test on their own, and the targets that accept them.
@@ -694,28 +697,40 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
   return more;
 }
 
-// Evaluates the entries of a two-ended list that `sel` picks (bits of the
-// entry's second word; dense lists: any) on the evaluator's targets: cells
-// list[0 .. nc), runs list[cap - nr .. cap).  Windows of 32 entries, the next
-// one loaded while the current one is used, fill a ring; full batches of it
-// are evaluated.  tn: the targets.
+// Entries i and i + 1 of a list of n, at p.
+__device__ __forceinline__ uint4 load_pair(const uint4* p, uint32_t i, uint32_t n) {
+  uint4 v = make_uint4(0u, 0u, 0u, 0u);
+  if (i < n) v = *p;
+  if (i + 1 >= n) v.w = 0u;
+  return v;
+}
+
+// Evaluates the entries of the job's dense or partial list that `sel` picks
+// (bits of the entry's second word) on the evaluator's tn targets: first the
+// cells, then the runs.  Windows of 64 cells or 32 runs, the next one loaded
+// while the current one is used, fill a ring; full batches of it are evaluated.
 template <class E>
-__device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S, const uint2* list, uint32_t nc,
-                                          uint32_t cap, uint32_t nr, bool dense, uint32_t sel, uint32_t tn,
+__device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S, bool dense, uint32_t sel, uint32_t tn,
                                           int lane) {
   const uint32_t lt = lanemask_lt();
   uint32_t at = 0, held = 0;
-  uint2 next = (uint32_t)lane < nc ? list[lane] : make_uint2(0u, 0u);
+  // two entries per lane and window (16-byte loads; the list's end is read as
+  // entries that nothing picks)
+  const uint4* pairs = reinterpret_cast<const uint4*>(dense ? S.job.dense : S.job.partial) + lane;
+  const uint32_t nc = dense ? S.job.w.ndc : S.job.w.npc;
+  uint4 next = load_pair(pairs, 2u * lane, nc);
   for (;;) {
     while (held < (uint32_t)E::kCellBatch && at < nc) {
-      const uint2 e = next;
-      at += 32;
-      const uint32_t j = at + (uint32_t)lane;
-      next = j < nc ? list[j] : make_uint2(0u, 0u);
-      const bool hit = (e.y & sel) != 0u;
-      const uint32_t m = __ballot_sync(kFull, hit);
-      if (hit) S.ring[held + __popc(m & lt)] = e.x;
-      held += __popc(m);
+      const uint4 e = next;
+      at += 64;
+      pairs += 32;
+      next = load_pair(pairs, at + 2u * lane, nc);
+      const bool h0 = (e.y & sel) != 0u, h1 = (e.w & sel) != 0u;
+      const uint32_t m0 = __ballot_sync(kFull, h0), m1 = __ballot_sync(kFull, h1);
+      const uint32_t pos = held + __popc(m0 & lt) + __popc(m1 & lt);
+      if (h0) S.ring[pos] = e.x;
+      if (h1) S.ring[pos + (h0 ? 1u : 0u)] = e.z;
+      held += __popc(m0) + __popc(m1);
     }
     if (!held) break;
     __syncwarp();
@@ -723,16 +738,18 @@ __device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S,
     ev.cells(S.ring, (int)cnt);
     if (lane == 0) S.ncell += cnt * tn;
     held -= cnt;
-    if (held) {
-      const uint32_t v = S.ring[cnt + lane];  // at most 31 are left
+    if (held) {  // at most kCellBatch - 1 + 64 - kCellBatch = 63 are left
+      const uint32_t v0 = S.ring[cnt + lane], v1 = S.ring[cnt + 32 + lane];
       __syncwarp();
-      if ((uint32_t)lane < held) S.ring[lane] = v;
+      if ((uint32_t)lane < held) S.ring[lane] = v0;
+      if ((uint32_t)lane + 32 < held) S.ring[lane + 32] = v1;
     }
   }
   // runs: the particles of the picked runs of a window, 32 at a time
-  const uint2* back = list + cap - 1;
+  const uint2* back = dense ? S.job.dense + kDenseCap - 1 : S.job.partial + kListCap - 1;
+  const uint32_t nr = dense ? S.job.w.ndr : S.job.w.npr;
   at = 0;
-  next = (uint32_t)lane < nr ? back[-lane] : make_uint2(0u, 0u);
+  uint2 ahead = (uint32_t)lane < nr ? back[-lane] : make_uint2(0u, 0u);
   uint32_t tot = 0, base = 0, before = 0, cnt = 0, excl = 0;
   for (;;) {
     while (held < (uint32_t)E::kPartBatch) {
@@ -749,10 +766,10 @@ __device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S,
         continue;
       }
       if (at >= nr) break;
-      uint2 e = next;
+      uint2 e = ahead;
       at += 32;
       const uint32_t j = at + (uint32_t)lane;
-      next = j < nr ? back[-(int)j] : make_uint2(0u, 0u);
+      ahead = j < nr ? back[-(int)j] : make_uint2(0u, 0u);
       const bool hit = (e.y & sel) != 0u;
       const uint32_t m = __ballot_sync(kFull, hit);
       if (!m) continue;
@@ -861,7 +878,6 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
   for (;;) {
     const uint32_t ngroups = a.st->n_groups, ntargets = a.st->n_targets;
     const bool two_pass = ngroups <= a.nslots;
-    const size_t wid = (size_t)blockIdx.x * kWalkWarps + warp;
     uint32_t next = 0;
     if (lane == 0) next = atomicAdd(J.jobs ? &a.st->walk_next2 : &a.st->walk_next, 1u);
     next = __shfl_sync(kFull, next, 0);
@@ -890,6 +906,10 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
     }
     J.w = Walk{0u, 0u, 0u, 0u, 0u, 0u};
     set_units(S, a.sys[J.sys].hw);
+    // the dense list is the warp's, the partial one the warp's or (two-pass schedule) the group's
+    const size_t wid = (size_t)blockIdx.x * kWalkWarps + warp;
+    J.dense = a.dlist + wid * kDenseCap;
+    J.partial = a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap;
     if (J.jobs) {
       if (J.k == 1) continue;  // done whole by its group
       uint32_t len = ld_volatile(a.gnl + J.gi);
@@ -928,13 +948,10 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
         J.w.top = 1, J.w.steps = 0;
         __syncwarp();
       }
-      // the lists: the dense one is the warp's, the partial one the warp's or
-      // (two-pass schedule) the group's
       do {
         uint32_t pass = J.pass1;
         if (!J.jobs) {
-          const bool more = traverse(a, S, a.prm[J.sys].theta2, a.dlist + wid * kDenseCap,
-                                     a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap, lane);
+          const bool more = traverse(a, S, a.prm[J.sys].theta2, J.dense, J.partial, lane);
           // all passes when the partial list is full or complete, else the dense one
           const bool all = more ? J.w.npc + J.w.npr + 64 > kListCap : !(two_pass && J.k > 1);
           J.more = more;
@@ -945,8 +962,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
         E ev(a, S, lane, a.prm[J.sys].eps2);
         for (; pass <= J.pass1; ++pass) {
           const bool dense = pass == 0;
-          const uint32_t nc = dense ? J.w.ndc : J.w.npc, nr = dense ? J.w.ndr : J.w.npr;
-          if (nc + nr == 0) continue;
+          if ((dense ? J.w.ndc + J.w.ndr : J.w.npc + J.w.npr) == 0) continue;
           const uint32_t i = pass - 1;
           const uint32_t tn = dense ? min(J.n - J.b0, (uint32_t)kGroupMax) : S.tcnt[i];
           {
@@ -955,9 +971,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
             ev.setup(dense ? J.p0 + J.b0 : S.tbeg[i], (int)tn, 0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]),
                      0.5 * (lo[2] + hi[2]));
           }
-          list_pass(ev, a, S,
-                    dense ? a.dlist + wid * kDenseCap : a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap, nc,
-                    dense ? kDenseCap : kListCap, nr, dense, dense ? kFull : 1u << i, tn, lane);
+          list_pass(ev, a, S, dense, dense ? kFull : 1u << i, tn, lane);
           ev.finish((int)tn, S.acc + (dense ? 0u : S.tbeg[i] - J.p0));
         }
         __syncwarp();
