@@ -65,7 +65,7 @@ struct bhg_context {
   SysDev* sys = nullptr;
   SysParam* prm = nullptr;
   Nodes nd{};
-  uint32_t *level_lb = nullptr, *mark = nullptr, *targets = nullptr, *scan_lb = nullptr;
+  uint32_t *unit_counts = nullptr, *mark = nullptr, *targets = nullptr, *scan_lb = nullptr;
   uint32_t *groups = nullptr, *chunks = nullptr;
   double* accel = nullptr;
   std::vector<std::pair<void*, size_t>> text_scratch;  // cached buffers of the text calls
@@ -193,8 +193,7 @@ int ensure_nodes(bhg_context* c, size_t need) {
       (r = grow(c, &c->nd.info, cap)) || (r = grow(c, &c->nd.box, cap)) || (r = grow(c, &c->nd.mom, cap)) ||
       (r = grow(c, &c->nd.iab, cap * 6)) || (r = grow(c, &c->nd.wcom, cap)) || (r = grow(c, &c->nd.wlink, cap)) ||
       (r = grow(c, &c->nd.src, cap)) || (r = grow(c, &c->nd.parent, cap)) || (r = grow(c, &c->nd.upcnt, cap)) ||
-      (r = grow(c, &c->targets, cap)) || (r = grow(c, &c->groups, cap)) || (r = grow(c, &c->chunks, cap)) ||
-      (r = grow(c, &c->level_lb, cap / 32 + kLevels + 8)))
+      (r = grow(c, &c->targets, cap)) || (r = grow(c, &c->groups, cap)) || (r = grow(c, &c->chunks, cap)))
     return r;
   c->nd.cap = (uint32_t)cap;
   c->cap_nodes = cap;
@@ -262,7 +261,10 @@ int ensure_particles(bhg_context* c, size_t n, int nsys, size_t ntiles, size_t n
     ntiles = std::max(ntiles, c->cap_tiles + c->cap_tiles / 2);
     drop_graph(c);
     c->cap_tiles = 0;
-    if ((r = grow(c, &c->tiles, ntiles)) || (r = grow(c, &c->partial, ntiles * 6))) return r;
+    // the node kernels' counts: kLevels per unit (eight units per tile where tiles are few)
+    if ((r = grow(c, &c->tiles, ntiles)) || (r = grow(c, &c->partial, ntiles * 6)) ||
+        (r = grow(c, &c->unit_counts, std::max<size_t>(ntiles, 8 * std::min<size_t>(ntiles, 256)) * kLevels)))
+      return r;
     c->cap_tiles = ntiles;
   }
   if (nstiles > c->cap_stiles) {
@@ -438,7 +440,7 @@ void enq_pre(bhg_context* c) {
   cudaMemsetAsync(reinterpret_cast<char*>(c->st) + kBuildResetOffset, 0, sizeof(DevState) - kBuildResetOffset, s);
   cudaMemsetAsync(c->hist, 0, (size_t)c->nsys * kSortPasses * 256 * sizeof(uint32_t), s);
   cudaMemsetAsync(c->sort_lb, 0, c->stiles_host.size() * kSortPasses * 256 * sizeof(uint32_t), s);
-  cudaMemsetAsync(c->level_lb, 0, (c->cap_nodes / 32 + kLevels + 8) * sizeof(uint32_t), s);
+  cudaMemsetAsync(c->nd.info, 0, c->cap_nodes * sizeof(uint32_t), s);
   launch_bounds_domain(c->part, c->tiles, nt, c->sys, c->nsys, c->partial, c->st, s);
   launch_keys(c->part, c->tiles, nt, c->sys, c->nsys, c->keys[0], c->hist, c->offs, s);
 }
@@ -453,8 +455,9 @@ void enq_sort(bhg_context* c) {
 void enq_tree(bhg_context* c) {
   // kSortPasses is even: sorted keys and the permutation are back in [0]
   launch_gather(c->part, c->vals[0], (uint32_t)c->n, c->staged, c->pm, c->sms, c->stream);
-  launch_topology(c->sys, c->nsys, c->nd, c->keys[0], c->max_leaf, (uint32_t)c->n, c->level_lb, c->st, c->sms,
-                  c->stream);
+  // the other value buffer is free after the sort
+  launch_topology(c->tiles, (int)c->tiles_host.size(), c->sys, c->nd, c->keys[0], c->max_leaf, c->vals[1],
+                  c->unit_counts, c->st, c->stream);
 }
 
 // Multipoles in one launch up to this many particles (the per-level launches
@@ -1480,11 +1483,11 @@ int bhg_get_stats(bhg_context* c, bhg_stats* out, int reset) {
   out->targets = c->st_host->n_targets;
   out->depth = c->st_host->max_depth;
   out->sort_passes = kSortPasses;
-  // bounds + domain + keys + digit offsets; the sort passes; gather + roots +
-  // one per level; the multipoles (one kernel, or one per level); mark +
+  // bounds + domain + keys + digit offsets; the sort passes; gather + the
+  // three topology kernels; the multipoles (one kernel, or one per level); mark +
   // compact of the targets, of the packing chunks, packing + compact of the
   // walk groups; the walk and its completion count
-  out->kernels_per_eval = 4 + kSortPasses + (2 + kMortonDepth) + (c->n <= kMomentsOneLaunchMax ? 1 : kMortonDepth + 1) + 6 +
+  out->kernels_per_eval = 4 + kSortPasses + 4 + (c->n <= kMomentsOneLaunchMax ? 1 : kMortonDepth + 1) + 6 +
                           2;
   if (reset) {
     for (double& t : c->tot_ms) t = 0.0;

@@ -442,42 +442,31 @@ __global__ void k_gather(const Particle* __restrict__ p, const uint32_t* __restr
 }
 
 // ---------------------------------------------------------------------------
-// a4: octree topology, one level per launch.
-// The root of system s is node s (level 0).  For a non-leaf parent at depth
-// d-1 holding sorted keys [b, e), its children are the non-empty octants of
-// the depth-d digit, in octant order (split_octants, flat_tree.h:167-180);
-// a node stops splitting at count <= max_leaf or depth 21 (LeafRule,
-// flat_tree.h:144-156); child centres are parent centre +- half of the
-// parent's half width (child_center, flat_tree.h:182-185).  Level d's nodes
-// are numbered in parent order (a block scan plus a look-back across tiles),
-// so the layout is breadth first and deterministic.
+// a4: octree topology, from the sorted keys alone.
+// The root of system s is node s (level 0).  A non-leaf node at depth d-1 has
+// the non-empty octants of the depth-d digit as children, in octant order
+// (split_octants, flat_tree.h:167-180); a node stops splitting at count <=
+// max_leaf or depth 21 (LeafRule, flat_tree.h:144-156); child centres are
+// parent centre +- half of the parent's half width (child_center,
+// flat_tree.h:182-185).  The nodes are numbered level by level, in particle
+// order within a level (parent order: breadth first, deterministic).
+//
+// A node is the run of particles that share its key prefix.  At which depths
+// a node starts at particle i follows from a few keys: no run starts there
+// above the first digit in which keys i-1 and i differ; the run that starts
+// at i at depth d holds more than max_leaf particles exactly when keys i and i
+// + max_leaf share their first d digits; and the first node of i exists when
+// its parent's run, which starts to the left of i, holds more than max_leaf.  So
+// the depths are a range of consecutive ones, found by every particle on its
+// own (k_node_depths); a scan of the counts per depth and unit of particles
+// (k_node_offsets) numbers the nodes, and k_node_emit writes them.  Three
+// launches that stream the keys twice, instead of one launch per level whose
+// blocks searched every octant's start: gather and topology take 0.025 ms
+// instead of 0.061 at 1,021 particles, 0.032 instead of 0.099 at 65k, 0.121
+// instead of 0.276 at 1M and 0.435 instead of 0.735 at 4M.
 
-__global__ void k_roots(const SysDev* __restrict__ sys, int nsys, Nodes nd, unsigned max_leaf, DevState* st) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) {
-    st->level_begin[0] = 0;
-    st->level_count[0] = (uint32_t)nsys;
-    st->level_begin[1] = (uint32_t)nsys;
-    st->max_depth = 1;
-    st->n_nodes = (uint32_t)nsys;
-  }
-  if (s >= nsys) return;
-  const SysDev& d = sys[s];
-  bool leaf = d.n <= max_leaf;  // depth 0 < 21
-  nd.begin[s] = d.begin;
-  nd.count[s] = d.n;
-  nd.first[s] = leaf ? d.begin : 0u;
-  nd.info[s] = (leaf ? 16u : 0u);
-  nd.box[s] = make_double4(d.cx, d.cy, d.cz, d.hw);
-  nd.parent[s] = kNoParent;
-  nd.upcnt[s] = 0u;
-}
-
-constexpr int kLevelThreads = 256;  // 8 threads (one per octant) per parent
-constexpr int kLevelParents = kLevelThreads / 8;
-// blocks per SM of a level launch (tiles are taken dynamically): the tree
-// phase at 4M takes 0.97 ms with 4, 0.74 with 8, 0.75 with 16
-constexpr int kLevelBlocksPerSm = 8;
+constexpr int kNodeThreads = 256;
+constexpr int kNodeWarps = kNodeThreads / 32;
 
 // The first index in [lo, hi) whose key is >= thr (hi if none; keys sorted),
 // by an 8-way search: each round loads 7 evenly spaced keys at once and keeps
@@ -500,96 +489,198 @@ __device__ __forceinline__ uint32_t first_at_least(const uint64_t* __restrict__ 
   return lo + m;
 }
 
-__global__ void __launch_bounds__(kLevelThreads) k_level(int depth, Nodes nd, const uint64_t* __restrict__ keys,
-                                                         unsigned max_leaf, uint32_t* __restrict__ lookback_all,
-                                                         DevState* st) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_scan[kLevelThreads / 32 + 2];
-  __shared__ uint32_t s_base;
-  const uint32_t pb = st->level_begin[depth - 1], pc = st->level_count[depth - 1];
-  const uint32_t cb = pb + pc;  // level_begin[depth]
-  if (cb > nd.cap) {  // an earlier level overflowed the slots: nothing to read here
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&st->status, kStNodeOverflow);
-    return;
+// Digits (of 21) that two keys share from the top.
+__device__ __forceinline__ int shared_digits(uint64_t a, uint64_t b) {
+  const uint64_t x = a ^ b;
+  return x ? (__clzll((long long)x) + 2) / 3 - 1 : kMortonDepth;
+}
+
+// The digits that key i shares with key i + max_leaf of its system [.., end),
+// -1 when there is none: the run of i at depth d is larger than max_leaf for
+// d up to this.
+__device__ __forceinline__ int large_to(const uint64_t* __restrict__ keys, uint32_t i, uint32_t end, unsigned max_leaf) {
+  return max_leaf < end - i ? shared_digits(keys[i], keys[i + max_leaf]) : -1;
+}
+
+// A unit: `unit` particles (a multiple of kNodeThreads) of a tile, by one block.
+__device__ __forceinline__ Tile node_unit(const Tile* __restrict__ tiles, uint32_t unit, uint32_t u) {
+  const uint32_t per = kTile / unit, off = (u % per) * unit;
+  Tile t = tiles[u / per];
+  t.start += off;
+  t.count = t.count > off ? min(t.count - off, unit) : 0u;
+  return t;
+}
+
+// depths[i]: bit d set when a node of depth d starts at particle i; counts:
+// [depth][unit].
+__global__ void __launch_bounds__(kNodeThreads) k_node_depths(const Tile* __restrict__ tiles, uint32_t unit,
+                                                              const SysDev* __restrict__ sys,
+                                                              const uint64_t* __restrict__ keys, unsigned max_leaf,
+                                                              uint32_t* __restrict__ depths,
+                                                              uint32_t* __restrict__ counts) {
+  __shared__ uint32_t cnt[kLevels];
+  if (threadIdx.x < kLevels) cnt[threadIdx.x] = 0u;
+  __syncthreads();
+  const Tile t = node_unit(tiles, unit, blockIdx.x);
+  const uint32_t begin = sys[t.sys].begin, end = begin + sys[t.sys].n;
+  for (uint32_t o = threadIdx.x; o < t.count; o += kNodeThreads) {
+    const uint32_t i = t.start + o;
+    const uint64_t key = keys[i];
+    // the first depth at which a run starts at i (22: none, equal keys)
+    const int first = i == begin ? 0 : shared_digits(keys[i - 1], key) + 1;
+    uint32_t mask = 0u;
+    if (first <= kMortonDepth) {
+      const int large = large_to(keys, i, end, max_leaf);
+      bool exists = first == 0 || large >= first - 1;
+      if (!exists) {
+        // the parent's run starts at s < i: is it larger than max_leaf?
+        const int sh = 63 - 3 * (first - 1);
+        const uint64_t prefix = key >> sh;
+        const uint32_t s = first_at_least(keys, i - begin > max_leaf ? i - max_leaf : begin, i, prefix << sh);
+        exists = i - s >= max_leaf || (max_leaf < end - s && keys[s + max_leaf] >> sh == prefix);
+      }
+      if (exists) {
+        const int last = min(max(first, large + 1), (int)kMortonDepth);
+        mask = (2u << last) - (1u << first);
+        for (int d = first; d <= last; ++d) atomicAdd(&cnt[d], 1u);
+      }
+    }
+    depths[i] = mask;
   }
-  const uint32_t ntiles = (pc + kLevelParents - 1) / kLevelParents;
-  uint32_t* lookback = lookback_all + pb / kLevelParents + depth;
-  const int tid = threadIdx.x, lane = tid & 31, oct = tid & 7;
-  const int csh = 63 - 3 * depth;  // digit shift at this depth
-  for (;;) {
-    if (tid == 0) s_tile = atomicAdd(&st->level_tiles[depth], 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    if (tile >= ntiles) break;
-    const uint32_t parent = pb + tile * kLevelParents + (tid >> 3);
-    const bool valid = parent < cb;
-    uint32_t b = 0, c = 0, info = 16u;
-    if (valid) {
-      b = nd.begin[parent];
-      c = nd.count[parent];
-      info = nd.info[parent];
+  __syncthreads();
+  if (threadIdx.x < kLevels) counts[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = cnt[threadIdx.x];
+}
+
+// Exclusive scan of each depth's counts over the units, one warp per depth,
+// and the levels' first nodes.  One block.
+__global__ void __launch_bounds__(32 * kLevels) k_node_offsets(uint32_t* __restrict__ counts, uint32_t units,
+                                                               uint32_t cap, DevState* st) {
+  __shared__ uint32_t total[32];
+  const uint32_t lane = threadIdx.x & 31u, d = threadIdx.x >> 5;
+  uint32_t* c = counts + (size_t)d * units;
+  uint32_t run = 0;
+  constexpr int kAhead = 8;  // loads in flight per lane
+  for (uint32_t base = 0; base < units; base += 32 * kAhead) {
+    uint32_t v[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const uint32_t u = base + 32 * j + lane;
+      v[j] = u < units ? c[u] : 0u;
     }
-    const bool split = valid && !info_leaf(info);
-    // octant o starts at the first key in [b, b+c) whose depth digit is >= o
-    uint32_t start = b;
-    if (split && oct > 0) {
-      const uint64_t cell = 1ull << (csh + 3);  // parent's cell size in keys
-      const uint64_t thr = (keys[b] & ~(cell - 1)) | ((uint64_t)oct << csh);
-      start = first_at_least(keys, b, b + c, thr);
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      const uint32_t u = base + 32 * j + lane, inc = warp_incl_scan(v[j]);
+      if (u < units) c[u] = run + inc - v[j];
+      run += __shfl_sync(0xffffffffu, inc, 31);
     }
-    uint32_t next = __shfl_down_sync(0xffffffffu, start, 1);
-    if (oct == 7) next = b + c;
-    const bool child = split && next > start;
-    const uint32_t grp = (__ballot_sync(0xffffffffu, child) >> (lane & ~7)) & 0xffu;
-    const uint32_t nch = __popc(grp);
-    const uint32_t rank = __popc(grp & ((1u << oct) - 1u));
-    // exclusive scan of nch over the tile's parents (counted once, at oct 0)
-    uint32_t total;
-    uint32_t pex = block_excl_scan<kLevelThreads>(oct == 0 ? nch : 0u, s_scan, &total);
-    pex = __shfl_sync(0xffffffffu, pex, lane & ~7);
-    if (tid == 0) {
-      const bool first = tile == 0;
-      st_volatile(&lookback[tile], (first ? kFlagPre : kFlagAgg) | total);
-      uint32_t excl = 0;
-      if (!first) {
-        excl = look_back(lookback, tile, 0, 1, st);
-        st_volatile(&lookback[tile], kFlagPre | (excl + total));
+  }
+  if (lane == 0) total[d] = run;
+  __syncthreads();
+  if (d != 0) return;
+  const uint32_t n = lane < kLevels ? total[lane] : 0u, inc = warp_incl_scan(n);
+  const uint32_t levels = (uint32_t)__popc(__ballot_sync(0xffffffffu, n != 0u));  // none is empty above the deepest
+  if (lane < kLevels) st->level_begin[lane] = inc - n, st->level_count[lane] = n;
+  if (lane == kLevels - 1) {
+    st->level_begin[kLevels] = inc;
+    st->n_nodes = inc;
+    st->max_depth = levels;
+    if (inc > cap) atomicOr(&st->status, kStNodeOverflow);
+  }
+}
+
+__global__ void __launch_bounds__(kNodeThreads) k_node_emit(const Tile* __restrict__ tiles, uint32_t unit,
+                                                            const SysDev* __restrict__ sys,
+                                                            const uint64_t* __restrict__ keys, unsigned max_leaf,
+                                                            const uint32_t* __restrict__ depths,
+                                                            const uint32_t* __restrict__ offsets, Nodes nd,
+                                                            const DevState* __restrict__ st) {
+  __shared__ uint32_t cnt[kNodeWarps][32];
+  const Tile t = node_unit(tiles, unit, blockIdx.x);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t le = lanemask_lt() | (1u << lane);
+  const uint32_t share = unit / kNodeWarps;  // particles of a warp, consecutive
+  const uint32_t o0 = warp * share, o1 = min(t.count, o0 + share);
+  // the warp's nodes per depth (lane d: depth d), then its first node of each
+  uint32_t base = 0;
+  for (uint32_t o = o0; o < o1; o += 32) {
+    const uint32_t mask = o + lane < o1 ? depths[t.start + o + lane] : 0u;
+    for (uint32_t any = __reduce_or_sync(0xffffffffu, mask); any; any &= any - 1) {
+      const int d = __ffs(any) - 1;
+      const uint32_t k = (uint32_t)__popc(__ballot_sync(0xffffffffu, (mask >> d) & 1u));
+      if ((int)lane == d) base += k;
+    }
+  }
+  cnt[warp][lane] = base;
+  __syncthreads();
+  if (lane < kLevels) {
+    base = st->level_begin[lane] + offsets[(size_t)lane * gridDim.x + blockIdx.x];
+    for (uint32_t w = 0; w < warp; ++w) base += cnt[w][lane];
+  }
+  const SysDev& sd = sys[t.sys];
+  const uint32_t end = sd.begin + sd.n;
+  for (uint32_t o = o0; o < o1; o += 32) {
+    const uint32_t i = t.start + o + lane;
+    const uint32_t mask = o + lane < o1 ? depths[i] : 0u;
+    const uint32_t any = __reduce_or_sync(0xffffffffu, mask);
+    if (!any) continue;
+    const int first = __ffs(mask) - 1;
+    uint64_t key = 0;
+    int large = -1;
+    double cx = 0.0, cy = 0.0, cz = 0.0, hw = 0.0;
+    uint32_t stop = end;  // end of the run one depth up
+    if (mask) {
+      key = keys[i];
+      large = large_to(keys, i, end, max_leaf);
+      cx = sd.cx, cy = sd.cy, cz = sd.cz, hw = sd.hw;
+    }
+    // depths from the one above the first node's (its parent is the last node
+    // of that depth that starts at or before the particle) to the deepest
+    const int lo = max(__ffs(any) - 2, 0), hi = 31 - __clz(any);
+    uint32_t prev = 0;  // nodes up to this particle, one depth up
+    if (mask)
+      for (int d = 1; d < lo; ++d) {  // the centre, down from the root
+        const uint32_t oct = (uint32_t)(key >> (63 - 3 * d)) & 7u;
+        hw = __dmul_rn(0.5, hw);
+        cx = (oct & 1) ? __dadd_rn(cx, hw) : __dsub_rn(cx, hw);
+        cy = (oct & 2) ? __dadd_rn(cy, hw) : __dsub_rn(cy, hw);
+        cz = (oct & 4) ? __dadd_rn(cz, hw) : __dsub_rn(cz, hw);
       }
-      s_base = cb + excl;
-      if (tile == ntiles - 1) {
-        const uint32_t end = cb + excl + total;
-        st->level_count[depth] = excl + total;
-        st->level_begin[depth + 1] = end;
-        st->n_nodes = end;
-        if (excl + total > 0) st->max_depth = depth + 1;
-        if (end > nd.cap) atomicOr(&st->status, kStNodeOverflow);
+    for (int d = lo; d <= hi; ++d) {
+      const uint32_t m = __ballot_sync(0xffffffffu, (mask >> d) & 1u);
+      const uint32_t upto = __shfl_sync(0xffffffffu, base, d) + (uint32_t)__popc(m & le);
+      if ((int)lane == d) base += (uint32_t)__popc(m);
+      if (mask && d > 0) {
+        const uint32_t oct = (uint32_t)(key >> (63 - 3 * d)) & 7u;
+        hw = __dmul_rn(0.5, hw);
+        cx = (oct & 1) ? __dadd_rn(cx, hw) : __dsub_rn(cx, hw);
+        cy = (oct & 2) ? __dadd_rn(cy, hw) : __dsub_rn(cy, hw);
+        cz = (oct & 4) ? __dadd_rn(cz, hw) : __dsub_rn(cz, hw);
       }
-    }
-    __syncthreads();
-    const uint32_t firstc = s_base + pex;
-    if (child) {
-      const uint32_t ci = firstc + rank;
-      if (ci < nd.cap) {
-        const uint32_t cnt = next - start;
-        const bool leaf = cnt <= max_leaf || depth >= kMortonDepth;
-        const double4 pbx = nd.box[parent];
-        const double q = __dmul_rn(0.5, pbx.w);
-        nd.begin[ci] = start;
-        nd.count[ci] = cnt;
-        nd.first[ci] = leaf ? start : 0u;
-        nd.info[ci] = (leaf ? 16u : 0u) | ((uint32_t)depth << 8);
-        nd.parent[ci] = parent;
-        nd.upcnt[ci] = 0u;
-        nd.box[ci] = make_double4((oct & 1) ? __dadd_rn(pbx.x, q) : __dsub_rn(pbx.x, q),
-                                  (oct & 2) ? __dadd_rn(pbx.y, q) : __dsub_rn(pbx.y, q),
-                                  (oct & 4) ? __dadd_rn(pbx.z, q) : __dsub_rn(pbx.z, q), q);
+      if ((mask >> d) & 1u) {
+        const uint32_t idx = upto - 1u, par = prev - 1u;
+        const int sh = 63 - 3 * d;
+        const uint64_t next = ((key >> sh) + 1u) << sh;  // past the run's keys
+        const bool small = d > large;
+        const uint32_t e = small ? first_at_least(keys, i + 1u, max_leaf < stop - i ? i + max_leaf : stop, next)
+                                 : first_at_least(keys, i + max_leaf + 1u, stop, next);
+        stop = e;
+        const bool leaf = small || d >= kMortonDepth;
+        if (idx < nd.cap) {
+          nd.begin[idx] = i;
+          nd.count[idx] = e - i;
+          if (leaf) nd.first[idx] = i;
+          nd.box[idx] = make_double4(cx, cy, cz, hw);
+          nd.parent[idx] = d ? par : kNoParent;
+          nd.upcnt[idx] = 0u;
+          // the bits of a node's word are added by several threads (zeroed before)
+          atomicAdd(&nd.info[idx], (leaf ? 16u : 0u) | ((uint32_t)d << 8));
+          if (d) atomicAdd(&nd.info[par], 1u);
+        }
+        // the first child starts where its parent does
+        if (d > first && par < nd.cap) nd.first[par] = idx;
       }
+      prev = upto;
     }
-    if (split && oct == 0 && parent < nd.cap) {
-      nd.first[parent] = firstc;
-      nd.info[parent] = info | nch;
-    }
-    __syncthreads();
   }
 }
 
@@ -941,22 +1032,16 @@ static int grid_for(uint64_t units, uint64_t per_block, int cap) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(b, (uint64_t)cap));
 }
 
-// The nodes of level d-1 (the parents k_level reads) are at most 8^(d-1)
-// per root, at most n, and at most 8 per interior node of the level above
-// (an interior node holds more than max_leaf particles: at most
-// n / (max_leaf + 1) of them per level), so the upper levels launch only the
-// blocks that can find a tile.
-void launch_topology(const SysDev* sys, int nsys, const Nodes& nd, const uint64_t* keys, unsigned max_leaf, uint32_t n,
-                     uint32_t* lookback, DevState* st, int sms, cudaStream_t s) {
-  k_roots<<<(nsys + 127) / 128, 128, 0, s>>>(sys, nsys, nd, max_leaf, st);
-  const uint64_t below = std::min<uint64_t>(n, 8 * ((uint64_t)n / ((uint64_t)max_leaf + 1) + (uint64_t)nsys));
-  uint64_t width = (uint64_t)nsys;  // 8^(d-1) per root
-  for (int d = 1; d <= kMortonDepth; ++d) {
-    const uint64_t parents = std::min(width, below);
-    k_level<<<grid_for(parents, kLevelParents, sms * kLevelBlocksPerSm), kLevelThreads, 0, s>>>(d, nd, keys, max_leaf,
-                                                                                               lookback, st);
-    width = std::min<uint64_t>(width * 8, 1ull << 40);
-  }
+// Particles per unit: a tile, or an eighth of one where there are few tiles
+// (more blocks; the one block that scans the counts takes 3 us for 2,000 units).
+uint32_t node_unit_size(int ntiles) { return ntiles <= 256 ? kTile / 8 : kTile; }
+
+void launch_topology(const Tile* tiles, int ntiles, const SysDev* sys, const Nodes& nd, const uint64_t* keys,
+                     unsigned max_leaf, uint32_t* depths, uint32_t* counts, DevState* st, cudaStream_t s) {
+  const uint32_t unit = node_unit_size(ntiles), units = (uint32_t)ntiles * (kTile / unit);
+  k_node_depths<<<units, kNodeThreads, 0, s>>>(tiles, unit, sys, keys, max_leaf, depths, counts);
+  k_node_offsets<<<1, 32 * kLevels, 0, s>>>(counts, units, nd.cap, st);
+  k_node_emit<<<units, kNodeThreads, 0, s>>>(tiles, unit, sys, keys, max_leaf, depths, counts, nd, st);
 }
 
 // Grids of the cut kernels (tiles and nodes taken by grid stride or by a

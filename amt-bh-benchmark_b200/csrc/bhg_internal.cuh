@@ -97,7 +97,6 @@ struct DevState {
   uint32_t max_depth;
   uint32_t level_begin[kLevels + 1];
   uint32_t level_count[kLevels + 1];
-  uint32_t level_tiles[kLevels + 1];  // tiles taken by each level kernel
   uint32_t sort_tiles[16];            // tiles taken by each sort pass
   // per walk (zeroed by every walk)
   uint32_t n_targets;

@@ -105,3 +105,22 @@ def test_repeated_shapes_give_the_same_bits():
                 ctx.step(fp, 8, 256, 16, 0.01, 0.02)
             got = ctx.download().tobytes()
             assert ref.setdefault(what, got) == got, what
+
+
+@pytest.mark.parametrize("leaf", [1, 2, 16, 255, 5000])
+def test_topology_sizes_match_oracle(gpu, oracle, leaf):
+    """The octree at particle counts around a warp's, a unit's and a tile's
+    share, with runs of equal keys (depth-21 leaves) across them."""
+    for n in (1, 2, 31, 33, 255, 257, 511, 513, 4095, 4097, 8193):
+        parts = cube(n, 200 + n)
+        parts["pos"][n // 3: n // 3 + n // 5] = parts["pos"][0]
+        dom, sk, perm, mp, t = _oracle_build(oracle, parts, leaf)
+        gpu.upload(parts)
+        gpu.build_tree(leaf, 256)
+        gpu.compute_multipoles()
+        g = gpu.tree()
+        assert g["n"] == t["n"], n
+        for k in ("begin", "count", "first_child", "nchild", "leaf", "depth"):
+            assert np.array_equal(g[k], t[k][:t["n"]]), (n, k)
+        for k in ("center", "hw", "mass", "com", "iab"):
+            assert np.array_equal(g[k], np.asarray(t[k][:t["n"]]), equal_nan=True), (n, k)
