@@ -307,7 +307,7 @@ int walk_grid(bhg_context* c) {
 // (walk_slot_bytes(), ~34 KB each) - one per warp in the one-pass schedule,
 // one per group in the two-pass schedule, which therefore serves as many
 // groups as there are slots: 32 per SM, 4,736 on a 148-SM B200 (161 MB, and
-// 58 MB of dense lists).  Allocated before the walk is captured (walk_grid has
+// 58 MB of dense lists), fewer for contexts of fewer particles.  Allocated before the walk is captured (walk_grid has
 // also set the kernels' shared-memory limit by then).  Under a tight HBM
 // budget there are fewer and the walk runs on as many blocks as have both per
 // warp (at least one block): a group's result does not depend on the warp
@@ -318,8 +318,10 @@ constexpr size_t kSlotsPerSm = 32;
 int ensure_walk_scratch(bhg_context* c, int grid) {
   const size_t per_slot = walk_slot_bytes(), per_dense = walk_dense_bytes();
   const size_t wpb = walk_threads() / 32;
-  size_t warps = (size_t)grid * wpb;
-  size_t slots = std::max(warps, kSlotsPerSm * (size_t)c->sms / wpb * wpb);
+  // a context of few particles has no more jobs than particles
+  const size_t jobs = (c->n + wpb - 1) / wpb * wpb;
+  size_t warps = std::min((size_t)grid * wpb, jobs);
+  size_t slots = std::max(warps, std::min(kSlotsPerSm * (size_t)c->sms / wpb * wpb, jobs));
   if (c->list_warps >= slots && c->dense_warps >= warps) return BHG_OK;
   if (c->budget) {
     const size_t held = c->list_warps * per_slot + c->dense_warps * per_dense;  // freed below, so it counts as room
@@ -498,18 +500,11 @@ void enq_walk(bhg_context* c, bool want_accel) {
   a.out = c->part;
   a.accel = want_accel ? c->accel : nullptr;
   a.st = c->st;
-  // the slots' lists, then the groups' sums, the list lengths, the dense lists
-  a.nslots = (uint32_t)c->list_warps;
-  a.wlist = static_cast<uint2*>(c->list_buf);
-  a.gsum = reinterpret_cast<double*>(
-      reinterpret_cast<char*>(c->list_buf) +
-      c->list_warps * (walk_slot_bytes() - kGroupMax * 3 * sizeof(double) - sizeof(uint32_t)));
-  a.gnl = reinterpret_cast<uint32_t*>(a.gsum + c->list_warps * kGroupMax * 3);
-  a.dlist = reinterpret_cast<uint2*>(reinterpret_cast<char*>(c->list_buf) + c->list_warps * walk_slot_bytes());
-  // list lengths "pending" (bytes 0xfe): the two-pass schedule's target jobs
-  // wait for their group's length
-  cudaMemsetAsync(a.gnl, 0xfe, c->list_warps * sizeof(uint32_t), c->stream);
-  launch_walk(a, c->precision, c->quad != 0, c->mask, walk_launch_grid(c), c->stream);
+  walk_scratch(a, c->list_buf, c->list_warps);
+  // list lengths and progress "pending" (bytes 0xfe): the two-pass schedule's
+  // jobs wait for their group's
+  cudaMemsetAsync(a.gnl, 0xfe, 2 * c->list_warps * sizeof(uint32_t), c->stream);
+  launch_walk(a, (uint32_t)c->n, c->precision, c->quad != 0, c->mask, walk_launch_grid(c), c->stream);
   launch_eval_done(c->st, c->stream);
 }
 

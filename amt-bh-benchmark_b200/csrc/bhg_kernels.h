@@ -71,17 +71,21 @@ struct WalkArgs {
   uint2* wlist;
   double* gsum;
   uint32_t* gnl;
+  uint32_t* prog;  // per slot: what a group's traversal has written of its dense list
+  uint32_t* plen;  // per slot: the lengths of its partial list
   uint32_t nslots;
 };
 
 // Walks every target and kicks/drifts its particles.  precision:
-// 0 = split (FP32 offsets and FP32 interactions, FP64 sums), 1 = FP64.
-void launch_walk(const WalkArgs& a, int precision, bool quad, bool mask, int grid, cudaStream_t s);
+// 0 = split (FP32 offsets and FP32 interactions, FP64 sums), 1 = FP64.  n:
+// particles.
+void launch_walk(const WalkArgs& a, uint32_t n, int precision, bool quad, bool mask, int grid, cudaStream_t s);
 int walk_blocks_per_sm(int precision, bool quad, bool mask);
 int walk_threads();
 // device bytes of one list slot, and of one warp's dense list
 size_t walk_slot_bytes();
 size_t walk_dense_bytes();
+void walk_scratch(WalkArgs& a, void* base, size_t slots);
 
 void launch_integrate(Particle* p, const double* accel, uint32_t n, const SysDev* sys, const SysParam* prm, int nsys,
                       int sms, cudaStream_t s);

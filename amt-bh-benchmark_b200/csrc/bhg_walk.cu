@@ -37,6 +37,7 @@
 // kick/drift of integrate_ttg.h:74-77 is applied in FP64 in the epilogue.
 #include "bhg_walk.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace bhg {
@@ -67,6 +68,15 @@ struct Walk {
   uint32_t ndc, ndr, npc, npr;  // dense cells and runs, partial cells and runs
 };
 
+// Jobs of the walk (k_walk): a group's traversal (and whatever passes no
+// other job takes), a group's dense pass beside it, a target's pass.
+enum : uint32_t { kWholeJob, kDenseJob, kTargetJob };
+// A group's progress (the word the host fills with kListPending before every
+// walk): cells in its dense list so far; or kFinal | runs << 12 | cells; or
+// kAborted, when the traversal paused and evaluates its lists itself.
+constexpr uint32_t kFinal = 1u << 31, kAborted = 1u << 30;
+static_assert(kDenseCap < 1u << 12, "two lengths and the flags share a word");
+
 // A warp's job, kept in shared memory (every lane writes the same values, a
 // __syncwarp away from reads of older ones): the evaluation loops need the
 // registers.
@@ -75,7 +85,9 @@ struct Job {
   uint32_t t0, k, p0, sys;  // the group's first target, targets, first particle, system
   uint32_t n, b0;          // particles; a large target's batch start
   uint32_t pass1;          // the last pass to run
-  uint32_t more, jobs;     // the traversal paused; this is a target job
+  uint32_t more, kind;     // the traversal paused; kWholeJob, kDenseJob or kTargetJob
+  uint32_t poll, aborted;  // dense jobs: cells are still to come; the traversal paused
+  uint32_t left, told;     // left to the dense job; the traversal's cells published so far
   uint2 *dense, *partial;  // the lists
   Walk w;
 };
@@ -89,6 +101,7 @@ struct WarpSmem {
   double glo[3], ghi[3];                            // the group's particle box
   double centre[3], scale, scale2, eps2;            // evaluators' reference point and units
   unsigned long long ncell, npart;                  // interactions of this warp
+  unsigned long long kept[2];                       // of them, before a dense job that may be aborted
   Job job;
   uint32_t tbeg[kMaxTargets], tcnt[kMaxTargets];    // the targets' particles
   uint32_t ring[kRing];
@@ -565,10 +578,13 @@ __device__ __forceinline__ float far2f(const float lo[3], const float hi[3], flo
   return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
 }
 
+// prog: where to publish the cells written so far (a dense job evaluates
+// them meanwhile), or null.
 // Returns true when a list may be too full for another step (the lists are
 // then to be taken and reset, and the traversal goes on where it stopped).
+template <bool PAIRS>
 __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double theta2, uint2* __restrict__ dl,
-                                         uint2* __restrict__ pl, int lane) {
+                                         uint2* __restrict__ pl, uint32_t* prog, int lane) {
   const uint32_t k = S.job.k;
   Walk w = S.job.w;
   const uint32_t lt = lanemask_lt();
@@ -586,6 +602,7 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
   }
   const float inv_theta2 = (float)(1.0 / theta2);
   const uint32_t max_steps = a.st->n_nodes + 2;  // a walk pops each node at most once
+  S.job.told = 0u;
   bool more = false;
   while (w.top) {
     if (w.ndc + w.ndr + 32 > kDenseCap || w.npc + w.npr + 64 > kListCap) {
@@ -673,6 +690,12 @@ __device__ __forceinline__ bool traverse(const WalkArgs& a, WarpSmem& S, double 
     uint32_t m = __ballot_sync(kFull, dc);
     if (dc) dl[w.ndc + __popc(m & lt)] = make_uint2(node, 1u);
     w.ndc += __popc(m);
+    if (PAIRS && prog && w.ndc - S.job.told >= 64) {  // the dense job may take them
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) st_volatile(prog, w.ndc);
+      S.job.told = w.ndc;
+    }
     m = __ballot_sync(kFull, pc);
     if (pc) pl[w.npc + __popc(m & lt)] = make_uint2(node, A);
     w.npc += __popc(m);
@@ -705,11 +728,38 @@ __device__ __forceinline__ uint4 load_pair(const uint4* p, uint32_t i, uint32_t 
   return v;
 }
 
+// A dense job's wait (bounded) for cells beyond `at` (a multiple of 64): the
+// cells that may be read, a multiple of 64 too unless they are all.
+__device__ __forceinline__ uint32_t more_cells(const WalkArgs& a, WarpSmem& S, uint32_t at, int lane) {
+  Job& J = S.job;
+  uint32_t v = 0;
+  for (int spins = 0;; ++spins) {
+    v = ld_volatile(a.prog + J.gi);
+    v = __shfl_sync(kFull, v == kListPending ? 0u : v, 0);
+    if ((v & (kFinal | kAborted)) || (v & ~63u) > at) break;
+    if (spins >= kSpinLimit) {
+      if (lane == 0) atomicOr(&a.st->status, kStSpinLimit);
+      v = kAborted;
+      break;
+    }
+    __nanosleep(64);
+  }
+  __threadfence();  // the cells after the word
+  if (!(v & (kFinal | kAborted))) return v & ~63u;
+  __syncwarp();
+  J.poll = 0u;
+  J.aborted = v & kAborted ? 1u : 0u;
+  J.w.ndc = J.aborted ? at : v & 0xfffu;
+  J.w.ndr = J.aborted ? 0u : (v >> 12) & 0xfffu;
+  __syncwarp();
+  return J.w.ndc;
+}
+
 // Evaluates the entries of the job's dense or partial list that `sel` picks
 // (bits of the entry's second word) on the evaluator's tn targets: first the
 // cells, then the runs.  Windows of 64 cells or 32 runs, the next one loaded
 // while the current one is used, fill a ring; full batches of it are evaluated.
-template <class E>
+template <bool PAIRS, class E>
 __device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S, bool dense, uint32_t sel, uint32_t tn,
                                           int lane) {
   const uint32_t lt = lanemask_lt();
@@ -717,10 +767,16 @@ __device__ __forceinline__ void list_pass(E& ev, const WalkArgs& a, WarpSmem& S,
   // two entries per lane and window (16-byte loads; the list's end is read as
   // entries that nothing picks)
   const uint4* pairs = reinterpret_cast<const uint4*>(dense ? S.job.dense : S.job.partial) + lane;
-  const uint32_t nc = dense ? S.job.w.ndc : S.job.w.npc;
+  uint32_t nc = dense ? S.job.w.ndc : S.job.w.npc;
   uint4 next = load_pair(pairs, 2u * lane, nc);
   for (;;) {
-    while (held < (uint32_t)E::kCellBatch && at < nc) {
+    while (held < (uint32_t)E::kCellBatch) {
+      if (at >= nc) {
+        if (!PAIRS || !S.job.poll) break;
+        nc = more_cells(a, S, at, lane);
+        next = load_pair(pairs, at + 2u * lane, nc);
+        continue;
+      }
       const uint4 e = next;
       at += 64;
       pairs += 32;
@@ -862,11 +918,16 @@ __device__ __forceinline__ uint32_t group_boxes(const WalkArgs& a, WarpSmem& S, 
 // groups of one target whole), each leaving its group's FP64 sums and partial
 // list in the group's slot and publishing the list's lengths; then they take
 // every target's pass as a job of its own, starting as soon as the group's
-// lengths are published.  A job waits only for a group whose walk a running
-// warp has taken, so every wait ends; a wait is still bounded (kStSpinLimit,
-// the job skipped).  Both schedules run the same passes and add their parts
-// in the same order, so the results are the same bits.
-template <class E, bool QUAD>
+// lengths are published.  With fewer groups still (two warps for each), a
+// group's dense pass is a job of its own too, which takes the cells while the
+// traversal finds them; if that has to pause, it evaluates its lists itself.  A
+// job waits only for jobs handed out before it, which running warps hold and
+// which wait for none or for such jobs, so every wait ends; a wait is still
+// bounded (kStSpinLimit, the job skipped).  All schedules run the same passes
+// on the same batches and add their parts in the same order, so the results
+// are the same bits.  Walk with / without dense jobs: 0.25 / 0.34 ms
+// at 16k, 0.42 / 0.56 at 65k, 0.63 / 0.72 at 40k in FP64.
+template <class E, bool QUAD, bool PAIRS>
 __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -874,15 +935,15 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
   if (a.st->status & (kStNonFinite | kStNodeOverflow | kStSpinLimit)) return;  // the build failed: touch nothing
   Job& J = S.job;
   if (lane == 0) S.ncell = S.npart = 0ull;
-  J.jobs = 0u;
+  J.kind = kWholeJob;
   for (;;) {
     const uint32_t ngroups = a.st->n_groups, ntargets = a.st->n_targets;
-    const bool two_pass = ngroups <= a.nslots;
+    const bool two_pass = ngroups <= a.nslots, paired = PAIRS && two_pass && 2 * ngroups <= gridDim.x * kWalkWarps;
     uint32_t next = 0;
-    if (lane == 0) next = atomicAdd(J.jobs ? &a.st->walk_next2 : &a.st->walk_next, 1u);
+    if (lane == 0) next = atomicAdd(J.kind == kTargetJob ? &a.st->walk_next2 : &a.st->walk_next, 1u);
     next = __shfl_sync(kFull, next, 0);
     __syncwarp();  // every lane is done with the last job
-    if (J.jobs) {
+    if (J.kind == kTargetJob) {
       if (next >= ntargets) break;
       // its group: the last whose first target is at or before it
       uint32_t gi = 0, hi = ngroups;
@@ -894,8 +955,10 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
       J.gi = gi, J.ti = next;
     } else if (next < ngroups) {
       J.gi = next;
+    } else if (paired && next < 2 * ngroups) {
+      J.gi = next - ngroups, J.kind = kDenseJob;
     } else if (two_pass) {
-      J.jobs = 1u;
+      J.kind = kTargetJob;
       continue;
     } else {
       break;
@@ -904,14 +967,17 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
       const GroupInfo g = group_info(a, J.gi, ngroups, ntargets);
       J.t0 = g.t0, J.k = g.k, J.p0 = g.p0, J.sys = g.s;
     }
+    if (J.kind != kWholeJob && J.k == 1) continue;  // done whole by its group
     J.w = Walk{0u, 0u, 0u, 0u, 0u, 0u};
     set_units(S, a.sys[J.sys].hw);
-    // the dense list is the warp's, the partial one the warp's or (two-pass schedule) the group's
+    // the partial list is the warp's or (two-pass schedule) the group's, the
+    // dense one the warp's or (with dense jobs) the group's
     const size_t wid = (size_t)blockIdx.x * kWalkWarps + warp;
-    J.dense = a.dlist + wid * kDenseCap;
+    J.dense = a.dlist + (paired ? (size_t)J.gi : wid) * kDenseCap;
     J.partial = a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap;
-    if (J.jobs) {
-      if (J.k == 1) continue;  // done whole by its group
+    J.poll = J.kind == kDenseJob;
+    J.aborted = 0u;
+    if (J.kind == kTargetJob) {
       uint32_t len = ld_volatile(a.gnl + J.gi);
       for (int spins = 0; len == kListPending && spins < kSpinLimit; ++spins) {
         __nanosleep(128);
@@ -938,31 +1004,46 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
       __syncwarp();
     } else {
       J.n = group_boxes(a, S, lane);
+      J.pass1 = 0u;
+      if (lane == 0) S.kept[0] = S.ncell, S.kept[1] = S.npart;
     }
     for (uint32_t b0 = 0; b0 < J.n; b0 += kGroupMax) {  // once, but for a large target
       J.b0 = b0;
-      if (!J.jobs) {
+      if (J.kind != kTargetJob) {
         for (uint32_t i = lane; i < 3 * kGroupMax; i += 32) (&S.acc[0][0])[i] = 0.0;
         // the traversal starts with the root
         S.stack[0] = make_uint2(a.sys[J.sys].root, ((1u << J.k) - 1u) | (1u << 24));
         J.w.top = 1, J.w.steps = 0;
         __syncwarp();
       }
+      J.left = 0u;
       do {
         uint32_t pass = J.pass1;
-        if (!J.jobs) {
-          const bool more = traverse(a, S, a.prm[J.sys].theta2, J.dense, J.partial, lane);
+        J.more = 0u;
+        if (J.kind == kWholeJob) {
+          const bool beside = paired && J.k > 1 && !J.aborted;  // a dense job evaluates beside
+          const bool more =
+              traverse<PAIRS>(a, S, a.prm[J.sys].theta2, J.dense, J.partial, beside ? a.prog + J.gi : nullptr, lane);
+          if (beside) {
+            if (!more && lane == 0) a.plen[J.gi] = J.w.npc | (J.w.npr << 16);
+            __threadfence();  // the lists before the word
+            __syncwarp();
+            if (lane == 0) st_volatile(a.prog + J.gi, more ? kAborted : kFinal | (J.w.ndr << 12) | J.w.ndc);
+            if (!more) {
+              J.left = 1u;
+              break;
+            }
+            J.aborted = 1u;
+          }
           // all passes when the partial list is full or complete, else the dense one
           const bool all = more ? J.w.npc + J.w.npr + 64 > kListCap : !(two_pass && J.k > 1);
           J.more = more;
           pass = 0, J.pass1 = all && J.w.npc + J.w.npr ? J.k : 0u;
-        } else {
-          J.more = 0u;
         }
         E ev(a, S, lane, a.prm[J.sys].eps2);
         for (; pass <= J.pass1; ++pass) {
           const bool dense = pass == 0;
-          if ((dense ? J.w.ndc + J.w.ndr : J.w.npc + J.w.npr) == 0) continue;
+          if ((dense ? J.w.ndc + J.w.ndr + J.poll : J.w.npc + J.w.npr) == 0) continue;
           const uint32_t i = pass - 1;
           const uint32_t tn = dense ? min(J.n - J.b0, (uint32_t)kGroupMax) : S.tcnt[i];
           {
@@ -971,7 +1052,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
             ev.setup(dense ? J.p0 + J.b0 : S.tbeg[i], (int)tn, 0.5 * (lo[0] + hi[0]), 0.5 * (lo[1] + hi[1]),
                      0.5 * (lo[2] + hi[2]));
           }
-          list_pass(ev, a, S, dense, dense ? kFull : 1u << i, tn, lane);
+          list_pass<PAIRS>(ev, a, S, dense, dense ? kFull : 1u << i, tn, lane);
           ev.finish((int)tn, S.acc + (dense ? 0u : S.tbeg[i] - J.p0));
         }
         __syncwarp();
@@ -979,15 +1060,21 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
         if (J.pass1) J.w.npc = J.w.npr = 0;
         __syncwarp();
       } while (J.more);
+      if (J.left) continue;  // to the dense job
+      if (J.kind == kDenseJob && J.aborted) {  // the group's own job evaluates its lists
+        if (lane == 0) S.ncell = S.kept[0], S.npart = S.kept[1];
+        continue;
+      }
       const uint32_t nb = min(J.n - J.b0, (uint32_t)kGroupMax);
-      if (two_pass && J.k > 1 && !J.jobs) {  // leave the sums and the partial list to the target jobs
+      if (two_pass && J.k > 1 && J.kind != kTargetJob) {  // leave the sums and the partial list to the target jobs
         double* gs = a.gsum + (size_t)J.gi * (kGroupMax * 3);
         for (uint32_t i = lane; i < 3 * nb; i += 32) gs[i] = (&S.acc[0][0])[i];
         __threadfence();  // the sums and the list before the lengths
         __syncwarp();
-        if (lane == 0) st_volatile(a.gnl + J.gi, J.w.npc | (J.w.npr << 16));
+        if (lane == 0)
+          st_volatile(a.gnl + J.gi, J.kind == kDenseJob ? __ldcg(a.plen + J.gi) : J.w.npc | (J.w.npr << 16));
       } else {
-        const uint32_t off = J.jobs ? S.tbeg[J.ti - J.t0] - J.p0 : 0u;
+        const uint32_t off = J.kind == kTargetJob ? S.tbeg[J.ti - J.t0] - J.p0 : 0u;
         kick_drift(a, a.prm[J.sys], S.acc + off, J.p0 + off + J.b0, nb, lane);
       }
     }
@@ -999,27 +1086,40 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
 }
 
 template <class E, bool QUAD>
-static void launch_one(const WalkArgs& a, int grid, cudaStream_t s) {
-  k_walk<E, QUAD><<<grid, kWalkThreads, kWalkSmem, s>>>(a);
+static void launch_one(const WalkArgs& a, uint32_t n, int grid, cudaStream_t s) {
+  // Dense jobs pay from 4,096 particles on (with / without: 0.178 / 0.182 ms
+  // there; 0.091 / 0.086 at 1,021, whose dense lists are too short to share
+  // out).  Groups hold at most kGroupMax particles (or one large target, which
+  // has no dense job): with more than this there are never two warps for
+  // each, and the kernel without dense jobs is 0.6% faster.
+  if (n >= 4096u && n <= (uint32_t)grid * kWalkWarps / 2 * kGroupMax)
+    k_walk<E, QUAD, true><<<grid, kWalkThreads, kWalkSmem, s>>>(a);
+  else k_walk<E, QUAD, false><<<grid, kWalkThreads, kWalkSmem, s>>>(a);
 }
 
 // Unsoftened split walks have a kernel of their own (bhg_walk_unsoftened.cu).
-void launch_walk(const WalkArgs& a, int precision, bool quad, bool mask, int grid, cudaStream_t s) {
+void launch_walk(const WalkArgs& a, uint32_t n, int precision, bool quad, bool mask, int grid, cudaStream_t s) {
   if (precision == 0) {
     if (mask) launch_walk_unsoftened(a, quad, grid, s);
-    else quad ? launch_one<SplitEval<true>, true>(a, grid, s) : launch_one<SplitEval<false>, false>(a, grid, s);
+    else quad ? launch_one<SplitEval<true>, true>(a, n, grid, s) : launch_one<SplitEval<false>, false>(a, n, grid, s);
   } else {
-    if (quad) mask ? launch_one<F64Eval<true, true>, true>(a, grid, s) : launch_one<F64Eval<true, false>, true>(a, grid, s);
-    else mask ? launch_one<F64Eval<false, true>, false>(a, grid, s) : launch_one<F64Eval<false, false>, false>(a, grid, s);
+    if (quad) mask ? launch_one<F64Eval<true, true>, true>(a, n, grid, s) : launch_one<F64Eval<true, false>, true>(a, n, grid, s);
+    else mask ? launch_one<F64Eval<false, true>, false>(a, n, grid, s) : launch_one<F64Eval<false, false>, false>(a, n, grid, s);
   }
+}
+
+template <class E, bool QUAD, bool PAIRS>
+static int occ_of() {
+  const auto k = k_walk<E, QUAD, PAIRS>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem);
+  int b = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, kWalkThreads, kWalkSmem);
+  return b > 0 ? b : 1;
 }
 
 template <class E, bool QUAD>
 static int occ() {
-  cudaFuncSetAttribute(k_walk<E, QUAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkSmem);
-  int b = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_walk<E, QUAD>, kWalkThreads, kWalkSmem);
-  return b > 0 ? b : 1;
+  return std::min(occ_of<E, QUAD, true>(), occ_of<E, QUAD, false>());
 }
 
 static int walk_blocks_per_sm_query(int precision, bool quad, bool mask) {
@@ -1042,10 +1142,24 @@ int walk_blocks_per_sm(int precision, bool quad, bool mask) {
 
 int walk_threads() { return kWalkThreads; }
 
-// Device bytes of one list slot: the partial list, and the group's FP64 sums
-// and list lengths for the two-pass schedule; and of a warp's dense list.
-size_t walk_slot_bytes() { return kListCap * sizeof(uint2) + kGroupMax * 3 * sizeof(double) + sizeof(uint32_t); }
+// Device bytes of one list slot: the partial list, and for the two-pass
+// schedule the group's FP64 sums, list lengths, progress and partial lengths;
+// and of a dense list.
+size_t walk_slot_bytes() { return kListCap * sizeof(uint2) + kGroupMax * 3 * sizeof(double) + 3 * sizeof(uint32_t); }
 size_t walk_dense_bytes() { return kDenseCap * sizeof(uint2); }
+
+// Lays the slots out over `base`: the lists, sums, lengths and progress words
+// (from a.gnl on 2 * slots words, to be filled with kListPending's bytes
+// before every walk), partial lengths, dense lists.
+void walk_scratch(WalkArgs& a, void* base, size_t slots) {
+  a.nslots = (uint32_t)slots;
+  a.wlist = static_cast<uint2*>(base);
+  a.gsum = reinterpret_cast<double*>(a.wlist + slots * kListCap);
+  a.gnl = reinterpret_cast<uint32_t*>(a.gsum + slots * kGroupMax * 3);
+  a.prog = a.gnl + slots;
+  a.plen = a.prog + slots;
+  a.dlist = reinterpret_cast<uint2*>(a.plen + slots);
+}
 
 // ---------------------------------------------------------------------------
 // Unfused integrate phase: kick_one / drift_one (integrate.h:15-16) with
