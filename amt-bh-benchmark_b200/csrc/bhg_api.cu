@@ -71,6 +71,10 @@ struct bhg_context {
   std::vector<std::pair<void*, size_t>> text_scratch;  // cached buffers of the text calls
   DevState* st = nullptr;
   DevState* st_host = nullptr;  // pinned
+  // a snapshot's copies to the host run beside its formatting
+  cudaStream_t copy_stream = nullptr;
+  cudaEvent_t copy_ev[4] = {};
+  uint64_t* vtk_totals = nullptr;  // pinned
 
   // phase state
   bool built = false, moments = false, walked = false;
@@ -703,6 +707,10 @@ int bhg_destroy(bhg_context* c) {
   for (auto& a : c->allocs) cudaFree(a.first);
   c->allocs.clear();
   if (c->st_host) cudaFreeHost(c->st_host);
+  if (c->vtk_totals) cudaFreeHost(c->vtk_totals);
+  for (auto& ev : c->copy_ev)
+    if (ev) cudaEventDestroy(ev);
+  if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
   for (auto& ev : c->ev_all)
     if (ev) cudaEventDestroy(ev);
   for (auto& ev : c->cap_ev)
@@ -937,6 +945,24 @@ struct Scratch {
   }
 };
 
+// Parts of a snapshot (bhg_snapshot_vtk) and the tiles from which it pays
+// to part it: 500,009 particles (3,907 tiles) into pinned memory take 0.91 ms in
+// one part, 0.81 in four (0.65 the copy alone, 1.08 before).
+constexpr uint32_t kVtkParts = 4, kVtkPartTiles = 512;
+
+// The copy stream, events and pinned totals, made by the first snapshot.
+int snapshot_resources(bhg_context* c) {
+  static_assert(kVtkParts <= sizeof(bhg_context::copy_ev) / sizeof(cudaEvent_t), "an event per part");
+  if (!c->copy_stream) CK(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+  for (auto& ev : c->copy_ev)
+    if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  if (!c->vtk_totals && cudaMallocHost(&c->vtk_totals, 3 * kVtkParts * sizeof(uint64_t)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(c, BHG_ENOMEM, "no pinned memory for the snapshot's totals");
+  }
+  return BHG_OK;
+}
+
 // read_csv's header rule (io.cc:136-141): the first line is a header when its
 // first field (after blanks) does not parse as an id.
 bool csv_has_header(const char* text, size_t n) {
@@ -1078,44 +1104,58 @@ int bhg_snapshot_vtk(bhg_context* c, uint64_t handle, char* out, size_t cap, siz
   size_t start = 0;
   for (size_t k = 0; k < sidx; ++k) start += c->counts[k];
   const uint32_t n = (uint32_t)c->counts[sidx];
+  int r = snapshot_resources(c);
+  if (r) return r;
   Scratch sc(c);
-  char* slots = nullptr;
-  uint32_t* lens = nullptr;
-  uint32_t* bsum = nullptr;
-  uint64_t* boff = nullptr;
-  uint64_t* totals = nullptr;
-  int r;
-  if ((r = sc.get(&slots, vtk_slot_bytes(n))) || (r = sc.get(&lens, 3 * (size_t)n)) ||
-      (r = sc.get(&bsum, 3 * vtk_blocks(n))) || (r = sc.get(&boff, 3 * vtk_blocks(n))) || (r = sc.get(&totals, 3)))
+  char *pieces = nullptr, *sect[3] = {nullptr, nullptr, nullptr};
+  uint32_t* sums = nullptr;
+  uint64_t *off = nullptr, *totals = nullptr;
+  const uint32_t tiles = vtk_tiles(n);
+  if ((r = sc.get(&pieces, vtk_piece_bytes(n))) || (r = sc.get(&sect[0], vtk_piece_bytes(n))) ||
+      (r = sc.get(&sums, 3 * (size_t)tiles)) || (r = sc.get(&off, 3 * (size_t)tiles)) || (r = sc.get(&totals, 3)))
     return r;
-  launch_vtk_format(c->part + start, n, slots, lens, bsum, boff, totals, c->sms, c->stream);
-  CK(cudaGetLastError());
-  uint64_t t[3];
-  CK(cudaMemcpyAsync(t, totals, sizeof t, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  sect[1] = sect[0] + vtk_section_bytes(n, 0), sect[2] = sect[1] + vtk_section_bytes(n, 1);
+  CK(cudaMemsetAsync(totals, 0, 3 * sizeof(uint64_t), c->stream));
   // write_vtk's layout (io.cc:180-195)
   const std::string h0 = "# vtk DataFile Version 3.0\npepc-ttg particle snapshot\nASCII\nDATASET POLYDATA\nPOINTS " +
                          std::to_string(n) + " double\n";
   const std::string h1 = "POINT_DATA " + std::to_string(n) + "\nSCALARS mass double 1\nLOOKUP_TABLE default\n";
   const std::string h2 = "VECTORS velocity double\n";
+  // In several parts, so that the points of one are copied to the host while
+  // the next is formatted (the other sections' places need the points' total);
+  // only into a buffer that holds any snapshot of n particles, else nothing is
+  // written before the size is known.
+  const bool early = out && cap >= vtk_most_bytes(n) + h0.size() + h1.size() + h2.size();
+  const uint32_t parts = early && tiles >= kVtkPartTiles ? kVtkParts : 1;
+  auto first = [&](uint32_t k) { return (uint32_t)((uint64_t)tiles * k / parts); };
+  for (uint32_t k = 0; k < parts; ++k) {
+    launch_vtk_tiles(c->part + start, n, first(k), first(k + 1) - first(k), pieces, sums, off, totals,
+                     c->vtk_totals + 3 * k, sect, c->stream);
+    CK(cudaEventRecord(c->copy_ev[k], c->stream));
+  }
+  CK(cudaGetLastError());
+  uint64_t t[3] = {0, 0, 0};
+  for (uint32_t k = 0; k < parts; ++k) {
+    CK(cudaEventSynchronize(c->copy_ev[k]));
+    const uint64_t from = t[0];
+    for (int q = 0; q < 3; ++q) t[q] = c->vtk_totals[3 * k + q];
+    if (early && t[0] > from)
+      CK(cudaMemcpyAsync(out + h0.size() + from, sect[0] + from, t[0] - from, cudaMemcpyDeviceToHost, c->copy_stream));
+  }
   const size_t total = h0.size() + t[0] + h1.size() + t[1] + h2.size() + t[2];
   *len = total;
   if (!out) return BHG_OK;
   if (cap < total) return fail(c, BHG_EINVAL, "buffer too small: the snapshot needs " + std::to_string(total) + " bytes");
-  char* dev = nullptr;
-  if ((r = sc.get(&dev, t[0] + t[1] + t[2]))) return r;
-  char* sect[3] = {dev, dev + t[0], dev + t[0] + t[1]};
-  launch_vtk_gather(slots, n, lens, boff, sect, c->stream);
-  CK(cudaGetLastError());
   const std::string* head[3] = {&h0, &h1, &h2};
   size_t at = 0;
   for (int k = 0; k < 3; ++k) {
     std::memcpy(out + at, head[k]->data(), head[k]->size());
     at += head[k]->size();
-    if (t[k]) CK(cudaMemcpyAsync(out + at, sect[k], t[k], cudaMemcpyDeviceToHost, c->stream));
+    if (t[k] && !(k == 0 && early))
+      CK(cudaMemcpyAsync(out + at, sect[k], t[k], cudaMemcpyDeviceToHost, c->copy_stream));
     at += t[k];
   }
-  CK(cudaStreamSynchronize(c->stream));
+  CK(cudaStreamSynchronize(c->copy_stream));
   return BHG_OK;
 }
 

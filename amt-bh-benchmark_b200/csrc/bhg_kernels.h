@@ -106,9 +106,7 @@ double measure_fp32_peak(int device);
 // scan of the tile counts (total newlines to *total), then the line starts
 // (newlines + 1 of them), then one parse per line of [first, nlines), then
 // the compaction of the particle lines (kept count to *total; dst may be
-// null to count only).  Snapshot: formats the three text lines of every
-// particle into slots (lengths, exclusive offsets and the three section
-// totals), then gathers each section back to back.
+// null to count only).
 size_t csv_tiles(size_t nbytes);
 void launch_csv_count(const char* text, size_t n, uint32_t* tile_count, uint64_t* total, cudaStream_t s);
 void launch_csv_emit(const char* text, size_t n, const uint32_t* tile_off, uint64_t* line_start, cudaStream_t s);
@@ -117,12 +115,16 @@ void launch_csv_parse(const char* text, size_t n, const uint64_t* line_start, ui
 size_t csv_keep_blocks(uint64_t m);
 void launch_csv_compact(const Particle* tmp, const uint32_t* keep, uint64_t m, uint32_t* block_count,
                         uint64_t* total, Particle* dst, cudaStream_t s);
-size_t vtk_slot_bytes(uint32_t n);
-size_t vtk_blocks(uint32_t n);
-void launch_vtk_format(const Particle* p, uint32_t n, char* slots, uint32_t* len, uint32_t* block_sum,
-                       uint64_t* block_off, uint64_t* totals, int sms, cudaStream_t s);
-void launch_vtk_gather(const char* slots, uint32_t n, const uint32_t* len, const uint64_t* block_off,
-                       char* const out[3], cudaStream_t s);
+// Tiles [tile0, tile0 + count) of a snapshot's vtk_tiles(n) tiles, in order:
+// formatted into their pieces (vtk_piece_bytes), placed in the three sections
+// out[k] (vtk_section_bytes each) after the text that totals[k] counts (0
+// before the first); the totals so far also to host memory.
+uint32_t vtk_tiles(uint32_t n);
+size_t vtk_section_bytes(uint32_t n, int k);
+size_t vtk_piece_bytes(uint32_t n);
+size_t vtk_most_bytes(uint32_t n);  // the three sections together are never longer
+void launch_vtk_tiles(const Particle* p, uint32_t n, uint32_t tile0, uint32_t count, char* pieces, uint32_t* sums,
+                      uint64_t* off, uint64_t* totals, uint64_t* host_totals, char* const out[3], cudaStream_t s);
 
 // n particles of one Plummer sphere (scale a, total mass `mass`, centre c[3],
 // bulk velocity b[3], ids id0..), drawn from a counter-based generator keyed

@@ -124,3 +124,20 @@ def test_topology_sizes_match_oracle(gpu, oracle, leaf):
             assert np.array_equal(g[k], t[k][:t["n"]]), (n, k)
         for k in ("center", "hw", "mass", "com", "iab"):
             assert np.array_equal(g[k], np.asarray(t[k][:t["n"]]), equal_nan=True), (n, k)
+
+
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 3000, 65541])
+def test_snapshot_sizes_match_oracle(oracle, n):
+    """Snapshots around a tile's particles, in one part and in several, into a
+    buffer that holds any snapshot (copied as it is formatted) and into one of
+    exactly its size; one byte less is refused."""
+    parts = cube(n, 70 + n, spread=1e-3)
+    parts["vel"] = np.random.default_rng(n).normal(size=(n, 3)) * 10.0 ** np.random.default_rng(n).integers(-9, 9, (n, 1))
+    want = oracle.write_vtk(parts)
+    with bhg.Context(device=0) as ctx:
+        ctx.upload(parts)
+        assert ctx.snapshot_vtk() == want
+        exact = np.zeros(len(want), np.uint8)
+        assert ctx.snapshot_vtk_into(exact) == len(want) and exact.tobytes() == want
+        with pytest.raises(bhg.BhgError):
+            ctx.snapshot_vtk_into(np.zeros(len(want) - 1, np.uint8))
