@@ -1208,7 +1208,8 @@ void launch_eval_done(DevState* st, cudaStream_t s) { k_eval_done<<<1, 1, 0, s>>
 // that any number of rows fills the GPU (about 8 blocks of 128 threads per
 // SM), and the parts are added in order by k_direct_add.  Bound by the FP64
 // pipe: 17 operations per pair, 5 of them the reciprocal square root.
-// The call with 4,096 rows of 1,048,576 particles takes 7.5 ms; with one row
+// The call with 4,096 rows of 1,048,576 particles takes 6.6 ms (7.5 with a
+// branch of its own for each row's reciprocal); with one row
 // per 8 threads, 128 blocks, a division and a square root per pair and the
 // particles repacked by the host 66.7 ms.
 
@@ -1217,11 +1218,13 @@ constexpr int kDirThreads = 128;
 
 // 1 / (x sqrt(x)): an approximate reciprocal square root (about 20 bits) and
 // one step of Householder's third-order iteration, y (1 + e / 2 + 3 e^2 / 8)
-// with e = 1 - x y^2, which triples its bits.  Values far enough from the ends of
-// the range for that (all but zero, the smallest and the largest): else the
-// plain quotient.
+// with e = 1 - x y^2, which triples its bits; for values far enough from the
+// ends of the range (2^-600 .. 2^600), `ordinary`.  Others - zero, the smallest,
+// the largest, NaN - take the plain quotient.
+__device__ __forceinline__ bool ordinary(double x) {
+  return (uint32_t)__double2hiint(x) - (423u << 20) <= (1200u << 20);
+}
 __device__ __forceinline__ double inv_r3(double x) {
-  if ((uint32_t)__double2hiint(x) - (423u << 20) > (1200u << 20)) return 1.0 / (x * sqrt(x));  // not in 2^-600 .. 2^600
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-(x * y), y, 1.0);
@@ -1255,14 +1258,17 @@ __global__ void __launch_bounds__(kDirThreads, 8) k_direct(const Particle* __res
     const uint32_t cnt = min((uint32_t)kDirThreads, end - base);
     for (uint32_t k = sub; k < cnt; k += nsub) {
       const double4 s = src[k];
-      double dx = s.x - x0, dy = s.y - y0, dz = s.z - z0;
-      double c = s.w * inv_r3(dx * dx + dy * dy + dz * dz + eps2);
-      c = base + k == me0 ? 0.0 : c;  // not itself
-      a0x += c * dx, a0y += c * dy, a0z += c * dz;
-      dx = s.x - x1, dy = s.y - y1, dz = s.z - z1;
-      c = s.w * inv_r3(dx * dx + dy * dy + dz * dz + eps2);
-      c = base + k == me1 ? 0.0 : c;
-      a1x += c * dx, a1y += c * dy, a1z += c * dz;
+      const double d0x = s.x - x0, d0y = s.y - y0, d0z = s.z - z0;
+      const double d1x = s.x - x1, d1y = s.y - y1, d1z = s.z - z1;
+      const double v0 = d0x * d0x + d0y * d0y + d0z * d0z + eps2, v1 = d1x * d1x + d1y * d1y + d1z * d1z + eps2;
+      // one branch for both rows, so that their chains run side by side
+      double c0, c1;
+      if (ordinary(v0) && ordinary(v1)) c0 = inv_r3(v0), c1 = inv_r3(v1);
+      else c0 = 1.0 / (v0 * sqrt(v0)), c1 = 1.0 / (v1 * sqrt(v1));
+      c0 = base + k == me0 ? 0.0 : s.w * c0;  // not itself
+      c1 = base + k == me1 ? 0.0 : s.w * c1;
+      a0x += c0 * d0x, a0y += c0 * d0y, a0z += c0 * d0z;
+      a1x += c1 * d1x, a1y += c1 * d1y, a1z += c1 * d1z;
     }
   }
   double* r = red[threadIdx.x];
