@@ -66,7 +66,7 @@ struct bhg_context {
   SysParam* prm = nullptr;
   Nodes nd{};
   uint32_t *unit_counts = nullptr, *mark = nullptr, *targets = nullptr, *scan_lb = nullptr;
-  uint32_t *groups = nullptr, *chunks = nullptr;
+  uint32_t *groups = nullptr, *restart = nullptr;
   double* accel = nullptr;
   std::vector<std::pair<void*, size_t>> text_scratch;  // cached buffers of the text calls
   DevState* st = nullptr;
@@ -197,16 +197,16 @@ int ensure_nodes(bhg_context* c, size_t need) {
       (r = grow(c, &c->nd.info, cap)) || (r = grow(c, &c->nd.box, cap)) || (r = grow(c, &c->nd.mom, cap)) ||
       (r = grow(c, &c->nd.iab, cap * 6)) || (r = grow(c, &c->nd.wcom, cap)) || (r = grow(c, &c->nd.wlink, cap)) ||
       (r = grow(c, &c->nd.src, cap)) || (r = grow(c, &c->nd.parent, cap)) || (r = grow(c, &c->nd.upcnt, cap)) ||
-      (r = grow(c, &c->targets, cap)) || (r = grow(c, &c->groups, cap)) || (r = grow(c, &c->chunks, cap)))
+      (r = grow(c, &c->targets, cap)) || (r = grow(c, &c->groups, cap)) || (r = grow(c, &c->restart, cap)))
     return r;
   c->nd.cap = (uint32_t)cap;
   c->cap_nodes = cap;
   return BHG_OK;
 }
 
-// Look-back words of the three compactions of the walk targets, groups and
-// packing chunks (one word per 4096-item tile each, and some slack).
-size_t scan_words(size_t n) { return 3 * (n / 4096) + 48; }
+// Look-back words of the two compactions of the walk targets and groups (one
+// word per 4096-item tile each, and some slack).
+size_t scan_words(size_t n) { return 2 * (n / 4096) + 48; }
 
 // Particle-sized buffers and the per-system tables for n particles.  The
 // state (c->part) keeps its first c->n particles across a growth, so
@@ -443,10 +443,12 @@ int ensure_layout(bhg_context* c) {
 void enq_pre(bhg_context* c) {
   cudaStream_t s = c->stream;
   const int nt = (int)c->tiles_host.size();
-  cudaMemsetAsync(reinterpret_cast<char*>(c->st) + kBuildResetOffset, 0, sizeof(DevState) - kBuildResetOffset, s);
-  cudaMemsetAsync(c->hist, 0, (size_t)c->nsys * kSortPasses * 256 * sizeof(uint32_t), s);
-  cudaMemsetAsync(c->sort_lb, 0, c->stiles_host.size() * kSortPasses * 256 * sizeof(uint32_t), s);
-  cudaMemsetAsync(c->nd.info, 0, c->cap_nodes * sizeof(uint32_t), s);
+  FillList f;
+  f.add(reinterpret_cast<char*>(c->st) + kBuildResetOffset, sizeof(DevState) - kBuildResetOffset, 0);
+  f.add(c->hist, (size_t)c->nsys * kSortPasses * 256 * sizeof(uint32_t), 0);
+  f.add(c->sort_lb, c->stiles_host.size() * kSortPasses * 256 * sizeof(uint32_t), 0);
+  f.add(c->nd.info, c->cap_nodes * sizeof(uint32_t), 0);
+  launch_fill(f, c->sms, s);
   launch_bounds_domain(c->part, c->tiles, nt, c->sys, c->nsys, c->partial, c->st, s);
   launch_keys(c->part, c->tiles, nt, c->sys, c->nsys, c->keys[0], c->hist, c->offs, s);
 }
@@ -478,10 +480,17 @@ void enq_moments(bhg_context* c) {
 
 void enq_targets(bhg_context* c, uint32_t target_size) {
   cudaStream_t s = c->stream;
-  cudaMemsetAsync(reinterpret_cast<char*>(c->st) + kWalkResetOffset, 0, sizeof(DevState) - kWalkResetOffset, s);
-  cudaMemsetAsync(c->scan_lb, 0, scan_words(c->n) * sizeof(uint32_t), s);
+  WalkArgs a;
+  walk_scratch(a, c->list_buf, c->list_warps);
+  FillList f;
+  f.add(reinterpret_cast<char*>(c->st) + kWalkResetOffset, sizeof(DevState) - kWalkResetOffset, 0);
+  f.add(c->scan_lb, scan_words(c->n) * sizeof(uint32_t), 0);
+  // the walk's list lengths and progress "pending": the two-pass schedule's
+  // jobs wait for their group's
+  f.add(a.gnl, 2 * c->list_warps * sizeof(uint32_t), kWalkPending);
+  launch_fill(f, c->sms, s);
   const uint32_t lim = std::min(target_size, c->group_size);
-  launch_targets(c->nd, lim, c->walk_pack, (uint32_t)c->n, c->mark, c->targets, c->chunks, c->groups, c->scan_lb, c->st,
+  launch_targets(c->nd, lim, c->walk_pack, (uint32_t)c->n, c->mark, c->targets, c->restart, c->groups, c->scan_lb, c->st,
                  c->sms, s);
 }
 
@@ -505,9 +514,6 @@ void enq_walk(bhg_context* c, bool want_accel) {
   a.accel = want_accel ? c->accel : nullptr;
   a.st = c->st;
   walk_scratch(a, c->list_buf, c->list_warps);
-  // list lengths and progress "pending" (bytes 0xfe): the two-pass schedule's
-  // jobs wait for their group's
-  cudaMemsetAsync(a.gnl, 0xfe, 2 * c->list_warps * sizeof(uint32_t), c->stream);
   launch_walk(a, (uint32_t)c->n, c->precision, c->quad != 0, c->mask, walk_launch_grid(c), c->stream);
   launch_eval_done(c->st, c->stream);
 }
@@ -1518,12 +1524,11 @@ int bhg_get_stats(bhg_context* c, bhg_stats* out, int reset) {
   out->targets = c->st_host->n_targets;
   out->depth = c->st_host->max_depth;
   out->sort_passes = kSortPasses;
-  // bounds + domain + keys + digit offsets; the sort passes; gather + the
-  // three topology kernels; the multipoles (one kernel, or one per level); mark +
-  // compact of the targets, of the packing chunks, packing + compact of the
-  // walk groups; the walk and its completion count
-  out->kernels_per_eval = 4 + kSortPasses + 4 + (c->n <= kMomentsOneLaunchMax ? 1 : kMortonDepth + 1) + 6 +
-                          2;
+  // resets + bounds + domain + keys + digit offsets; the sort passes; gather + the
+  // three topology kernels; the multipoles (one kernel, or one per level);
+  // resets + mark + compact of the targets, packing + compact of the walk
+  // groups; the walk and its completion count
+  out->kernels_per_eval = 5 + kSortPasses + 4 + (c->n <= kMomentsOneLaunchMax ? 1 : kMortonDepth + 1) + 5 + 2;
   if (reset) {
     for (double& t : c->tot_ms) t = 0.0;
     c->walks_timed = 0;

@@ -85,6 +85,13 @@ void launch_wait_probe(const uint32_t* words, uint32_t tile, int limit, DevState
   k_wait_probe<<<1, 32, 0, s>>>(words, tile, limit, st, out);
 }
 
+// Several ranges of words set in one launch (a launch or a memset costs about
+// 1.6 us of a small evaluation each).
+__global__ void __launch_bounds__(256) k_fill(FillList f) {
+  for (int r = 0; r < f.n; ++r)
+    for (size_t i = blockIdx.x * 256u + threadIdx.x; i < f.words[r]; i += gridDim.x * 256u) f.p[r][i] = f.v[r];
+}
+
 // ---------------------------------------------------------------------------
 // a1: bounds per tile, then the domain per system
 // particle_bounds (flat_build_ttg.h:93-113) + domain_from_bounds (domain.h:23-30)
@@ -685,24 +692,36 @@ __global__ void __launch_bounds__(kNodeThreads) k_node_emit(const Tile* __restri
 }
 
 // ---------------------------------------------------------------------------
-// Cuts of the tree: the topmost nodes that are leaves or hold at most `lim`
-// particles, marked at their first particle and compacted in Morton order.
-// Used for the walk targets (lim = min(target_size, group_size)); the same
+// Cuts of the tree: the topmost nodes that are leaves or hold at most a limit
+// of particles.  The walk targets (lim = min(target_size, group_size)) are
+// marked at their first particle, with kNoRestart unless a packing chunk (lim
+// = kPackChunk) starts there too, and compacted in Morton order; the same
 // compaction then lists the walk groups (k_pack_groups).
 
+constexpr uint32_t kPackChunk = 2048;
+constexpr uint32_t kNoRestart = 0x80000000u;  // of a mark; an empty mark has all other bits set
+
+// Marks are all ones before; the target's index and the chunk's start clear
+// the bits they do not have, in any order.
 __global__ void k_mark_cut(Nodes nd, uint32_t lim, const DevState* __restrict__ st, uint32_t* __restrict__ mark) {
   if (st->status & kStNodeOverflow) return;  // children may lie beyond the slots
   const uint32_t nn = min(st->n_nodes, nd.cap), nroots = st->level_count[0];
+  const auto put = [&](uint32_t i, bool target, bool chunk) {
+    const uint32_t bits = (target ? i | kNoRestart : 0xffffffffu) & (chunk ? ~kNoRestart : 0xffffffffu);
+    if (target || chunk) atomicAnd(&mark[nd.begin[i]], bits);
+  };
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += gridDim.x * blockDim.x) {
     const uint32_t info = nd.info[i], cnt = nd.count[i];
-    const bool cut = info_leaf(info) || cnt <= lim;
-    if (i < nroots && cut) mark[nd.begin[i]] = i;
-    if (!cut) {
+    const bool leaf = info_leaf(info), target = leaf || cnt <= lim, chunk = leaf || cnt <= kPackChunk;
+    if (i < nroots) put(i, target, chunk);
+    if (!target || !chunk) {
       const uint32_t f = nd.first[i], k = info_nchild(info);
       for (uint32_t j = 0; j < k; ++j) {
         const uint32_t ch = f + j;
         if (ch >= nd.cap) break;
-        if (info_leaf(nd.info[ch]) || nd.count[ch] <= lim) mark[nd.begin[ch]] = ch;
+        const bool cl = info_leaf(nd.info[ch]);
+        const uint32_t cc = nd.count[ch];
+        put(ch, !target && (cl || cc <= lim), !chunk && (cl || cc <= kPackChunk));
       }
     }
   }
@@ -711,10 +730,12 @@ __global__ void k_mark_cut(Nodes nd, uint32_t lim, const DevState* __restrict__ 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 
-// Compacts the marked entries of mark[0..n) into out (Morton order), resets
+// Compacts the marked entries of mark[0..n) into out (Morton order) without
+// their kNoRestart bits, whose complements go to restart (optional), resets
 // the marks, and writes the count.  Tiles chain through a decoupled look-back.
 __global__ void __launch_bounds__(kScanThreads) k_compact(uint32_t* __restrict__ mark, uint32_t n,
-                                                          uint32_t* __restrict__ out, uint32_t* __restrict__ lookback,
+                                                          uint32_t* __restrict__ out,
+                                                          uint32_t* __restrict__ restart, uint32_t* __restrict__ lookback,
                                                           uint32_t* tile_counter, uint32_t* count_out,
                                                           DevState* st) {
   __shared__ uint32_t s_tile, s_base;
@@ -730,7 +751,7 @@ __global__ void __launch_bounds__(kScanThreads) k_compact(uint32_t* __restrict__
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
       v[j] = base + j < n ? mark[base + j] : 0xffffffffu;
-      cnt += v[j] != 0xffffffffu;
+      cnt += (v[j] | kNoRestart) != 0xffffffffu;
     }
     uint32_t total;
     uint32_t ex = block_excl_scan<kScanThreads>(cnt, s_scan, &total);
@@ -748,7 +769,11 @@ __global__ void __launch_bounds__(kScanThreads) k_compact(uint32_t* __restrict__
     uint32_t o = s_base + ex;
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
-      if (v[j] != 0xffffffffu) out[o++] = v[j];
+      if ((v[j] | kNoRestart) != 0xffffffffu) {
+        out[o] = v[j] & ~kNoRestart;
+        if (restart) restart[o] = v[j] & kNoRestart ? 0u : 1u;
+        ++o;
+      }
       if (base + j < n) mark[base + j] = 0xffffffffu;  // ready for the next use
     }
     __syncthreads();
@@ -767,78 +792,53 @@ __global__ void __launch_bounds__(kScanThreads) k_compact(uint32_t* __restrict__
 // particles (or leaves) - one warp per chunk: a chunk lies inside one system
 // and its targets depend on that system alone, so a system's groups, and
 // with them its results bit for bit, do not depend on the other systems of
-// the context.  Group starts are marked at their first target's index for
-// the compaction.
-constexpr uint32_t kPackChunk = 2048;
+// the context.  Every chunk that a target starts in starts at a target (restart).
+// Group starts are marked at their first target's index for the compaction.
 constexpr int kPackWindows = 4;  // windows of 32 targets whose counts are loaded together
 
-// Index of the first target whose particles start at or after particle p
-// (the targets lie in particle order), by one warp: each round probes 32
-// evenly spaced targets and keeps the stretch between the last probe before
-// p and the first one at or after it.
-__device__ __forceinline__ uint32_t first_target_at(const uint32_t* __restrict__ targets,
-                                                    const uint32_t* __restrict__ nbegin, uint32_t nt, uint32_t p,
-                                                    int lane) {
-  uint32_t lo = 0, hi = nt;  // the answer lies in [lo, hi]
-  while (hi - lo > 32u) {
-    const uint32_t step = (hi - lo + 31u) / 32u;
-    const uint32_t q = lo + (uint32_t)lane * step;
-    const bool before = q < hi && nbegin[targets[q]] < p;
-    const uint32_t m = (uint32_t)__popc(__ballot_sync(0xffffffffu, before));  // probes 0 .. m-1 lie before p
-    const uint32_t nlo = m ? lo + (m - 1u) * step + 1u : lo;
-    hi = min(hi, lo + m * step);
-    lo = nlo;
-  }
-  const uint32_t q = lo + (uint32_t)lane;
-  const bool before = q < hi && nbegin[targets[q]] < p;
-  return lo + (uint32_t)__popc(__ballot_sync(0xffffffffu, before));
-}
-
-__global__ void k_pack_groups(const uint32_t* __restrict__ chunks, const uint32_t* __restrict__ targets,
-                              const uint32_t* __restrict__ nbegin, const uint32_t* __restrict__ ncount,
-                              uint32_t pack, const DevState* __restrict__ st, uint32_t* __restrict__ mark) {
+__global__ void k_pack_groups(const uint32_t* __restrict__ restart, const uint32_t* __restrict__ targets,
+                              const uint32_t* __restrict__ ncount, uint32_t pack, const DevState* __restrict__ st,
+                              uint32_t* __restrict__ mark) {
   if (st->status & kStNodeOverflow) return;
-  const uint32_t nchunks = st->n_chunks, nt = st->n_targets;
+  const uint32_t nt = st->n_targets;
   const int lane = threadIdx.x & 31;
-  const uint32_t wpb = blockDim.x >> 5;
-  for (uint32_t c = blockIdx.x * wpb + (threadIdx.x >> 5); c < nchunks; c += gridDim.x * wpb) {
-    const uint32_t cn = chunks[c];
-    const uint32_t cb = nbegin[cn], ce = cb + ncount[cn];
-    uint32_t cnt = 0, k = 0;
-    bool first = true, end = false;
-    for (uint32_t t0 = first_target_at(targets, nbegin, nt, cb, lane); !end; t0 += 32u * kPackWindows) {
-      // the particle counts of the next windows' targets (past the chunk: ~0)
-      uint32_t n[kPackWindows];
+  const uint32_t nw = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  for (uint32_t at = warp * 32u; at < nt; at += nw * 32u) {
+    uint32_t starts_here = __ballot_sync(0xffffffffu, at + lane < nt && restart[at + lane]);
+    for (; starts_here; starts_here &= starts_here - 1u) {
+      const uint32_t start = at + (uint32_t)__ffs(starts_here) - 1u;  // the chunk's first target
+      uint32_t cnt = 0, k = 0;
+      bool first = true, end = false;
+      for (uint32_t t0 = start; !end; t0 += 32u * kPackWindows) {
+        // the particle counts of the next windows' targets (past the chunk: ~0)
+        uint32_t n[kPackWindows];
 #pragma unroll
-      for (int w = 0; w < kPackWindows; ++w) {
-        const uint32_t t = t0 + 32u * w + (uint32_t)lane;
-        n[w] = 0xffffffffu;
-        if (t < nt) {
-          const uint32_t tn = targets[t];
-          if (nbegin[tn] < ce) n[w] = ncount[tn];
+        for (int w = 0; w < kPackWindows; ++w) {
+          const uint32_t t = t0 + 32u * w + (uint32_t)lane;
+          n[w] = t < nt && (t == start || !restart[t]) ? ncount[targets[t]] : 0xffffffffu;
         }
-      }
 #pragma unroll
-      for (int w = 0; w < kPackWindows; ++w) {
-        if (end) break;
-        // the greedy packing, run alike by every lane over the window's 32 counts
-        uint32_t starts = 0;
-        for (int i = 0; i < 32; ++i) {
-          const uint32_t ni = __shfl_sync(0xffffffffu, n[w], i);
-          if (ni == 0xffffffffu) {
-            end = true;
-            break;
+        for (int w = 0; w < kPackWindows; ++w) {
+          if (end) break;
+          // the greedy packing, run alike by every lane over the window's 32 counts
+          uint32_t starts = 0;
+          for (int i = 0; i < 32; ++i) {
+            const uint32_t ni = __shfl_sync(0xffffffffu, n[w], i);
+            if (ni == 0xffffffffu) {
+              end = true;
+              break;
+            }
+            if (first || cnt + ni > pack || k >= (uint32_t)kMaxTargets) {
+              starts |= 1u << i;
+              cnt = 0;
+              k = 0;
+              first = false;
+            }
+            cnt += ni;
+            ++k;
           }
-          if (first || cnt + ni > pack || k >= (uint32_t)kMaxTargets) {
-            starts |= 1u << i;
-            cnt = 0;
-            k = 0;
-            first = false;
-          }
-          cnt += ni;
-          ++k;
+          if ((starts >> lane) & 1u) mark[t0 + 32u * w + (uint32_t)lane] = t0 + 32u * w + (uint32_t)lane;
         }
-        if ((starts >> lane) & 1u) mark[t0 + 32u * w + (uint32_t)lane] = t0 + 32u * w + (uint32_t)lane;
       }
     }
   }
@@ -1017,6 +1017,12 @@ void launch_sort_pass(const uint64_t* kin, const uint32_t* vin, uint64_t* kout, 
                                                                       lookback, st);
 }
 
+void launch_fill(const FillList& f, int sms, cudaStream_t s) {
+  size_t most = 0;
+  for (int r = 0; r < f.n; ++r) most = std::max(most, f.words[r]);
+  k_fill<<<(unsigned)std::max<size_t>(1, std::min<size_t>((most + 1023) / 1024, (size_t)sms * 8)), 256, 0, s>>>(f);
+}
+
 void launch_gather(const Particle* p, const uint32_t* perm, uint32_t n, Particle* staged, double4* pm, int sms,
                    cudaStream_t s) {
   int blocks = (int)((n + 255) / 256);
@@ -1045,19 +1051,19 @@ void launch_topology(const Tile* tiles, int ntiles, const SysDev* sys, const Nod
 }
 
 // Grids of the cut kernels (tiles and nodes taken by grid stride or by a
-// counter): measured at 4M, the targets phase takes 0.179 ms with 4/2/2
-// blocks per SM and 0.140 with 16/8/8.
+// counter): measured at 4M with three compactions, the targets phase took
+// 0.179 ms with 4/2/2 blocks per SM and 0.140 with 16/8/8.  The packing chunks'
+// starts ride on the targets' marks: with a marking and a compaction of their
+// own the phase took 0.055 ms at 16k (now 0.038), 0.064 at 65k (0.047), 0.221
+// at 4M (0.186), resets included.
 void launch_targets(const Nodes& nd, uint32_t lim, uint32_t pack, uint32_t n, uint32_t* mark, uint32_t* targets,
-                    uint32_t* chunks, uint32_t* groups, uint32_t* lookback, DevState* st, int sms, cudaStream_t s) {
+                    uint32_t* restart, uint32_t* groups, uint32_t* lookback, DevState* st, int sms, cudaStream_t s) {
   const uint32_t ntiles = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
   const int gmark = grid_for(nd.cap, 256, sms * 16), gscan = grid_for(ntiles, 1, sms * 8);
   k_mark_cut<<<gmark, 256, 0, s>>>(nd, lim, st, mark);
-  k_compact<<<gscan, kScanThreads, 0, s>>>(mark, n, targets, lookback, &st->scan_tiles, &st->n_targets, st);
-  k_mark_cut<<<gmark, 256, 0, s>>>(nd, kPackChunk, st, mark);
-  k_compact<<<gscan, kScanThreads, 0, s>>>(mark, n, chunks, lookback + (ntiles + 8), &st->chunk_tiles, &st->n_chunks,
-                                           st);
-  k_pack_groups<<<sms * 4, 256, 0, s>>>(chunks, targets, nd.begin, nd.count, pack, st, mark);
-  k_compact<<<gscan, kScanThreads, 0, s>>>(mark, n, groups, lookback + 2 * (ntiles + 8), &st->group_tiles,
+  k_compact<<<gscan, kScanThreads, 0, s>>>(mark, n, targets, restart, lookback, &st->scan_tiles, &st->n_targets, st);
+  k_pack_groups<<<grid_for(n, 256, sms * 4), 256, 0, s>>>(restart, targets, nd.count, pack, st, mark);
+  k_compact<<<gscan, kScanThreads, 0, s>>>(mark, n, groups, nullptr, lookback + (ntiles + 8), &st->group_tiles,
                                            &st->n_groups, st);
 }
 

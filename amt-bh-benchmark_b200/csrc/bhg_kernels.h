@@ -18,6 +18,18 @@ void launch_keys(const Particle* p, const Tile* tiles, int ntiles, const SysDev*
 void launch_sort_pass(const uint64_t* kin, const uint32_t* vin, uint64_t* kout, uint32_t* vout, int pass,
                       const Tile* tiles, int ntiles, int tile_keys, const uint32_t* offs, uint32_t* lookback,
                       DevState* st, cudaStream_t s);
+// Ranges of words and the value each is set to, in one launch.
+struct FillList {
+  int n = 0;
+  uint32_t* p[4];
+  size_t words[4];
+  uint32_t v[4];
+  void add(void* at, size_t bytes, uint32_t value) {
+    p[n] = static_cast<uint32_t*>(at), words[n] = bytes / 4, v[n] = value;
+    ++n;
+  }
+};
+void launch_fill(const FillList& f, int sms, cudaStream_t s);
 void launch_gather(const Particle* p, const uint32_t* perm, uint32_t n, Particle* staged, double4* pm, int sms,
                    cudaStream_t s);
 // Octree topology of the sorted keys (nd.info zeroed before).  depths: n
@@ -35,11 +47,11 @@ void launch_topology(const Tile* tiles, int ntiles, const SysDev* sys, const Nod
 // pass) and target_size 0 both give the leaves.  The walk groups are runs of
 // consecutive targets of one system, at most `pack` particles and
 // kMaxTargets targets each (a larger target alone), packed inside chunks of
-// the tree (chunks: node-sized scratch): groups[g] is the index of group g's
-// first target, st->n_groups their number.  lookback: 3 regions of
+// the tree (restart: node-sized scratch): groups[g] is the index of group g's
+// first target, st->n_groups their number.  lookback: 2 regions of
 // n / 4096 + 9 words.
 void launch_targets(const Nodes& nd, uint32_t lim, uint32_t pack, uint32_t n, uint32_t* mark, uint32_t* targets,
-                    uint32_t* chunks, uint32_t* groups, uint32_t* lookback, DevState* st, int sms, cudaStream_t s);
+                    uint32_t* restart, uint32_t* groups, uint32_t* lookback, DevState* st, int sms, cudaStream_t s);
 // one_launch: k_moments_up (one kernel, children-first by counters) instead of
 // one kernel per level; the same bits either way
 void launch_moments(const Nodes& nd, const double4* pm, const DevState* st, int sms, bool one_launch, cudaStream_t s);
@@ -85,6 +97,8 @@ int walk_threads();
 // device bytes of one list slot, and of one warp's dense list
 size_t walk_slot_bytes();
 size_t walk_dense_bytes();
+// what the words from a.gnl on (2 * slots) are set to before every walk
+constexpr uint32_t kWalkPending = 0xfefefefeu;
 void walk_scratch(WalkArgs& a, void* base, size_t slots);
 
 void launch_integrate(Particle* p, const double* accel, uint32_t n, const SysDev* sys, const SysParam* prm, int nsys,

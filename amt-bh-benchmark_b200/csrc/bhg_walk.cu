@@ -71,8 +71,7 @@ struct Walk {
 // Jobs of the walk (k_walk): a group's traversal (and whatever passes no
 // other job takes), a group's dense pass beside it, a target's pass.
 enum : uint32_t { kWholeJob, kDenseJob, kTargetJob };
-// A group's progress (the word the host fills with kListPending before every
-// walk): cells in its dense list so far; or kFinal | runs << 12 | cells; or
+// A group's progress (kListPending before the walk): cells in its dense list so far; or kFinal | runs << 12 | cells; or
 // kAborted, when the traversal paused and evaluates its lists itself.
 constexpr uint32_t kFinal = 1u << 31, kAborted = 1u << 30;
 static_assert(kDenseCap < 1u << 12, "two lengths and the flags share a word");
@@ -1149,8 +1148,8 @@ size_t walk_slot_bytes() { return kListCap * sizeof(uint2) + kGroupMax * 3 * siz
 size_t walk_dense_bytes() { return kDenseCap * sizeof(uint2); }
 
 // Lays the slots out over `base`: the lists, sums, lengths and progress words
-// (from a.gnl on 2 * slots words, to be filled with kListPending's bytes
-// before every walk), partial lengths, dense lists.
+// (from a.gnl on 2 * slots words, kWalkPending before every walk), partial
+// lengths, dense lists.
 void walk_scratch(WalkArgs& a, void* base, size_t slots) {
   a.nslots = (uint32_t)slots;
   a.wlist = static_cast<uint2*>(base);

@@ -11,8 +11,8 @@ constexpr int kWalkWarps = 4;
 constexpr int kWalkThreads = kWalkWarps * 32;
 constexpr uint32_t kListCap = 4096;  // entries of a list of the sources some targets of a group take (32 KB)
 // a group's list length(s) before its shared walk has finished (two-pass
-// schedule; the host fills the lengths with this byte pattern before every walk)
-constexpr uint32_t kListPending = 0xfefefefeu;
+// schedule; set before every walk)
+constexpr uint32_t kListPending = kWalkPending;
 
 __device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t v, int lane) {
 #pragma unroll
