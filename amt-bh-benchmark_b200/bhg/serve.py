@@ -26,7 +26,7 @@ from . import ENOMEM, PRECISION_SPLIT, BhgError, Context
 
 #: device bytes per particle of a resident system: state and staging copy
 #: (128), sources (32), sort keys and values (24), marks (4), ~0.45 node
-#: slots of 264 bytes (~119), rounded up
+#: slots of 256 bytes (~115), rounded up
 BYTES_PER_PARTICLE = 320
 RESERVED_SYSTEMS = 4096  # per-system tables sized up front by Server
 
