@@ -265,9 +265,10 @@ int ensure_particles(bhg_context* c, size_t n, int nsys, size_t ntiles, size_t n
     ntiles = std::max(ntiles, c->cap_tiles + c->cap_tiles / 2);
     drop_graph(c);
     c->cap_tiles = 0;
-    // the node kernels' counts: kLevels per unit (eight units per tile where tiles are few)
-    if ((r = grow(c, &c->tiles, ntiles)) || (r = grow(c, &c->partial, ntiles * 6)) ||
-        (r = grow(c, &c->unit_counts, std::max<size_t>(ntiles, 8 * std::min<size_t>(ntiles, 256)) * kLevels)))
+    // bounds and node counts per unit (eight units per tile where tiles are few)
+    const size_t units = std::max<size_t>(ntiles, 8 * std::min<size_t>(ntiles, 256));
+    if ((r = grow(c, &c->tiles, ntiles)) || (r = grow(c, &c->partial, units * 6)) ||
+        (r = grow(c, &c->unit_counts, units * kLevels)))
       return r;
     c->cap_tiles = ntiles;
   }

@@ -96,11 +96,20 @@ __global__ void __launch_bounds__(256) k_fill(FillList f) {
 // a1: bounds per tile, then the domain per system
 // particle_bounds (flat_build_ttg.h:93-113) + domain_from_bounds (domain.h:23-30)
 
+// A unit: `unit` particles of a tile (a multiple of 256), by one block.
+__device__ __forceinline__ Tile node_unit(const Tile* __restrict__ tiles, uint32_t unit, uint32_t u) {
+  const uint32_t per = kTile / unit, off = (u % per) * unit;
+  Tile t = tiles[u / per];
+  t.start += off;
+  t.count = t.count > off ? min(t.count - off, unit) : 0u;
+  return t;
+}
+
 constexpr int kBoundsThreads = 256;
 
 __global__ void __launch_bounds__(kBoundsThreads) k_bounds(const Particle* __restrict__ p, const Tile* __restrict__ tiles,
-                                                           double* __restrict__ partial, DevState* st) {
-  const Tile t = tiles[blockIdx.x];
+                                                           uint32_t unit, double* __restrict__ partial, DevState* st) {
+  const Tile t = node_unit(tiles, unit, blockIdx.x);
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   bool bad = false;
   for (uint32_t i = threadIdx.x; i < t.count; i += kBoundsThreads) {
@@ -139,14 +148,14 @@ __global__ void __launch_bounds__(kBoundsThreads) k_bounds(const Particle* __res
 }
 
 // One warp per system.
-__global__ void k_domain(SysDev* sys, int nsys, const double* __restrict__ partial) {
+__global__ void k_domain(SysDev* sys, int nsys, uint32_t per_tile, const double* __restrict__ partial) {
   const int s = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (s >= nsys) return;
   SysDev& d = sys[s];
   double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (uint32_t t = lane; t < d.tile_count; t += 32) {
-    const double* q = partial + (size_t)(d.tile_begin + t) * 6;
+  for (uint32_t t = lane; t < d.tile_count * per_tile; t += 32) {
+    const double* q = partial + (size_t)(d.tile_begin * per_tile + t) * 6;
     for (int a = 0; a < 3; ++a) {
       lo[a] = fmin(lo[a], q[a]);
       hi[a] = fmax(hi[a], q[3 + a]);
@@ -206,13 +215,13 @@ __device__ __forceinline__ uint32_t quantise(double v, double lo, double scale) 
 
 constexpr int kKeyThreads = 256;
 
-__global__ void __launch_bounds__(kKeyThreads) k_keys(const Particle* __restrict__ p, const Tile* __restrict__ tiles,
+__global__ void __launch_bounds__(kKeyThreads) k_keys(const Particle* __restrict__ p, const Tile* __restrict__ tiles, uint32_t unit,
                                                       const SysDev* __restrict__ sys, uint64_t* __restrict__ keys,
                                                       uint32_t* __restrict__ hist) {
   __shared__ uint32_t h[kSortPasses * 256];
   for (int i = threadIdx.x; i < kSortPasses * 256; i += kKeyThreads) h[i] = 0;
   __syncthreads();
-  const Tile t = tiles[blockIdx.x];
+  const Tile t = node_unit(tiles, unit, blockIdx.x);
   const SysDev& d = sys[t.sys];
   const double lox = d.lox, loy = d.loy, loz = d.loz, sc = d.scale;
   for (uint32_t i = threadIdx.x; i < t.count; i += kKeyThreads) {
@@ -507,15 +516,6 @@ __device__ __forceinline__ int shared_digits(uint64_t a, uint64_t b) {
 // d up to this.
 __device__ __forceinline__ int large_to(const uint64_t* __restrict__ keys, uint32_t i, uint32_t end, unsigned max_leaf) {
   return max_leaf < end - i ? shared_digits(keys[i], keys[i + max_leaf]) : -1;
-}
-
-// A unit: `unit` particles (a multiple of kNodeThreads) of a tile, by one block.
-__device__ __forceinline__ Tile node_unit(const Tile* __restrict__ tiles, uint32_t unit, uint32_t u) {
-  const uint32_t per = kTile / unit, off = (u % per) * unit;
-  Tile t = tiles[u / per];
-  t.start += off;
-  t.count = t.count > off ? min(t.count - off, unit) : 0u;
-  return t;
 }
 
 // depths[i]: bit d set when a node of depth d starts at particle i; counts:
@@ -820,24 +820,27 @@ __global__ void k_pack_groups(const uint32_t* __restrict__ restart, const uint32
 #pragma unroll
         for (int w = 0; w < kPackWindows; ++w) {
           if (end) break;
-          // the greedy packing, run alike by every lane over the window's 32 counts
-          uint32_t starts = 0;
-          for (int i = 0; i < 32; ++i) {
-            const uint32_t ni = __shfl_sync(0xffffffffu, n[w], i);
-            if (ni == 0xffffffffu) {
-              end = true;
-              break;
-            }
-            if (first || cnt + ni > pack || k >= (uint32_t)kMaxTargets) {
-              starts |= 1u << i;
-              cnt = 0;
-              k = 0;
-              first = false;
-            }
-            cnt += ni;
-            ++k;
-          }
-          if ((starts >> lane) & 1u) mark[t0 + 32u * w + (uint32_t)lane] = t0 + 32u * w + (uint32_t)lane;
+          // the greedy packing: from place `pos` on, the next group starts at the
+        // first target that would make the current one too large, found for
+        // all 32 at once from the sums of the counts
+        const uint32_t nv = (uint32_t)__ffs(~__ballot_sync(0xffffffffu, n[w] != 0xffffffffu)) - 1u;  // ~0: all 32
+        const uint32_t live = min(nv, 32u), in = (uint32_t)lane < live ? n[w] : 0u, sum = warp_incl_scan(in);
+        end = live < 32u;
+        uint32_t starts = 0, pos = 0, before = 0;  // before: the counts up to pos
+        for (;;) {
+          const uint32_t i = (uint32_t)lane;
+          const bool over = first || cnt + (sum - before) > pack || k + (i - pos) >= (uint32_t)kMaxTargets;
+          const uint32_t m = __ballot_sync(0xffffffffu, i >= pos && i < live && over);
+          if (!m) break;
+          const uint32_t at_i = (uint32_t)__ffs(m) - 1u;
+          starts |= 1u << at_i;
+          first = false;
+          cnt = __shfl_sync(0xffffffffu, in, at_i), k = 1u;
+          before = __shfl_sync(0xffffffffu, sum, at_i), pos = at_i + 1u;
+        }
+        cnt += __shfl_sync(0xffffffffu, sum, 31) - before;
+        k += live - pos;
+        if ((starts >> lane) & 1u) mark[t0 + 32u * w + (uint32_t)lane] = t0 + 32u * w + (uint32_t)lane;
         }
       }
     }
@@ -994,15 +997,27 @@ void set_build_attributes() {
   done = true;
 }
 
+// Particles per unit of the node kernels: a tile, or an eighth of one where
+// there are few tiles (more blocks; the one block that scans the counts takes 3
+// us for 2,000 units).
+uint32_t node_unit_size(int ntiles) { return ntiles <= 256 ? kTile / 8 : kTile; }
+
+// The same for bounds and keys, up to fewer tiles: every block of the keys adds
+// its digit counts to the system's.  Bounds, domain and keys by tiles / by
+// eighths: 0.030 / 0.021 ms at 65k, 0.035 / 0.035 at 262k, 0.049 / 0.080 at 1M.
+static uint32_t key_unit_size(int ntiles) { return ntiles <= 48 ? kTile / 8 : kTile; }
+
 void launch_bounds_domain(const Particle* p, const Tile* tiles, int ntiles, SysDev* sys, int nsys, double* partial,
                           DevState* st, cudaStream_t s) {
-  k_bounds<<<ntiles, kBoundsThreads, 0, s>>>(p, tiles, partial, st);
-  k_domain<<<(nsys + 3) / 4, 128, 0, s>>>(sys, nsys, partial);
+  const uint32_t unit = key_unit_size(ntiles), per = kTile / unit;
+  k_bounds<<<(unsigned)ntiles * per, kBoundsThreads, 0, s>>>(p, tiles, unit, partial, st);
+  k_domain<<<(nsys + 3) / 4, 128, 0, s>>>(sys, nsys, per, partial);
 }
 
 void launch_keys(const Particle* p, const Tile* tiles, int ntiles, const SysDev* sys, int nsys, uint64_t* keys,
                  uint32_t* hist, uint32_t* offs, cudaStream_t s) {
-  k_keys<<<ntiles, kKeyThreads, 0, s>>>(p, tiles, sys, keys, hist);
+  const uint32_t unit = key_unit_size(ntiles);
+  k_keys<<<(unsigned)ntiles * (kTile / unit), kKeyThreads, 0, s>>>(p, tiles, unit, sys, keys, hist);
   k_digit_offsets<<<nsys, 256, 0, s>>>(sys, hist, offs);
 }
 
@@ -1038,10 +1053,6 @@ static int grid_for(uint64_t units, uint64_t per_block, int cap) {
   return (int)std::max<uint64_t>(1, std::min<uint64_t>(b, (uint64_t)cap));
 }
 
-// Particles per unit: a tile, or an eighth of one where there are few tiles
-// (more blocks; the one block that scans the counts takes 3 us for 2,000 units).
-uint32_t node_unit_size(int ntiles) { return ntiles <= 256 ? kTile / 8 : kTile; }
-
 void launch_topology(const Tile* tiles, int ntiles, const SysDev* sys, const Nodes& nd, const uint64_t* keys,
                      unsigned max_leaf, uint32_t* depths, uint32_t* counts, DevState* st, cudaStream_t s) {
   const uint32_t unit = node_unit_size(ntiles), units = (uint32_t)ntiles * (kTile / unit);
@@ -1054,8 +1065,9 @@ void launch_topology(const Tile* tiles, int ntiles, const SysDev* sys, const Nod
 // counter): measured at 4M with three compactions, the targets phase took
 // 0.179 ms with 4/2/2 blocks per SM and 0.140 with 16/8/8.  The packing chunks'
 // starts ride on the targets' marks: with a marking and a compaction of their
-// own the phase took 0.055 ms at 16k (now 0.038), 0.064 at 65k (0.047), 0.221
-// at 4M (0.186), resets included.
+// own the phase took 0.055 ms at 16k, 0.064 at 65k and 0.221 at 4M (resets
+// included), without 0.038, 0.047 and 0.186, and with group starts found for 32
+// targets at once 0.035, 0.043 and 0.172.
 void launch_targets(const Nodes& nd, uint32_t lim, uint32_t pack, uint32_t n, uint32_t* mark, uint32_t* targets,
                     uint32_t* restart, uint32_t* groups, uint32_t* lookback, DevState* st, int sms, cudaStream_t s) {
   const uint32_t ntiles = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
