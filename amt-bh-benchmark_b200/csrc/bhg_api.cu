@@ -81,7 +81,7 @@ struct bhg_context {
   unsigned max_leaf = 16;
   uint32_t group_size = 256;
   int quad = 1, precision = 0;
-  bool mask = false;
+  bool mask = false, soft = true;  // some walked system is unsoftened; some is softened
 
   // timing: CUDA events around every phase, summed on request
   struct Pending {
@@ -303,8 +303,12 @@ void push_tiles(std::vector<Tile>& out, uint32_t sys, uint32_t begin, uint32_t n
   for (uint32_t o = 0; o < n; o += tile) out.push_back(Tile{sys, begin + o, std::min<uint32_t>(tile, n - o), first});
 }
 
+// A split walk of softened and unsoftened systems: one launch for each kind.
+bool mixed_walk(const bhg_context* c) { return c->precision == BHG_PRECISION_SPLIT && c->mask && c->soft; }
+
 int walk_grid(bhg_context* c) {
   int per = walk_blocks_per_sm(c->precision, c->quad != 0, c->mask);
+  if (mixed_walk(c)) per = std::max(per, walk_blocks_per_sm(c->precision, c->quad != 0, false));
   return c->sms * per;
 }
 
@@ -346,10 +350,11 @@ int ensure_walk_scratch(bhg_context* c, int grid) {
   return BHG_OK;
 }
 
-// Blocks of the walk launch: the occupancy grid, or fewer when the HBM
-// budget limited the lists (both kinds per warp at least).
-int walk_launch_grid(bhg_context* c) {
-  return (int)std::min<size_t>((size_t)walk_grid(c), std::min(c->list_warps, c->dense_warps) / (walk_threads() / 32));
+// Blocks of a walk launch: the occupancy grid, or fewer when the HBM budget
+// limited the lists (both kinds per warp at least).
+int walk_launch_grid(bhg_context* c, bool mask) {
+  return (int)std::min<size_t>((size_t)c->sms * walk_blocks_per_sm(c->precision, c->quad != 0, mask),
+                               std::min(c->list_warps, c->dense_warps) / (walk_threads() / 32));
 }
 
 // Lays out the systems c->counts back to back with their sort tiles, sizes
@@ -515,7 +520,12 @@ void enq_walk(bhg_context* c, bool want_accel) {
   a.accel = want_accel ? c->accel : nullptr;
   a.st = c->st;
   walk_scratch(a, c->list_buf, c->list_warps);
-  launch_walk(a, (uint32_t)c->n, c->precision, c->quad != 0, c->mask, walk_launch_grid(c), c->stream);
+  const auto walk = [&](bool mask, WalkOnly only) {
+    a.only = only;
+    launch_walk(a, (uint32_t)c->n, c->precision, c->quad != 0, mask, walk_launch_grid(c, mask), c->stream);
+  };
+  if (mixed_walk(c)) walk(false, WalkOnly::kSoftened), walk(true, WalkOnly::kUnsoftened);
+  else walk(c->mask, WalkOnly::kAll);
   launch_eval_done(c->st, c->stream);
 }
 
@@ -587,9 +597,9 @@ int run_phase(bhg_context* c, int phase, F enq) {
 // grids), the state's place (it trades places with the staging buffer).
 std::string graph_key(const bhg_context* c, uint32_t target_size) {
   char key[256];
-  snprintf(key, sizeof key, "%zu/%d/%zu/%zu/%zu/%zu/%u/%p/%u/%u/%u/%u/%d/%d/%d", c->n, c->nsys, c->tiles_host.size(),
+  snprintf(key, sizeof key, "%zu/%d/%zu/%zu/%zu/%zu/%u/%p/%u/%u/%u/%u/%d/%d/%d/%d", c->n, c->nsys, c->tiles_host.size(),
            c->stiles_host.size(), c->cap_nodes, c->list_warps, c->sort_tile, (void*)c->part, c->walk_pack, c->max_leaf,
-           c->group_size, target_size, c->precision, c->quad, (int)c->mask);
+           c->group_size, target_size, c->precision, c->quad, (int)c->mask, (int)c->soft);
   return key;
 }
 
@@ -660,11 +670,12 @@ int set_force_params(bhg_context* c, const bhg_force_params* fp, double kick, do
   // systems' own eps2 decide, not fp->eps2: one unsoftened system among
   // softened ones needs the masked kernel (its self terms would be
   // rsqrt(0) = inf times 0 otherwise).
-  bool mask = !(fp->eps2 > 0.0);
+  bool mask = !(fp->eps2 > 0.0), soft = !mask;
   if (keep_per_system) {
-    mask = false;
-    for (const auto& p : c->prm_host) mask = mask || !(p.eps2 > 0.0);
+    mask = soft = false;
+    for (const auto& p : c->prm_host) (p.eps2 > 0.0 ? soft : mask) = true;
   }
+  c->soft = soft;
   c->mask = mask;
   return BHG_OK;
 }
@@ -1528,8 +1539,10 @@ int bhg_get_stats(bhg_context* c, bhg_stats* out, int reset) {
   // resets + bounds + domain + keys + digit offsets; the sort passes; gather + the
   // three topology kernels; the multipoles (one kernel, or one per level);
   // resets + mark + compact of the targets, packing + compact of the walk
-  // groups; the walk and its completion count
-  out->kernels_per_eval = 5 + kSortPasses + 4 + (c->n <= kMomentsOneLaunchMax ? 1 : kMortonDepth + 1) + 5 + 2;
+  // groups; the walk (two of softened and unsoftened systems together) and
+  // its completion count
+  out->kernels_per_eval = 5 + kSortPasses + 4 + (c->n <= kMomentsOneLaunchMax ? 1 : kMortonDepth + 1) + 5 + 2 +
+                          (mixed_walk(c) ? 1 : 0);
   if (reset) {
     for (double& t : c->tot_ms) t = 0.0;
     c->walks_timed = 0;

@@ -56,6 +56,11 @@ void launch_targets(const Nodes& nd, uint32_t lim, uint32_t pack, uint32_t n, ui
 // one kernel per level; the same bits either way
 void launch_moments(const Nodes& nd, const double4* pm, const DevState* st, int sms, bool one_launch, cudaStream_t s);
 
+// A context may hold softened and unsoftened systems, which a split walk takes
+// with different kernels, each leaving the other's systems alone: so no
+// system's bits depend on the others' softening.
+enum class WalkOnly : uint32_t { kAll, kSoftened, kUnsoftened };
+
 struct WalkArgs {
   const double4* wcom;
   const uint2* wlink;
@@ -86,6 +91,7 @@ struct WalkArgs {
   uint32_t* prog;  // per slot: what a group's traversal has written of its dense list
   uint32_t* plen;  // per slot: the lengths of its partial list
   uint32_t nslots;
+  WalkOnly only;  // which systems this launch walks
 };
 
 // Walks every target and kicks/drifts its particles.  precision:

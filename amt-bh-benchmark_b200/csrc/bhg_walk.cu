@@ -966,6 +966,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
       const GroupInfo g = group_info(a, J.gi, ngroups, ntargets);
       J.t0 = g.t0, J.k = g.k, J.p0 = g.p0, J.sys = g.s;
     }
+    if (walked_elsewhere(a, J.sys)) continue;
     if (J.kind != kWholeJob && J.k == 1) continue;  // done whole by its group
     J.w = Walk{0u, 0u, 0u, 0u, 0u, 0u};
     set_units(S, a.sys[J.sys].hw);

@@ -122,6 +122,11 @@ __device__ __forceinline__ uint32_t system_of(const WalkArgs& a, uint32_t p) {
   return lo;
 }
 
+// Whether another launch walks system s.
+__device__ __forceinline__ bool walked_elsewhere(const WalkArgs& a, uint32_t s) {
+  return a.only != WalkOnly::kAll && (a.prm[s].eps2 > 0.0) != (a.only == WalkOnly::kSoftened);
+}
+
 // The group of walk group gi: its targets, first particle and system.
 struct GroupInfo {
   uint32_t t0, k, p0, s;

@@ -610,7 +610,7 @@ __device__ __forceinline__ void target_jobs(E& ev, const WalkArgs& a, QueueSmem&
                                             int lane, Queues& q, unsigned long long& n_pp, unsigned long long& n_pc) {
   for (;;) {
     uint32_t ti = 0;
-    if (lane == 0) ti = atomicAdd(&a.st->walk_next2, 1u);
+    if (lane == 0) ti = atomicAdd(&a.st->walk_next4, 1u);
     ti = __shfl_sync(kFull, ti, 0);
     if (ti >= ntargets) break;
     // its group: the last whose first target is at or before ti
@@ -621,6 +621,7 @@ __device__ __forceinline__ void target_jobs(E& ev, const WalkArgs& a, QueueSmem&
       else hi = mid;
     }
     const GroupInfo g = group_info(a, gi, ngroups, ntargets);
+    if (walked_elsewhere(a, g.s)) continue;
     if (g.k == 1) continue;  // done whole in the first pass
     uint32_t nlist = ld_volatile(a.gnl + gi);
     for (int spins = 0; nlist == kListPending && spins < kSpinLimit; ++spins) {
@@ -696,10 +697,11 @@ __global__ void __launch_bounds__(kWalkThreads, 4) k_walk_unsoftened(WalkArgs a)
   Queues q;
   for (;;) {
     uint32_t gi = 0;
-    if (lane == 0) gi = atomicAdd(&a.st->walk_next, 1u);
+    if (lane == 0) gi = atomicAdd(&a.st->walk_next3, 1u);
     gi = __shfl_sync(kFull, gi, 0);
     if (gi >= ngroups) break;
     const GroupInfo g = group_info(a, gi, ngroups, ntargets);
+    if (walked_elsewhere(a, g.s)) continue;
     const uint32_t k = g.k, p0 = g.p0;
     const uint32_t root = a.sys[g.s].root;
     const SysParam& sp = a.prm[g.s];

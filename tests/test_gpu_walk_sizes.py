@@ -141,3 +141,30 @@ def test_snapshot_sizes_match_oracle(oracle, n):
         assert ctx.snapshot_vtk_into(exact) == len(want) and exact.tobytes() == want
         with pytest.raises(bhg.BhgError):
             ctx.snapshot_vtk_into(np.zeros(len(want) - 1, np.uint8))
+
+
+@pytest.mark.parametrize("precision", [bhg.PRECISION_SPLIT, bhg.PRECISION_FP64])
+def test_softening_of_others_changes_no_bits(precision):
+    """Softened and unsoftened systems in one context: each as it is alone, with
+    few walk groups and with many."""
+    for sizes in ((3000, 700, 1500, 1), (60000, 30000, 200000)):
+        systems = [cube(n, 80 + i, spread=2.0) for i, n in enumerate(sizes)]
+        eps2 = [1e-4 if i % 2 == 0 else 0.0 for i in range(len(sizes))]
+        fp = bhg.Context.params(0.5, 0.0, 1.0, True, precision)
+
+        def run(ctx, which):
+            ctx.upload_systems([systems[i] for i in which])
+            k = len(which)
+            ctx.set_system_params([0.6] * k, [eps2[i] for i in which], [0.01] * k, [0.02] * k)
+            ctx.stats()
+            for _ in range(2):
+                ctx.step_systems(fp, 16, 256, 16)
+            s = ctx.stats()
+            return np.split(ctx.download(), np.cumsum([sizes[i] for i in which])[:-1]), s["pp"], s["pc"]
+
+        with bhg.Context(device=0) as ctx:
+            mixed, pp, pc = run(ctx, range(len(sizes)))
+            alone = [run(ctx, [i]) for i in range(len(sizes))]
+        assert (pp, pc) == (sum(a[1] for a in alone), sum(a[2] for a in alone))
+        for i, a in enumerate(alone):
+            assert mixed[i].tobytes() == a[0][0].tobytes(), i
