@@ -83,7 +83,8 @@ struct WalkArgs {
   // some targets of a group take, per warp (one pass) or per group (two
   // passes, when there are at most nslots groups); per slot also the group's
   // FP64 sums (kGroupMax x 3) and list lengths; per warp of the grid a dense
-  // list (the sources every target of the group takes)
+  // list (the sources every target of the group takes: the warp's group, or as
+  // dense_slot says where dense jobs run)
   uint2* dlist;
   uint2* wlist;
   double* gsum;

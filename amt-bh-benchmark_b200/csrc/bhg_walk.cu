@@ -36,6 +36,7 @@
 // below); FP32 partials go into FP64 sums every 32 or more terms.  The
 // kick/drift of integrate_ttg.h:74-77 is applied in FP64 in the epilogue.
 #include "bhg_walk.cuh"
+#include "bhg_lists.h"
 
 #include <algorithm>
 #include <type_traits>
@@ -919,12 +920,12 @@ __device__ __forceinline__ uint32_t group_boxes(const WalkArgs& a, WarpSmem& S, 
 // every target's pass as a job of its own, starting as soon as the group's
 // lengths are published.  With fewer groups still (two warps for each), a
 // group's dense pass is a job of its own too, which takes the cells while the
-// traversal finds them; if that has to pause, it evaluates its lists itself.  A
-// job waits only for jobs handed out before it, which running warps hold and
-// which wait for none or for such jobs, so every wait ends; a wait is still
-// bounded (kStSpinLimit, the job skipped).  All schedules run the same passes
-// on the same batches and add their parts in the same order, so the results
-// are the same bits.  Walk with / without dense jobs: 0.25 / 0.34 ms
+// traversal finds them; if that has to pause, it evaluates its lists itself and
+// goes on in another dense list (dense_slot).  A job waits only for jobs
+// handed out before it, which running warps hold and which wait for none or
+// for such jobs, so every wait ends; a wait is still bounded (kStSpinLimit,
+// the job skipped).  All schedules run the same passes on the same batches and
+// add their parts in the same order, so the results are the same bits.  Walk with / without dense jobs: 0.25 / 0.34 ms
 // at 16k, 0.42 / 0.56 at 65k, 0.63 / 0.72 at 40k in FP64.
 template <class E, bool QUAD, bool PAIRS>
 __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs a) {
@@ -973,7 +974,7 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
     // the partial list is the warp's or (two-pass schedule) the group's, the
     // dense one the warp's or (with dense jobs) the group's
     const size_t wid = (size_t)blockIdx.x * kWalkWarps + warp;
-    J.dense = a.dlist + (paired ? (size_t)J.gi : wid) * kDenseCap;
+    J.dense = a.dlist + dense_slot(paired, false, J.gi, ngroups, wid) * kDenseCap;
     J.partial = a.wlist + (two_pass ? (size_t)J.gi : wid) * kListCap;
     J.poll = J.kind == kDenseJob;
     J.aborted = 0u;
@@ -1057,6 +1058,8 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
         }
         __syncwarp();
         J.w.ndc = J.w.ndr = 0;
+        // the dense job may still be reading the list it was given
+        if (paired && J.aborted) J.dense = a.dlist + dense_slot(true, true, J.gi, ngroups, wid) * kDenseCap;
         if (J.pass1) J.w.npc = J.w.npr = 0;
         __syncwarp();
       } while (J.more);

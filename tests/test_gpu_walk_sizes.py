@@ -72,6 +72,25 @@ def test_full_lists_give_the_same_bits_in_both_schedules(precision):
     assert out[0] == out[1]
 
 
+@pytest.mark.parametrize("precision", [bhg.PRECISION_SPLIT, bhg.PRECISION_FP64])
+@pytest.mark.parametrize("n,leaf,theta,budget", [(30000, 16, 0.2, 25), (65536, 16, 0.3, 40), (60000, 32, 0.25, 36)])
+def test_paused_traversals_beside_dense_jobs(n, leaf, theta, budget, precision):
+    """Few groups whose dense lists fill up, at leaf sizes with fewer node records
+    than particles: the group's own job evaluates its lists and goes on in
+    another one while its dense job may still read the first.  The same counts
+    and bits as the one-pass schedule without dense jobs (a budget of few lists)."""
+    parts = bhg.plummer(n, 600 + leaf)[0]
+    fp = bhg.Context.params(theta, 1e-4, 1.0, True, precision)
+    out = []
+    for mb in (0, budget):
+        with bhg.Context(device=0, hbm_budget=mb << 20) as ctx:
+            ctx.upload(parts)
+            ctx.step(fp, leaf, 256, leaf, 0.01, 0.01)
+            s = ctx.stats()
+            out.append((ctx.download().tobytes(), s["pp"], s["pc"]))
+    assert out[0] == out[1]
+
+
 @pytest.mark.parametrize("ns", [1, 2, 3, 127, 129, 256, 257, 700])
 def test_direct_sum_rows_and_splits(gpu, oracle, ns):
     """Row counts around the block's (1 .. 256 rows, a remainder block), source
