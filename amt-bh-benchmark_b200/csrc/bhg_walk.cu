@@ -956,8 +956,10 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
     } else if (next < ngroups) {
       J.gi = next;
     } else if (paired && next < 2 * ngroups) {
+      __syncwarp();
       J.gi = next - ngroups, J.kind = kDenseJob;
     } else if (two_pass) {
+      __syncwarp();  // every lane has read the kind
       J.kind = kTargetJob;
       continue;
     } else {
@@ -1017,10 +1019,9 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
         J.w.top = 1, J.w.steps = 0;
         __syncwarp();
       }
-      J.left = 0u;
-      do {
+      J.left = J.more = 0u;
+      do {  // J.more is read at the end of a turn and written after the next one's traversal
         uint32_t pass = J.pass1;
-        J.more = 0u;
         if (J.kind == kWholeJob) {
           const bool beside = paired && J.k > 1 && !J.aborted;  // a dense job evaluates beside
           const bool more =
