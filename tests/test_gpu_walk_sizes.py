@@ -187,3 +187,27 @@ def test_softening_of_others_changes_no_bits(precision):
         assert (pp, pc) == (sum(a[1] for a in alone), sum(a[2] for a in alone))
         for i, a in enumerate(alone):
             assert mixed[i].tobytes() == a[0][0].tobytes(), i
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 8, 10])
+def test_sources_of_one_record_add_in_64_bits(n):
+    """Up to ten particles in one leaf: a lane evaluates one record of two
+    sources for a target, so no two FP32 terms share a partial sum, and the
+    forces of all sources together are those of each alone (the others
+    massless) added in FP64: n additions of 2^-53 each, not 2^-24."""
+    parts = cube(n, 500 + n)
+    parts["mass"] = np.random.default_rng(n).uniform(0.5, 2.0, n)
+    fp = bhg.Context.params(0.5, 1e-4)
+
+    with bhg.Context(device=0) as ctx:
+        def forces(mass):
+            p = parts.copy()
+            p["mass"] = mass
+            ctx.upload(p)
+            ctx.build_tree(16, 256)
+            ctx.compute_multipoles()
+            return ctx.walk_forces(fp, 16)
+
+        alone = np.array([forces(np.where(np.arange(n) == i, parts["mass"], 0.0)) for i in range(n)])
+        together = forces(parts["mass"])
+    assert np.all(np.abs(together - alone.sum(0)) <= 2 * n * 2.0**-53 * np.abs(alone).sum(0))
