@@ -68,7 +68,8 @@ struct bhg_context {
   uint32_t *unit_counts = nullptr, *mark = nullptr, *targets = nullptr, *scan_lb = nullptr;
   uint32_t *groups = nullptr, *restart = nullptr;
   double* accel = nullptr;
-  std::vector<std::pair<void*, size_t>> text_scratch;  // cached buffers of the text calls
+  std::vector<std::pair<void*, size_t>> scratch;  // cached buffers of single calls (Scratch)
+  int scratch_users = 0;                          // calls that hold some of them
   DevState* st = nullptr;
   DevState* st_host = nullptr;  // pinned
   // a snapshot's copies to the host run beside its formatting
@@ -123,13 +124,21 @@ int fail(bhg_context* c, int code, const std::string& msg) {
     if (e_ != cudaSuccess) return fail(c, BHG_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+bool release_scratch(bhg_context* c);
+
+// Memory that single calls left cached makes room when the budget or the
+// device has none left.
 int dev_alloc(bhg_context* c, void** p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) bytes = 16;
-  if (c->budget && c->allocated + bytes > c->budget)
+  if (c->budget && c->allocated + bytes > c->budget && !(release_scratch(c) && c->allocated + bytes <= c->budget))
     return fail(c, BHG_ENOMEM, "HBM budget exceeded: need " + std::to_string(c->allocated + bytes) + " bytes of " +
                                    std::to_string(c->budget));
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (release_scratch(c)) e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(c, BHG_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -149,6 +158,15 @@ void dev_free(bhg_context* c, void* p) {
     }
   }
   cudaFree(p);
+}
+
+// Frees the cached buffers of single calls, unless one is running; whether
+// there were any.
+bool release_scratch(bhg_context* c) {
+  if (c->scratch_users || c->scratch.empty()) return false;
+  for (auto& s : c->scratch) dev_free(c, s.first);
+  c->scratch.clear();
+  return true;
 }
 
 template <typename T>
@@ -334,7 +352,9 @@ int ensure_walk_scratch(bhg_context* c, int grid) {
   if (c->list_warps >= slots && c->dense_warps >= warps) return BHG_OK;
   if (c->budget) {
     const size_t held = c->list_warps * per_slot + c->dense_warps * per_dense;  // freed below, so it counts as room
-    const size_t room = c->budget > c->allocated - held ? c->budget - (c->allocated - held) : 0;
+    const auto left = [&] { return c->budget > c->allocated - held ? c->budget - (c->allocated - held) : 0; };
+    size_t room = left();
+    if (room < slots * per_slot + warps * per_dense && release_scratch(c)) room = left();
     if (room < slots * per_slot + warps * per_dense)
       slots = warps = std::min(warps, std::max(wpb, room / (per_slot + per_dense) / wpb * wpb));
     if (c->list_warps >= slots && c->dense_warps >= warps) return BHG_OK;
@@ -938,19 +958,22 @@ size_t bhg_num_systems(const bhg_context* c) { return c ? c->counts.size() : 0; 
 
 namespace {
 
-// Device scratch of one text operation, freed on every way out.
-// Device scratch of one text operation: the k-th buffer a call asks for is
-// the context's k-th cached buffer, grown when too small and kept for the
-// next call (repeated ingests allocate nothing).
+// Device scratch of one call (text in and out, direct sums): the k-th buffer a
+// call asks for is the context's k-th cached buffer, grown when too small and
+// kept for the next call (repeated calls allocate nothing) until the memory is
+// needed elsewhere (release_scratch).
 struct Scratch {
   bhg_context* c;
   size_t k = 0;
-  explicit Scratch(bhg_context* c_) : c(c_) {}
+  explicit Scratch(bhg_context* c_) : c(c_) { ++c->scratch_users; }
+  ~Scratch() { --c->scratch_users; }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
   template <typename T>
   int get(T** p, size_t count) {
     const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-    if (k == c->text_scratch.size()) c->text_scratch.push_back({nullptr, 0});
-    auto& slot = c->text_scratch[k++];
+    if (k == c->scratch.size()) c->scratch.push_back({nullptr, 0});
+    auto& slot = c->scratch[k++];
     if (slot.second < bytes) {
       dev_free(c, slot.first);
       slot = {nullptr, 0};

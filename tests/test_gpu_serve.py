@@ -260,3 +260,31 @@ def test_reserve_then_add_equals_growth():
         assert e.value.code == bhg.ENOMEM
         small.add_system(systems[0])  # still usable
         assert small.download().tobytes() == systems[0].tobytes()
+
+
+@pytest.mark.parametrize("what", ["direct_sum", "snapshot"])
+def test_scratch_gives_way_to_systems(what):
+    """The buffers that direct sums and snapshots leave for the next call make
+    room when the HBM budget needs it: a budget that just holds a second system
+    still does after such a call."""
+    a, b = bhg.plummer(60000, 500)[0], bhg.plummer(120000, 501)[0]
+
+    def joins(budget, before=None):
+        with bhg.Context(device=0, hbm_budget=budget) as ctx:
+            try:
+                ctx.upload(a)
+                if before:
+                    before(ctx)
+                ctx.add_system(b)
+            except bhg.BhgError as e:
+                assert e.code == bhg.ENOMEM
+                return False
+            return ctx.download().tobytes() == a.tobytes() + b.tobytes()
+
+    lo, hi = 1, 256  # MB
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (lo, mid) if joins(mid << 20) else (mid, hi)
+    rows = np.arange(4096, dtype=np.uint32)
+    call = {"direct_sum": lambda ctx: ctx.direct_sum(rows, 1e-4, 1.0), "snapshot": lambda ctx: ctx.snapshot_vtk()}[what]
+    assert joins(hi << 20, call)
