@@ -456,10 +456,12 @@ int set_problem(bhg_context* c, const uint64_t* counts, size_t nsys) {
 }
 
 // After a growth that failed part-way some scratch may be missing (its
-// capacity is then 0): allocates it again before anything is launched.
+// capacity is then 0), and after one outside relayout (bhg_reserve) the tables
+// are new and empty: allocates and fills them again before anything is
+// launched.
 int ensure_layout(bhg_context* c) {
-  if (c->cap_n >= c->n && c->cap_sys >= c->counts.size() && c->cap_tiles >= c->tiles_host.size() &&
-      c->cap_stiles >= c->stiles_host.size())
+  if (!c->laid_counts.empty() && c->cap_n >= c->n && c->cap_sys >= c->counts.size() &&
+      c->cap_tiles >= c->tiles_host.size() && c->cap_stiles >= c->stiles_host.size())
     return BHG_OK;
   return relayout(c);
 }
@@ -860,9 +862,15 @@ int bhg_reserve(bhg_context* c, size_t particles, size_t systems) {
   const size_t nsys = std::max(systems, c->counts.size());
   int r;
   const size_t nst = std::max(n / kSortTileLarge, std::min(n, kSmallSortMax) / kSortTileSmall) + nsys;
-  if ((r = ensure_particles(c, n, (int)nsys, n / kTile + nsys, nst)) || (r = ensure_nodes(c, node_estimate(n, (int)nsys, 16))))
-    return r;
-  return BHG_OK;
+  const size_t cap_n = c->cap_n, cap_nodes = c->cap_nodes, cap_sys = c->cap_sys;
+  if (!(r = ensure_particles(c, n, (int)nsys, n / kTile + nsys, nst)))
+    r = ensure_nodes(c, node_estimate(n, (int)nsys, 16));
+  // phases under way end where the particles, systems or nodes they go on with
+  // were replaced
+  const bool moved = c->cap_n != cap_n || c->cap_sys != cap_sys;
+  if (moved || c->cap_nodes != cap_nodes) c->built = c->moments = false;
+  if (moved) c->walked = false;
+  return r;
 }
 
 int bhg_add_system(bhg_context* c, const bh_particle64* p, size_t n, uint64_t* id) {

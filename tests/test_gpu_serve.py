@@ -288,3 +288,31 @@ def test_scratch_gives_way_to_systems(what):
     rows = np.arange(4096, dtype=np.uint32)
     call = {"direct_sum": lambda ctx: ctx.direct_sum(rows, 1e-4, 1.0), "snapshot": lambda ctx: ctx.snapshot_vtk()}[what]
     assert joins(hi << 20, call)
+
+
+def test_reserve_keeps_resident_systems():
+    """Reserving more while systems are resident replaces the tables and buffers:
+    the systems step to the same bits as without, and phases that were under
+    way start again; one that grows neither particles, systems nor nodes leaves
+    them be."""
+    systems = [bhg.plummer(n, 520 + i)[0] for i, n in enumerate((5000, 12000))]
+    fp = bhg.Context.params(0.5, 1e-4)
+    out = []
+    for more in (None, (100, 1), (17000, 300), (400000, 2), (400000, 5000)):
+        with bhg.Context(device=0) as ctx:
+            ctx.upload_systems(systems)
+            ctx.step(fp, 16, 256, 16, 0.01, 0.01)
+            if more:
+                ctx.reserve(*more)
+            ctx.step(fp, 16, 256, 16, 0.01, 0.01)
+            out.append(ctx.download().tobytes())
+            ctx.build_tree(16, 256)
+            ctx.reserve(100, 1)
+            ctx.compute_multipoles()
+            ctx.reserve(1000000, 6000)
+            with pytest.raises(bhg.BhgError) as e:
+                ctx.walk_forces(fp, 16)
+            assert e.value.code == bhg.ESTATE
+            ctx.step(fp, 16, 256, 16, 0.01, 0.01)
+            out[-1] += ctx.download().tobytes()
+    assert all(o == out[0] for o in out)
