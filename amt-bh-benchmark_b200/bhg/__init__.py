@@ -37,7 +37,7 @@ EXPORTED = (
     "bhg_step_systems_async", "bhg_download_async", "bhg_sync",
     "bhg_run_schedule", "bhg_set_system_params", "bhg_get_stats", "bhg_device_status", "bhg_debug_export",
     "bhg_direct_sum", "bhg_energy", "bhg_energy_noalloc", "bhg_ic_plummer", "bhg_write_csv",
-    "bhg_measure_fp32_peak", "bhg_selftest_wait", "bhg_set_walk_group",
+    "bhg_measure_fp32_peak", "bhg_selftest_wait", "bhg_selftest_walk_wait", "bhg_set_walk_group",
 )
 
 
@@ -128,6 +128,7 @@ def lib() -> C.CDLL:
         "bhg_write_csv": ([C.c_char_p, vp, sz], i32),
         "bhg_measure_fp32_peak": ([i32, C.POINTER(f64)], i32),
         "bhg_selftest_wait": ([vp, i32, u32, C.POINTER(u32)], i32),
+        "bhg_selftest_walk_wait": ([vp, i32, u32, C.POINTER(u32)], i32),
         "bhg_set_walk_group": ([vp, u32], i32),
     }
     for name, (args, res) in sigs.items():
@@ -437,6 +438,13 @@ class Context:
         pre = C.c_uint32()
         r = self.L.bhg_selftest_wait(self.h, 1 if publish_first else 0, spin_limit, C.byref(pre))
         return r, pre.value
+
+    def selftest_walk_wait(self, publish: bool, spin_limit: int):
+        """bhg_selftest_walk_wait: (status code, words) of the walk's bounded
+        waits run on prepared words that are published or never are."""
+        words = (C.c_uint32 * 3)()
+        r = self.L.bhg_selftest_walk_wait(self.h, 1 if publish else 0, spin_limit, words)
+        return r, tuple(words)
 
     def last_error(self) -> str:
         return (self.L.bhg_last_error(self.h) or b"").decode(errors="replace")

@@ -651,7 +651,7 @@ std::string status_text(uint32_t s) {
   std::string t;
   if (s & kStNonFinite) t += " non-finite particle coordinate;";
   if (s & kStNodeOverflow) t += " octree larger than its node slots;";
-  if (s & kStSpinLimit) t += " a bounded wait in a sort/scan kernel gave up;";
+  if (s & kStSpinLimit) t += " a bounded wait in a sort, scan or walk kernel gave up;";
   if (s & kStTooLarge) t += " a count exceeded 30 bits;";
   if (s & kStWalkLimit) t += " a walk visited more nodes than the tree holds;";
   return t;
@@ -1724,6 +1724,41 @@ int bhg_energy(bhg_context* c, int sys, double G, double* kinetic, double* poten
   return BHG_OK;
 }
 
+}  // extern "C"
+
+// Runs a bounded wait on prepared words: launch(words, out) with nout words of
+// results to got (optional), and the status it left.
+template <typename F>
+static int selftest(bhg_context* c, uint32_t spin_limit, const std::vector<uint32_t>& words, uint32_t* got, size_t nout,
+                    F launch) {
+  if (!c) return BHG_EINVAL;
+  if (spin_limit == 0 || spin_limit > (1u << 20))
+    return fail(c, BHG_EINVAL, "spin_limit must be in 1 .. 2^20 (a short wait)");
+  cudaSetDevice(c->device);
+  int r = read_state(c);  // finish what is queued; its own errors come first
+  if (r || (r = finish_async(c))) return r;
+  uint32_t* dev = nullptr;
+  if ((r = dev_alloc(c, reinterpret_cast<void**>(&dev), (words.size() + nout) * sizeof(uint32_t)))) return r;
+  cudaError_t e = cudaMemcpyAsync(dev, words.data(), words.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) {
+    launch(dev, dev + words.size());
+    e = cudaGetLastError();
+  }
+  std::vector<uint32_t> out(nout, 0u);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(out.data(), dev + words.size(), nout * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+  dev_free(c, dev);
+  if (e != cudaSuccess) return fail(c, BHG_ECUDA, std::string("selftest: ") + cudaGetErrorString(e));
+  if (got) std::copy(out.begin(), out.end(), got);
+  if ((r = read_state(c))) return r;
+  r = check_status(c);  // a wait that gave up: BHG_EDEVICE, as from a real kernel
+  clear_status(c);
+  return r;
+}
+
+extern "C" {
+
 int bhg_set_walk_group(bhg_context* c, uint32_t particles) {
   if (!c) return BHG_EINVAL;
   if (particles > (uint32_t)kGroupMax)
@@ -1735,35 +1770,22 @@ int bhg_set_walk_group(bhg_context* c, uint32_t particles) {
 }
 
 int bhg_selftest_wait(bhg_context* c, int publish_first, uint32_t spin_limit, uint32_t* prefix) {
-  if (!c) return BHG_EINVAL;
-  if (spin_limit == 0 || spin_limit > (1u << 20))
-    return fail(c, BHG_EINVAL, "spin_limit must be in 1 .. 2^20 (a short wait)");
-  cudaSetDevice(c->device);
-  int r = read_state(c);  // finish what is queued; its own errors come first
-  if (r || (r = finish_async(c))) return r;
   constexpr uint32_t kTiles = 8;
-  uint32_t* words = nullptr;
-  if ((r = dev_alloc(c, reinterpret_cast<void**>(&words), (kTiles + 1) * sizeof(uint32_t)))) return r;
   // tiles 1..7 have published an aggregate of 1 each; tile 0 publishes an
   // inclusive prefix of 1, or nothing at all
-  uint32_t h[kTiles + 1] = {};
-  for (uint32_t t = 1; t < kTiles; ++t) h[t] = kFlagAgg | 1u;
-  h[0] = publish_first ? (kFlagPre | 1u) : 0u;
-  cudaError_t e = cudaMemcpyAsync(words, h, sizeof h, cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) {
-    launch_wait_probe(words, kTiles, (int)spin_limit, c->st, words + kTiles, c->stream);
-    e = cudaGetLastError();
-  }
-  uint32_t got = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&got, words + kTiles, sizeof got, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  dev_free(c, words);
-  if (e != cudaSuccess) return fail(c, BHG_ECUDA, std::string("selftest_wait: ") + cudaGetErrorString(e));
-  if (prefix) *prefix = got;
-  if ((r = read_state(c))) return r;
-  r = check_status(c);  // a wait that gave up: BHG_EDEVICE, as from a real sort or scan
-  clear_status(c);
-  return r;
+  std::vector<uint32_t> words(kTiles, kFlagAgg | 1u);
+  words[0] = publish_first ? (kFlagPre | 1u) : 0u;
+  return selftest(c, spin_limit, words, prefix, 1, [&](uint32_t* w, uint32_t* out) {
+    launch_wait_probe(w, kTiles, (int)spin_limit, c->st, out, c->stream);
+  });
+}
+
+int bhg_selftest_walk_wait(bhg_context* c, int publish, uint32_t spin_limit, uint32_t* words) {
+  std::vector<uint32_t> w(3, kWalkPending);
+  if (publish) w = {128u, 3u | 2u << 16, 5u | 4u << 16};
+  return selftest(c, spin_limit, w, words, 3, [&](uint32_t* at, uint32_t* out) {
+    launch_walk_wait_probe(at, (int)spin_limit, c->st, out, c->stream);
+  });
 }
 
 int bhg_measure_fp32_peak(int device, double* tflops) {

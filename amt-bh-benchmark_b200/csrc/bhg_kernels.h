@@ -100,6 +100,9 @@ struct WalkArgs {
 // particles.
 void launch_walk(const WalkArgs& a, uint32_t n, int precision, bool quad, bool mask, int grid, cudaStream_t s);
 int walk_blocks_per_sm(int precision, bool quad, bool mask);
+// The walk's two waits on prepared words (a group's progress and list length,
+// another's list length); out: progress and lengths as they left them.
+void launch_walk_wait_probe(uint32_t* words, int limit, DevState* st, uint32_t* out, cudaStream_t s);
 int walk_threads();
 // device bytes of one list slot, and of one warp's dense list
 size_t walk_slot_bytes();

@@ -58,7 +58,7 @@ constexpr uint32_t kByNode = 255;
 static_assert(kMaxTargets <= kCountShift, "target masks and counts share a word");
 constexpr uint32_t kDenseCap = 2048;  // entries of a dense list (16 KB)
 // a group's list lengths are cells | runs << 16 (two-pass schedule)
-static_assert(kListCap < 0xfefe, "list lengths never look pending");
+static_assert(kListCap < 0xfefe, "list lengths never look pending, nor lost");
 // a traversal step pops at most (free entries - kLevels - 1) nodes, one at
 // least, and every popped node pushes at most one run of children, so that
 // one-node steps (depth first, at most one run per level) never overflow
@@ -730,22 +730,46 @@ __device__ __forceinline__ uint4 load_pair(const uint4* p, uint32_t i, uint32_t 
   return v;
 }
 
-// A dense job's wait (bounded) for cells beyond `at` (a multiple of 64): the
-// cells that may be read, a multiple of 64 too unless they are all.
-__device__ __forceinline__ uint32_t more_cells(const WalkArgs& a, WarpSmem& S, uint32_t at, int lane) {
-  Job& J = S.job;
-  uint32_t v = 0;
+// A dense job's wait (bounded, as wait_lengths) for cells beyond `at` (a
+// multiple of 64) in its group's progress word: the word, or kAborted after
+// `limit` polls.  The group's target jobs, which wait for this one, are then
+// told (kListLost): each would poll to its own limit, half a second.
+__device__ __forceinline__ uint32_t wait_cells(const uint32_t* prog, uint32_t* length, uint32_t at, int limit,
+                                               DevState* st, int lane) {
   for (int spins = 0;; ++spins) {
-    v = ld_volatile(a.prog + J.gi);
+    uint32_t v = ld_volatile(prog);
     v = __shfl_sync(kFull, v == kListPending ? 0u : v, 0);
-    if ((v & (kFinal | kAborted)) || (v & ~63u) > at) break;
-    if (spins >= kSpinLimit) {
-      if (lane == 0) atomicOr(&a.st->status, kStSpinLimit);
-      v = kAborted;
-      break;
+    if ((v & (kFinal | kAborted)) || (v & ~63u) > at) return v;
+    if (spins >= limit) {
+      if (lane == 0) {
+        atomicOr(&st->status, kStSpinLimit);
+        st_volatile(length, kListLost);
+      }
+      return kAborted;
     }
     __nanosleep(64);
   }
+}
+
+// Both waits on prepared words (bhg_selftest_walk_wait), one warp: a group's
+// progress and its list length, and another group's list length.  out: the
+// progress, the first length as that wait left it, the second length.
+__global__ void k_walk_wait_probe(uint32_t* words, int limit, DevState* st, uint32_t* out) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t cells = wait_cells(words, words + 1, 64u, limit, st, lane);
+  const uint32_t len = wait_lengths(words + 2, limit, st, lane);
+  if (lane == 0) out[0] = cells, out[1] = ld_volatile(words + 1), out[2] = len;
+}
+
+void launch_walk_wait_probe(uint32_t* words, int limit, DevState* st, uint32_t* out, cudaStream_t s) {
+  k_walk_wait_probe<<<1, 32, 0, s>>>(words, limit, st, out);
+}
+
+// A dense job's further cells, beyond `at` (a multiple of 64): those that may
+// be read, a multiple of 64 too unless they are all.
+__device__ __forceinline__ uint32_t more_cells(const WalkArgs& a, WarpSmem& S, uint32_t at, int lane) {
+  Job& J = S.job;
+  const uint32_t v = wait_cells(a.prog + J.gi, a.gnl + J.gi, at, kSpinLimit, a.st, lane);
   __threadfence();  // the cells after the word
   if (!(v & (kFinal | kAborted))) return v & ~63u;
   __syncwarp();
@@ -983,16 +1007,8 @@ __global__ void __launch_bounds__(kWalkThreads, E::kBlocksPerSm) k_walk(WalkArgs
     J.poll = J.kind == kDenseJob;
     J.aborted = 0u;
     if (J.kind == kTargetJob) {
-      uint32_t len = ld_volatile(a.gnl + J.gi);
-      for (int spins = 0; len == kListPending && spins < kSpinLimit; ++spins) {
-        __nanosleep(128);
-        len = ld_volatile(a.gnl + J.gi);
-      }
-      len = __shfl_sync(kFull, len, 0);  // one value for the warp
-      if (len == kListPending) {
-        if (lane == 0) atomicOr(&a.st->status, kStSpinLimit);
-        continue;
-      }
+      const uint32_t len = wait_lengths(a.gnl + J.gi, kSpinLimit, a.st, lane);
+      if (len == kListLost) continue;
       __threadfence();  // the group's sums and list after its lengths
       J.w.npc = len & 0xffffu, J.w.npr = len >> 16;
       const uint32_t bit = J.ti - J.t0, tn = a.targets[J.ti];

@@ -13,6 +13,8 @@ constexpr uint32_t kListCap = 4096;  // entries of a list of the sources some ta
 // a group's list length(s) before its shared walk has finished (two-pass
 // schedule; set before every walk)
 constexpr uint32_t kListPending = kWalkPending;
+// ... and when the job that was to publish it gave up waiting itself
+constexpr uint32_t kListLost = 0xfffffffeu;
 
 __device__ __forceinline__ uint32_t warp_incl_scan_u32(uint32_t v, int lane) {
 #pragma unroll
@@ -125,6 +127,21 @@ __device__ __forceinline__ uint32_t system_of(const WalkArgs& a, uint32_t p) {
 // Whether another launch walks system s.
 __device__ __forceinline__ bool walked_elsewhere(const WalkArgs& a, uint32_t s) {
   return a.only != WalkOnly::kAll && (a.prm[s].eps2 > 0.0) != (a.only == WalkOnly::kSoftened);
+}
+
+// A target job's wait, by a warp, for its group's list length(s): them, or
+// kListLost.  Bounded: after `limit` polls it sets kStSpinLimit, so that the
+// kernel ends without the job and the host reports the error.
+__device__ __forceinline__ uint32_t wait_lengths(const uint32_t* length, int limit, DevState* st, int lane) {
+  uint32_t len = ld_volatile(length);
+  for (int spins = 0; len == kListPending && spins < limit; ++spins) {
+    __nanosleep(128);
+    len = ld_volatile(length);
+  }
+  len = __shfl_sync(kFull, len, 0);  // one value for the warp
+  if (len != kListPending) return len;
+  if (lane == 0) atomicOr(&st->status, kStSpinLimit);
+  return kListLost;
 }
 
 // The group of walk group gi: its targets, first particle and system.

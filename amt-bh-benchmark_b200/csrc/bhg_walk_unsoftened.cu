@@ -623,16 +623,8 @@ __device__ __forceinline__ void target_jobs(E& ev, const WalkArgs& a, QueueSmem&
     const GroupInfo g = group_info(a, gi, ngroups, ntargets);
     if (walked_elsewhere(a, g.s)) continue;
     if (g.k == 1) continue;  // done whole in the first pass
-    uint32_t nlist = ld_volatile(a.gnl + gi);
-    for (int spins = 0; nlist == kListPending && spins < kSpinLimit; ++spins) {
-      __nanosleep(128);
-      nlist = ld_volatile(a.gnl + gi);
-    }
-    nlist = __shfl_sync(kFull, nlist, 0);  // one value for the warp
-    if (nlist == kListPending) {
-      if (lane == 0) atomicOr(&a.st->status, kStSpinLimit);
-      continue;
-    }
+    const uint32_t nlist = wait_lengths(a.gnl + gi, kSpinLimit, a.st, lane);
+    if (nlist == kListLost) continue;
     __threadfence();  // the group's sums and list after its length
     const uint32_t tnode = a.targets[ti];
     const uint32_t tb = a.nbegin[tnode], tn = a.ncount[tnode];  // tn <= kGroupMax: inside a group

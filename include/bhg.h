@@ -313,6 +313,16 @@ int bhg_energy_noalloc(const bh_particle64* particles, size_t n, double G, doubl
  * either way.  No counterpart in the reference (its waits are TTG's). */
 int bhg_selftest_wait(bhg_context* ctx, int publish_first, uint32_t spin_limit, uint32_t* prefix);
 
+/* The same for the walk's waits: a dense job's for its group's progress beyond
+ * 64 cells, and a target job's for its group's list lengths.  publish != 0:
+ * both words are there (128 cells; lengths 5 and 4), BHG_OK, and words
+ * (optional, 3 of them) = the progress 128, the list length word 3 | 2 << 16
+ * of the first group untouched, and 5 | 4 << 16.  Else nothing is published:
+ * both waits give up after spin_limit polls (1 .. 2^20), BHG_EDEVICE, and
+ * words = aborted (1 << 30), and twice lost (0xfffffffe): the dense job told
+ * the targets of its group. */
+int bhg_selftest_walk_wait(bhg_context* ctx, int publish, uint32_t spin_limit, uint32_t* words);
+
 /* ---- workload generators (synthetic initial conditions) --------------------------- */
 
 /* Plummer sphere by Aarseth-Henon-Wielen sampling (G = 1): n particles of

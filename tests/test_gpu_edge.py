@@ -119,3 +119,22 @@ def test_bounded_wait_gives_up_and_context_survives(oracle):
         for bad in (0, (1 << 20) + 1):
             r, _ = ctx.selftest_wait(False, bad)
             assert r == bhg.EINVAL
+
+
+def test_bounded_walk_waits_give_up_and_context_survives(oracle):
+    """The walk's waits, for cells and for list lengths that nothing publishes,
+    give up after their poll limit: BHG_EDEVICE, the targets of the dense job's
+    group told, the context usable.  Published, they return the words."""
+    with bhg.Context(device=0) as ctx:
+        assert ctx.selftest_walk_wait(True, 1000) == (bhg.OK, (128, 3 | 2 << 16, 5 | 4 << 16))
+        r, words = ctx.selftest_walk_wait(False, 1000)
+        assert r == bhg.EDEVICE and words == (1 << 30, 0xfffffffe, 0xfffffffe)
+        assert "bounded wait" in ctx.last_error()
+        assert ctx.device_status() == 0
+        parts = cube(6000, 4)
+        out, _, _ = oracle.step(parts, theta=0.5, eps2=1e-6, max_leaf=8, group_size=64, target_size=0)
+        ctx.upload(parts)
+        ctx.step(bhg.Context.params(0.5, 1e-6, 1.0, True, bhg.PRECISION_FP64), 8, 64, 0, 0.0, 0.0)
+        assert np.array_equal(ctx.download()["id"], out["id"])
+        for bad in (0, (1 << 20) + 1):
+            assert ctx.selftest_walk_wait(False, bad)[0] == bhg.EINVAL
