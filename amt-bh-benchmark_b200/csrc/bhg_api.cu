@@ -1684,7 +1684,7 @@ int bhg_direct_sum(bhg_context* c, int sys, const uint32_t* idx, size_t ns, doub
   for (size_t k = 0; k < ns; ++k)
     if (idx[k] >= d.n) return fail(c, BHG_EINVAL, "sample index out of range");
   if (ns == 0) return BHG_OK;
-  if (ns > 0x7fffffffull / 3) return fail(c, BHG_EINVAL, "too many sample rows");
+  if (ns > 0xffffff00ull) return fail(c, BHG_EINVAL, "too many sample rows");  // row numbers of whole blocks in 32 bits
   // row indices, results and parts in the context's cached scratch
   const DirectPlan plan = direct_plan(d.n, (uint32_t)ns, c->sms);
   Scratch sc(c);
