@@ -490,7 +490,7 @@ void enq_sort(bhg_context* c) {
 
 void enq_tree(bhg_context* c) {
   // kSortPasses is even: sorted keys and the permutation are back in [0]
-  launch_gather(c->part, c->vals[0], (uint32_t)c->n, c->staged, c->pm, c->sms, c->stream);
+  launch_gather(c->part, c->vals[0], (uint32_t)c->n, c->staged, c->pm, c->st, c->sms, c->stream);
   // the other value buffer is free after the sort
   launch_topology(c->tiles, (int)c->tiles_host.size(), c->sys, c->nd, c->keys[0], c->max_leaf, c->vals[1],
                   c->unit_counts, c->st, c->stream);

@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(NT, MINB) k_sort_pass(const uint64_t* __restri
                                                         const uint32_t* __restrict__ offs, uint32_t* lookback,
                                                         DevState* st) {
   static_assert(NT >= kDigits && NT % 32 == 0, "one thread per digit");
+  constexpr uint32_t kNoTile = 0xffffffffu;
   constexpr int kWarps = NT / 32;
   constexpr int kSortTile = NT * ITEMS;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -361,10 +362,16 @@ __global__ void __launch_bounds__(NT, MINB) k_sort_pass(const uint64_t* __restri
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int shift = 8 * pass;
-  if (tid == 0) s_misc[0] = atomicAdd(&st->sort_tiles[pass], 1u);
+  if (tid == 0) {
+    const uint32_t status = st->status;  // in flight with the ticket
+    const uint32_t ticket = atomicAdd(&st->sort_tiles[pass], 1u);
+    // a wait gave up: the keys are not all there, and their digits not those counted
+    s_misc[0] = status & kStSpinLimit ? kNoTile : ticket;
+  }
   for (int i = tid; i < kWarps * kDigits; i += NT) s_whist[i] = 0;
   __syncthreads();
   const uint32_t tile = s_misc[0];
+  if (tile == kNoTile) return;
   const Tile t = tiles[tile];
   uint32_t* my_hist = s_whist + warp * kDigits;
 
@@ -439,11 +446,19 @@ static_assert(SortSmall::TILE == kSortTileSmall && SortLarge::TILE == kSortTileL
 // ---------------------------------------------------------------------------
 // gather into Morton order: staged[i] = particles[perm[i]], pm[i] = (x,y,z,m)
 // (sort_particles' final loop, flat_build_ttg.h:180-188)
+//
+// A sort whose wait gave up leaves places of its output unwritten: whatever
+// keys and indices lay there.  Neither its later passes nor the gather and the
+// octree use them: no node is counted or written, so nothing after them finds
+// a node either.
 
 __global__ void k_gather(const Particle* __restrict__ p, const uint32_t* __restrict__ perm, uint32_t n,
-                         Particle* __restrict__ staged, double4* __restrict__ pm) {
+                         Particle* __restrict__ staged, double4* __restrict__ pm, const DevState* __restrict__ st) {
+  const uint32_t status = st->status;  // in flight with the first index
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint4* src = reinterpret_cast<const uint4*>(p + perm[i]);
+    const uint32_t at = perm[i];
+    if (status & kStSpinLimit) return;
+    const uint4* src = reinterpret_cast<const uint4*>(p + at);
     uint4* dst = reinterpret_cast<uint4*>(staged + i);
     uint4 a = src[0], b = src[1], c = src[2], e = src[3];
     dst[0] = a;
@@ -563,6 +578,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_node_depths(const Tile* __rest
 __global__ void __launch_bounds__(32 * kLevels) k_node_offsets(uint32_t* __restrict__ counts, uint32_t units,
                                                                uint32_t cap, DevState* st) {
   __shared__ uint32_t total[32];
+  const uint32_t status = st->status;
   const uint32_t lane = threadIdx.x & 31u, d = threadIdx.x >> 5;
   uint32_t* c = counts + (size_t)d * units;
   uint32_t run = 0;
@@ -583,7 +599,7 @@ __global__ void __launch_bounds__(32 * kLevels) k_node_offsets(uint32_t* __restr
   }
   if (lane == 0) total[d] = run;
   __syncthreads();
-  if (d != 0) return;
+  if (d != 0 || (status & kStSpinLimit)) return;
   const uint32_t n = lane < kLevels ? total[lane] : 0u, inc = warp_incl_scan(n);
   const uint32_t levels = (uint32_t)__popc(__ballot_sync(0xffffffffu, n != 0u));  // none is empty above the deepest
   if (lane < kLevels) st->level_begin[lane] = inc - n, st->level_count[lane] = n;
@@ -602,6 +618,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_node_emit(const Tile* __restri
                                                             const uint32_t* __restrict__ offsets, Nodes nd,
                                                             const DevState* __restrict__ st) {
   __shared__ uint32_t cnt[kNodeWarps][32];
+  const uint32_t status = st->status;
   const Tile t = node_unit(tiles, unit, blockIdx.x);
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t le = lanemask_lt() | (1u << lane);
@@ -619,6 +636,7 @@ __global__ void __launch_bounds__(kNodeThreads) k_node_emit(const Tile* __restri
   }
   cnt[warp][lane] = base;
   __syncthreads();
+  if (status & kStSpinLimit) return;
   if (lane < kLevels) {
     base = st->level_begin[lane] + offsets[(size_t)lane * gridDim.x + blockIdx.x];
     for (uint32_t w = 0; w < warp; ++w) base += cnt[w][lane];
@@ -799,7 +817,7 @@ constexpr int kPackWindows = 4;  // windows of 32 targets whose counts are loade
 __global__ void k_pack_groups(const uint32_t* __restrict__ restart, const uint32_t* __restrict__ targets,
                               const uint32_t* __restrict__ ncount, uint32_t pack, const DevState* __restrict__ st,
                               uint32_t* __restrict__ mark) {
-  if (st->status & kStNodeOverflow) return;
+  if (st->status & (kStNodeOverflow | kStSpinLimit)) return;  // the targets are not all there
   const uint32_t nt = st->n_targets;
   const int lane = threadIdx.x & 31;
   const uint32_t nw = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1038,12 +1056,12 @@ void launch_fill(const FillList& f, int sms, cudaStream_t s) {
   k_fill<<<(unsigned)std::max<size_t>(1, std::min<size_t>((most + 1023) / 1024, (size_t)sms * 8)), 256, 0, s>>>(f);
 }
 
-void launch_gather(const Particle* p, const uint32_t* perm, uint32_t n, Particle* staged, double4* pm, int sms,
-                   cudaStream_t s) {
+void launch_gather(const Particle* p, const uint32_t* perm, uint32_t n, Particle* staged, double4* pm,
+                   const DevState* st, int sms, cudaStream_t s) {
   int blocks = (int)((n + 255) / 256);
   if (blocks > sms * 8) blocks = sms * 8;
   if (blocks < 1) blocks = 1;
-  k_gather<<<blocks, 256, 0, s>>>(p, perm, n, staged, pm);
+  k_gather<<<blocks, 256, 0, s>>>(p, perm, n, staged, pm, st);
 }
 
 // Blocks for a grid that takes `units` work items `per_block` at a time, at

@@ -30,8 +30,8 @@ struct FillList {
   }
 };
 void launch_fill(const FillList& f, int sms, cudaStream_t s);
-void launch_gather(const Particle* p, const uint32_t* perm, uint32_t n, Particle* staged, double4* pm, int sms,
-                   cudaStream_t s);
+void launch_gather(const Particle* p, const uint32_t* perm, uint32_t n, Particle* staged, double4* pm,
+                   const DevState* st, int sms, cudaStream_t s);
 // Octree topology of the sorted keys (nd.info zeroed before).  depths: n
 // words of scratch; counts: kLevels words per unit of node_unit_size particles.
 uint32_t node_unit_size(int ntiles);
