@@ -1,7 +1,7 @@
 // Tree build of the B200 Barnes-Hut path: bounds and domain, Morton keys,
 // a 64-bit LSD radix sort of (key, index), the gather into Morton order, the
-// level-by-level octree topology, the walk targets and the level-by-level
-// multipole upward pass.  Everything is exact: keys, order and topology are
+// octree topology from neighbouring keys, the walk targets and the multipole
+// upward pass.  Everything is exact: keys, order and topology are
 // bit-identical to the reference's build_flat_tree (flat_build_ttg.h:276-281),
 // and the multipoles repeat its floating-point operations in the same order
 // (explicit round-to-nearest intrinsics, no contraction).
@@ -839,26 +839,26 @@ __global__ void k_pack_groups(const uint32_t* __restrict__ restart, const uint32
         for (int w = 0; w < kPackWindows; ++w) {
           if (end) break;
           // the greedy packing: from place `pos` on, the next group starts at the
-        // first target that would make the current one too large, found for
-        // all 32 at once from the sums of the counts
-        const uint32_t nv = (uint32_t)__ffs(~__ballot_sync(0xffffffffu, n[w] != 0xffffffffu)) - 1u;  // ~0: all 32
-        const uint32_t live = min(nv, 32u), in = (uint32_t)lane < live ? n[w] : 0u, sum = warp_incl_scan(in);
-        end = live < 32u;
-        uint32_t starts = 0, pos = 0, before = 0;  // before: the counts up to pos
-        for (;;) {
-          const uint32_t i = (uint32_t)lane;
-          const bool over = first || cnt + (sum - before) > pack || k + (i - pos) >= (uint32_t)kMaxTargets;
-          const uint32_t m = __ballot_sync(0xffffffffu, i >= pos && i < live && over);
-          if (!m) break;
-          const uint32_t at_i = (uint32_t)__ffs(m) - 1u;
-          starts |= 1u << at_i;
-          first = false;
-          cnt = __shfl_sync(0xffffffffu, in, at_i), k = 1u;
-          before = __shfl_sync(0xffffffffu, sum, at_i), pos = at_i + 1u;
-        }
-        cnt += __shfl_sync(0xffffffffu, sum, 31) - before;
-        k += live - pos;
-        if ((starts >> lane) & 1u) mark[t0 + 32u * w + (uint32_t)lane] = t0 + 32u * w + (uint32_t)lane;
+          // first target that would make the current one too large, found for
+          // all 32 at once from the sums of the counts
+          const uint32_t nv = (uint32_t)__ffs(~__ballot_sync(0xffffffffu, n[w] != 0xffffffffu)) - 1u;  // ~0: all 32
+          const uint32_t live = min(nv, 32u), in = (uint32_t)lane < live ? n[w] : 0u, sum = warp_incl_scan(in);
+          end = live < 32u;
+          uint32_t starts = 0, pos = 0, before = 0;  // before: the counts up to pos
+          for (;;) {
+            const uint32_t i = (uint32_t)lane;
+            const bool over = first || cnt + (sum - before) > pack || k + (i - pos) >= (uint32_t)kMaxTargets;
+            const uint32_t m = __ballot_sync(0xffffffffu, i >= pos && i < live && over);
+            if (!m) break;
+            const uint32_t at_i = (uint32_t)__ffs(m) - 1u;
+            starts |= 1u << at_i;
+            first = false;
+            cnt = __shfl_sync(0xffffffffu, in, at_i), k = 1u;
+            before = __shfl_sync(0xffffffffu, sum, at_i), pos = at_i + 1u;
+          }
+          cnt += __shfl_sync(0xffffffffu, sum, 31) - before;
+          k += live - pos;
+          if ((starts >> lane) & 1u) mark[t0 + 32u * w + (uint32_t)lane] = t0 + 32u * w + (uint32_t)lane;
         }
       }
     }
