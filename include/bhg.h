@@ -140,7 +140,9 @@ typedef struct bhg_sphere {
 /* Grows the context's buffers now for up to `particles` particles in up to
  * `systems` systems, with the node slots they bring at max_leaf 16, so that
  * systems added later within those sizes neither allocate nor copy the
- * resident state.  Counts against the HBM budget (BHG_ENOMEM past it). */
+ * resident state.  Resident systems stay; a tree built before a growth of
+ * particles, systems or nodes is gone (BHG_ESTATE until the next build).
+ * Counts against the HBM budget (BHG_ENOMEM past it). */
 int bhg_reserve(bhg_context* ctx, size_t particles, size_t systems);
 
 /* Appends one system of n particles from host memory; its handle goes to
